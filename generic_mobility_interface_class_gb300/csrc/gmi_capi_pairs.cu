@@ -58,6 +58,7 @@ gmi_status gmi_context_destroy(gmi_context *ctx)
     ctx->rec_tgt.release();
     ctx->partial.release();
     ctx->cells.release();
+    ctx->fx.release();
     if (ctx->d_err) gmi::dev_free(ctx->d_err);
     if (ctx->h_err) gmi::host_free(ctx->h_err);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -115,11 +116,7 @@ gmi_status gmi_Mss_mult(gmi_context *ctx, double *V_d, const double *F_d, const 
     GMI_ARG_CHECK(rseg > 0 && mu > 0, "gmi_Mss_mult: radius and viscosity must be positive");
     gmi_status st = select_device(ctx);
     if (st != GMI_OK) return st;
-    st = pack_records(ctx, X_d, F_d, 6, total_segs, ctx->rec_src);
-    if (st != GMI_OK) return st;
-    PairConsts k;
-    fill_consts(k, rseg, rseg, rseg, mu);
-    return launch_pair(ctx, kSS, ctx->rec_src.ptr, start_seg, num_segs, ctx->rec_src.ptr, total_segs, k, V_d, 0);
+    return pair_sum(ctx, kSS, X_d, total_segs, start_seg, num_segs, X_d, F_d, total_segs, rseg, rseg, mu, V_d, 0);
 }
 
 gmi_status gmi_Mss_mult_wall(gmi_context *ctx, double *V_d, const double *F_d, const double *X_d, int start_seg,
@@ -132,11 +129,7 @@ gmi_status gmi_Mss_mult_wall(gmi_context *ctx, double *V_d, const double *F_d, c
                   "gmi_Mss_mult_wall: target range outside [0, total_segs)");
     gmi_status st = select_device(ctx);
     if (st != GMI_OK) return st;
-    st = pack_records(ctx, X_d, F_d, 6, total_segs, ctx->rec_src);
-    if (st != GMI_OK) return st;
-    PairConsts k;
-    fill_consts(k, 1.0, 1.0, 1.0, 1.0);
-    return launch_pair(ctx, kSSWall, ctx->rec_src.ptr, start_seg, num_segs, ctx->rec_src.ptr, total_segs, k, V_d, 0);
+    return pair_sum(ctx, kSSWall, X_d, total_segs, start_seg, num_segs, X_d, F_d, total_segs, 1.0, 1.0, 1.0, V_d, 0);
 }
 
 gmi_status gmi_Mbb_mult(gmi_context *ctx, double *V_d, const double *F_d, const double *X_d, int start_blob,
@@ -149,11 +142,8 @@ gmi_status gmi_Mbb_mult(gmi_context *ctx, double *V_d, const double *F_d, const 
     GMI_ARG_CHECK(rblob > 0 && mu > 0, "gmi_Mbb_mult: radius and viscosity must be positive");
     gmi_status st = select_device(ctx);
     if (st != GMI_OK) return st;
-    st = pack_records(ctx, X_d, F_d, 3, total_blobs, ctx->rec_src);
-    if (st != GMI_OK) return st;
-    PairConsts k;
-    fill_consts(k, rblob, rblob, rblob, mu);
-    return launch_pair(ctx, kBB, ctx->rec_src.ptr, start_blob, num_blobs, ctx->rec_src.ptr, total_blobs, k, V_d, 0);
+    return pair_sum(ctx, kBB, X_d, total_blobs, start_blob, num_blobs, X_d, F_d, total_blobs, rblob, rblob, mu, V_d,
+                    0);
 }
 
 gmi_status gmi_Msb_mult(gmi_context *ctx, double *V_d, const double *F_blobs_d, const double *Xs_d,
@@ -168,13 +158,8 @@ gmi_status gmi_Msb_mult(gmi_context *ctx, double *V_d, const double *F_blobs_d, 
     GMI_ARG_CHECK(total_blobs >= 0 && rseg > 0 && rblob > 0 && mu > 0, "gmi_Msb_mult: bad size or radius");
     gmi_status st = select_device(ctx);
     if (st != GMI_OK) return st;
-    st = pack_records(ctx, Xs_d, nullptr, 0, total_segs, ctx->rec_tgt);
-    if (st != GMI_OK) return st;
-    st = pack_records(ctx, Xb_d, F_blobs_d, 3, total_blobs, ctx->rec_src);
-    if (st != GMI_OK) return st;
-    PairConsts k;
-    fill_consts(k, rseg, rseg, rblob, mu);
-    return launch_pair(ctx, kSB, ctx->rec_tgt.ptr, start_seg, num_segs, ctx->rec_src.ptr, total_blobs, k, V_d, 1);
+    return pair_sum(ctx, kSB, Xs_d, total_segs, start_seg, num_segs, Xb_d, F_blobs_d, total_blobs, rseg, rblob, mu,
+                    V_d, 1);
 }
 
 gmi_status gmi_Mbs_mult(gmi_context *ctx, double *V_d, const double *F_segs_d, const double *Xb_d,
@@ -189,13 +174,8 @@ gmi_status gmi_Mbs_mult(gmi_context *ctx, double *V_d, const double *F_segs_d, c
     GMI_ARG_CHECK(total_segs >= 0 && rseg > 0 && rblob > 0 && mu > 0, "gmi_Mbs_mult: bad size or radius");
     gmi_status st = select_device(ctx);
     if (st != GMI_OK) return st;
-    st = pack_records(ctx, Xb_d, nullptr, 0, total_blobs, ctx->rec_tgt);
-    if (st != GMI_OK) return st;
-    st = pack_records(ctx, Xs_d, F_segs_d, 6, total_segs, ctx->rec_src);
-    if (st != GMI_OK) return st;
-    PairConsts k;
-    fill_consts(k, rseg, rseg, rblob, mu);
-    return launch_pair(ctx, kBS, ctx->rec_tgt.ptr, start_blob, num_blobs, ctx->rec_src.ptr, total_segs, k, V_d, 0);
+    return pair_sum(ctx, kBS, Xb_d, total_blobs, start_blob, num_blobs, Xs_d, F_segs_d, total_segs, rseg, rblob, mu,
+                    V_d, 0);
 }
 
 gmi_status gmi_barrier_forces(gmi_context *ctx, double *f_segs_d, double *f_blobs_repulsion_d, const double *x_segs_d,
@@ -278,6 +258,15 @@ gmi_status gmi_autotune(gmi_context *ctx, int kind, int num_targets, int num_sou
     GMI_ARG_CHECK(num_targets > 0 && num_sources > 0, "gmi_autotune: sizes must be positive");
     gmi_status st = select_device(ctx);
     if (st != GMI_OK) return st;
+    if (ctx->precision == GMI_FP64 && kind != kSSWall) {
+        // one kernel, which sizes its own splits: nothing to time
+        PairShape fx;
+        fx.tt = 1;
+        fx.packed = 0;
+        fx.fx = true;
+        ctx->tuned[TuneKey{kind, ctx->precision, num_targets, num_sources}] = fx;
+        return GMI_OK;
+    }
     // synthetic problem on a jittered lattice with unit-scale loads
     DeviceBuffer xt, xsrc, fsrc, out, rt, rs;
     const int nf = (kind == kBB || kind == kSB) ? 3 : 6;

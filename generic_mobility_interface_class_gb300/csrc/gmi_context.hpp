@@ -28,6 +28,7 @@ struct PairShape {
     int tt = 2;        // targets per thread
     int splits = 0;    // source splits; 0 = choose from the SM count
     int packed = -1;   // two sources per thread step (FP32, no wall): 1 yes, 0 no, -1 where available
+    bool fx = false;   // the fixed-point kernel (FP64, no wall), which chooses its own splits
 };
 
 enum PairKind : int { kSS = 0, kSSWall = 1, kBB = 2, kSB = 3, kBS = 4 };
@@ -47,6 +48,8 @@ struct gmi_context {
     long long launches = 0;          // kernels this context has launched
     gmi::DeviceBuffer rec_src, rec_tgt, partial;
     gmi::DeviceBuffer cells;  // the barrier's cell list
+    gmi::DeviceBuffer fx;     // the fixed-point pair sums: tickets (zero between launches), records, partial sums
+    size_t fx_tickets = 0;    // bytes of fx that are zeroed tickets
     std::map<gmi::TuneKey, gmi::PairShape> tuned;
     int last_splits = 1;  // source splits of the last tiled pair launch (the autotuner reads it)
     void *encode_tiled = nullptr;    // cuTensorMapEncodeTiled from the driver

@@ -1,0 +1,428 @@
+// gmi_fx_kernels.cu -- the FP64-grade free-space pair sums (precision
+// GMI_FP64) in 64-bit fixed point.
+//
+// Two kernels per sum.  The pack kernel turns the sources into integer
+// records (gmi_pairs_fx.cuh), one CTA per tile of 128 with the tile's
+// exponent found by a block maximum.  In the pair kernel a CTA owns 32
+// targets, one per lane, and a contiguous slice ("split") of the sources,
+// staged tile by tile into shared memory by bulk copies; its four warps take
+// a quarter of each tile each, fold their integer sums into FP64 per tile
+// and meet in shared memory at the end.  32 targets per CTA rather than 128
+// let a few hundred targets reach every SM.  With several splits the last CTA
+// of a target group to finish adds the group's partial sums in split order.
+//
+// A tile whose loads or positions the formats do not hold (not finite, a load
+// beyond 2^+-900, a particle further than about 400 radii from the first
+// source) is marked by the pack kernel, and its pairs, and all pairs of a
+// warp with such a target, are summed in FP64 from the original arrays.
+//
+// What bounds it: the integer pipes.  M_ss executes about 530 instructions a
+// pair and warp (210 on the FMA pipe, 146 of them 32x32 -> 64-bit, 290 on the
+// ALU) at 1.8 cycles each, whatever the split and the occupancy; the FP64
+// kernel executed 65 FP64 instructions at 76 cycles each.  12,800 segments:
+// 20.4 -> 3.9 ms (87 flop a pair: 0.70 -> 3.7 TFLOP/s); 4096 blobs: 1222 ->
+// 231 us; 12,800 segments with 4096 blobs, both ways: 9.7 -> 1.8 ms.  Error
+// against exact sums at 12,800 segments: 1.4e-15 -> 3.1e-16.
+#include <algorithm>
+
+#include "gmi_fx_kernels.hpp"
+#include "gmi_pair_kernels.hpp"
+#include "gmi_pairs.cuh"
+#include "gmi_pairs_fx.cuh"
+
+namespace gmi {
+
+static_assert((int)kFxSS == (int)kSS && (int)kFxBB == (int)kBB && (int)kFxSB == (int)kSB && (int)kFxBS == (int)kBS,
+              "FxKind follows PairKind");
+
+constexpr int kFxTile = 128;   // sources per tile: one exponent, one stage
+constexpr int kFxTpb = 128;    // four warps
+constexpr int kFxWarps = kFxTpb / 32;
+constexpr int kFxStages = 2;
+constexpr int kFxBadTile = -0x7fffffff;  // in place of a tile's exponent: sum it in FP64
+static_assert(kFxTile == kFxWarps * kFxFold, "a warp's quarter of a tile is one fold");
+
+template <int KIND> struct FxTraits {
+    static constexpr bool torque = KIND == kFxSS || KIND == kFxBS;
+    static constexpr int nout = (KIND == kFxSS || KIND == kFxSB) ? 6 : 3;
+    static constexpr int nf = torque ? 6 : 3;
+    static constexpr int words = torque ? 10 : 8;  // 64-bit words per record: X F [T] {gap, E} [pad]
+    static constexpr int meta = torque ? 9 : 6;
+};
+
+struct FxLaunch {
+    const double *xt, *xs, *fs;
+    const unsigned long long *rec;
+    int tgt_start, n_tgt, n_src, chunk;
+    double *out, *partial;
+    int *tickets;  // non-null: the last CTA of a target group adds the partials
+    int accumulate;
+    unsigned *err;
+    const int *skip;
+    unsigned long long wait_ns;
+    FxConsts K;
+    EqualK<double> eq;
+    UnequalK<double> uq;
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(kFxTile) fx_pack_kernel(const double *__restrict__ x, const double *__restrict__ f,
+                                                          int n, FxConsts K, unsigned long long *__restrict__ rec,
+                                                          const int *skip)
+{
+    using Tr = FxTraits<KIND>;
+    __shared__ int wmax[kFxTile / 32];
+    pdl_wait_then_release();
+    if (skip != nullptr && *skip != 0) return;
+    const int i = blockIdx.x * kFxTile + threadIdx.x, lane = threadIdx.x & 31;
+    long long X[3] = {0, 0, 0};
+    double F[Tr::nf];
+    int e = kFxNoLoad;
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < Tr::nf; ++c) F[c] = 0.0;
+    if (i < n) {
+        double mx = 0.0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            ok = fx_position(x[3 * (size_t)i + c], K.pos_scale, fx_origin(x[c], K.pos_scale), &X[c]) && ok;
+#pragma unroll
+        for (int c = 0; c < Tr::nf; ++c) {
+            F[c] = f[Tr::nf * (size_t)i + c] * (c < 3 ? 1.0 : K.inv_unit);
+            // the larger magnitude by its bits: a NaN or infinity stays the largest
+            mx = __longlong_as_double(max(__double_as_longlong(mx), __double_as_longlong(fabs(F[c]))));
+        }
+        ok = fx_load_exponent(mx, &e) && ok;
+    }
+    // the tile's exponent, or its mark
+    int v = ok ? e : 0x7fffffff;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (lane == 0) wmax[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int E = wmax[0];
+#pragma unroll
+    for (int w = 1; w < kFxTile / 32; ++w) E = max(E, wmax[w]);
+    if (i >= n) return;
+    int gap = 0, used = 0;
+    if (E == 0x7fffffff) {
+        E = kFxBadTile;
+#pragma unroll
+        for (int c = 0; c < Tr::nf; ++c) F[c] = 0.0;
+    } else if (E == kFxNoLoad) {
+        E = 0;
+    } else if (e != kFxNoLoad) {
+        gap = min(E - e, kFxMaxGap);
+        used = E - gap;
+    }
+    const double scale = fx_exp2(-used);
+    unsigned long long *r = rec + (size_t)i * Tr::words;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        r[c] = (unsigned long long)X[c];
+        const fx l = fx_split(fx_from_double(F[c] * scale));
+        r[3 + c] = ((unsigned long long)(unsigned)l.hi << 32) | (unsigned)l.lo;
+    }
+    if (Tr::torque)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) r[6 + c] = (unsigned long long)fx_from_double(F[3 + c] * scale);
+    r[Tr::meta] = ((unsigned long long)(unsigned)E << 32) | (unsigned)gap;
+}
+
+struct FxSum {
+    double v[6];
+};
+
+// The sources [j0, j1) on one target in FP64, for the tiles and targets that
+// the fixed-point formats do not hold.
+template <int KIND>
+static __device__ __noinline__ FxSum fx_sum_fp64(const FxLaunch &a, int ti, int j0, int j1)
+{
+    FxSum s{};
+    const double xi = a.xt[3 * (size_t)ti], yi = a.xt[3 * (size_t)ti + 1], zi = a.xt[3 * (size_t)ti + 2];
+    for (int j = j0; j < j1; ++j) {
+        double F[6] = {0, 0, 0, 0, 0, 0};
+        for (int c = 0; c < FxTraits<KIND>::nf; ++c) F[c] = a.fs[FxTraits<KIND>::nf * (size_t)j + c];
+        const double dx = xi - a.xs[3 * (size_t)j], dy = yi - a.xs[3 * (size_t)j + 1],
+                     dz = zi - a.xs[3 * (size_t)j + 2];
+        if constexpr (KIND == kFxSS) pair_ss<double>(dx, dy, dz, F, a.eq, s.v, s.v + 3);
+        if constexpr (KIND == kFxBB) pair_bb<double>(dx, dy, dz, F, a.eq, s.v);
+        if constexpr (KIND == kFxSB) pair_sb<double>(dx, dy, dz, F, a.uq, s.v, s.v + 3);
+        if constexpr (KIND == kFxBS) pair_bs<double>(dx, dy, dz, F, a.uq, s.v);
+    }
+    return s;
+}
+
+__device__ __forceinline__ fx fx_limbs(unsigned long long w) { return fx{(int)(w >> 32), (int)(unsigned)w}; }
+
+template <int KIND> __device__ __forceinline__ FxSource fx_load_source(const unsigned long long *p)
+{
+    const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p);
+    const ulonglong2 a = q[0], b = q[1], c = q[2];
+    FxSource s;
+    s.X[0] = (long long)a.x;
+    s.X[1] = (long long)a.y;
+    s.X[2] = (long long)b.x;
+    s.F[0] = fx_limbs(b.y);
+    s.F[1] = fx_limbs(c.x);
+    s.F[2] = fx_limbs(c.y);
+    if constexpr (FxTraits<KIND>::torque) {
+        const ulonglong2 d = q[3], e = q[4];
+        s.T[0] = (long long)d.x;
+        s.T[1] = (long long)d.y;
+        s.T[2] = (long long)e.x;
+        s.gap = (int)(unsigned)e.y;
+    } else {
+        s.gap = (int)(unsigned)p[FxTraits<KIND>::meta];
+    }
+    return s;
+}
+
+// bulk copy of whole records (a multiple of 16 bytes) into shared memory
+__device__ __forceinline__ void bulk_load(void *smem_dst, const void *src, unsigned bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(smem_dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(const __grid_constant__ FxLaunch a)
+{
+    using Tr = FxTraits<KIND>;
+    constexpr int NOUT = Tr::nout;
+    __shared__ __align__(128) unsigned long long ring[kFxStages][kFxTile * Tr::words];
+    __shared__ double red[kFxWarps][NOUT][33];
+    __shared__ uint64_t bars[kFxStages];
+    __shared__ int is_last;
+
+    pdl_wait();
+    if (a.skip != nullptr && *a.skip != 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int j_begin = blockIdx.y * a.chunk, j_end = min(j_begin + a.chunk, a.n_src);
+    const int ntiles = (j_end - j_begin + kFxTile - 1) / kFxTile;
+    if (tid == 0) {
+#pragma unroll
+        for (int s = 0; s < kFxStages; ++s) mbar_init(&bars[s], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    int issued = 0;  // tiles requested so far (meaningful on thread 0)
+    const auto request = [&](int t) {
+        const int j0 = j_begin + t * kFxTile;
+        const unsigned bytes = (unsigned)min(kFxTile, j_end - j0) * (Tr::words * 8u);
+        mbar_arrive_expect_tx(&bars[t % kFxStages], bytes);
+        bulk_load(ring[t % kFxStages], a.rec + (size_t)j0 * Tr::words, bytes, &bars[t % kFxStages]);
+    };
+    if (tid == 0)
+        for (; issued < kFxStages && issued < ntiles; ++issued) request(issued);
+
+    const int group0 = blockIdx.x * 32;
+    const int ti = a.tgt_start + min(group0 + lane, a.n_tgt - 1);
+    long long X[3];
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        ok = fx_position(a.xt[3 * (size_t)ti + c], a.K.pos_scale, fx_origin(a.xs[c], a.K.pos_scale), &X[c]) && ok;
+    const bool warp_ok = __all_sync(0xffffffffu, ok);
+    double tot[NOUT];
+#pragma unroll
+    for (int c = 0; c < NOUT; ++c) tot[c] = 0.0;
+
+    bool timed_out = false;
+    int t = 0;
+    for (; t < ntiles; ++t) {
+        const int s = t % kFxStages;
+        const bool arrived = mbar_wait_bounded(&bars[s], (t / kFxStages) & 1, a.wait_ns);
+        if (__syncthreads_or(!arrived)) {
+            timed_out = true;
+            break;
+        }
+        // every thread has finished tile t - 1: its stage can be refilled
+        if (tid == 0 && t >= 1 && issued < ntiles) request(issued++);
+        const int j0 = j_begin + t * kFxTile, jn = min(kFxTile, j_end - j0);
+        const int per = (jn + kFxWarps - 1) / kFxWarps, b = min(warp * per, jn), e = min(b + per, jn);
+        const unsigned long long *tile = ring[s];
+        const int E = (int)(tile[Tr::meta] >> 32);
+        if (E == kFxBadTile || !warp_ok) {
+            const FxSum r = fx_sum_fp64<KIND>(a, ti, j0 + b, j0 + e);
+#pragma unroll
+            for (int c = 0; c < NOUT; ++c) tot[c] += r.v[c];
+            continue;
+        }
+        long long H[NOUT], L[NOUT];
+#pragma unroll
+        for (int c = 0; c < NOUT; ++c) H[c] = L[c] = 0;
+#pragma unroll 1
+        for (int j = b; j < e; ++j) {
+            const FxSource src = fx_load_source<KIND>(tile + j * Tr::words);
+            fx_pair<KIND>(X, src, a.K, H, L);
+        }
+        const double scale = fx_exp2(E);
+#pragma unroll
+        for (int c = 0; c < NOUT; ++c) tot[c] += fx_fold(H[c], L[c], (c < 3 ? a.K.vscale : a.K.wscale) * scale);
+    }
+
+    if (timed_out && tid == 0) {
+        // the sums are invalid, which the error word reports; the CTA still
+        // takes its turn at the ticket, so that the next launch finds zeros
+        atomicOr(a.err, kDevErrWaitTimeout);
+        // let the copies still in flight land (bounded) before the CTA exits
+        for (int u = t; u < issued; ++u) (void)mbar_wait_bounded(&bars[u % kFxStages], (u / kFxStages) & 1);
+    }
+
+#pragma unroll
+    for (int c = 0; c < NOUT; ++c) red[warp][c][lane] = tot[c];
+    __syncthreads();
+    const int nt = min(32, a.n_tgt - group0);
+    const size_t base = (size_t)group0 * NOUT, count = (size_t)a.n_tgt * NOUT;
+    for (int o = tid; o < nt * NOUT; o += kFxTpb) {
+        const int i = o / NOUT, c = o - i * NOUT;
+        const double v = (red[0][c][i] + red[1][c][i]) + (red[2][c][i] + red[3][c][i]);
+        if (a.partial != nullptr)
+            a.partial[blockIdx.y * count + base + o] = v;
+        else
+            a.out[base + o] = a.accumulate ? a.out[base + o] + v : v;
+    }
+    if (a.partial == nullptr || a.tickets == nullptr) return;
+    // the last split of this target group adds the group's partial sums
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) is_last = atomicAdd(a.tickets + blockIdx.x, 1) == (int)gridDim.y - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int o = tid; o < nt * NOUT; o += kFxTpb) {
+        double v = a.accumulate ? a.out[base + o] : 0.0;
+        for (int p = 0; p < (int)gridDim.y; ++p) v += __ldcg(a.partial + p * count + base + o);
+        a.out[base + o] = v;
+    }
+    if (tid == 0) a.tickets[blockIdx.x] = 0;
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+static int words_of(int kind) { return (kind == kSS || kind == kBS) ? 10 : 8; }
+static int nout_of(int kind) { return (kind == kBB || kind == kBS) ? 3 : 6; }
+
+size_t fx_record_bytes(int kind) { return (size_t)words_of(kind) * 8; }
+
+bool fx_supported(int kind, double as, double ab, double mu)
+{
+    FxConsts K;
+    return kind != kSSWall && fx_consts(kind, as, ab, mu, &K);
+}
+
+using FxPairFn = void (*)(FxLaunch);
+using FxPackFn = void (*)(const double *, const double *, int, FxConsts, unsigned long long *, const int *);
+
+static FxPairFn pair_fn(int kind)
+{
+    return kind == kSS ? rpy_fx_kernel<kFxSS> : kind == kBB ? rpy_fx_kernel<kFxBB>
+         : kind == kSB ? rpy_fx_kernel<kFxSB> : rpy_fx_kernel<kFxBS>;
+}
+static FxPackFn pack_fn(int kind)
+{
+    return kind == kSS ? fx_pack_kernel<kFxSS> : kind == kBB ? fx_pack_kernel<kFxBB>
+         : kind == kSB ? fx_pack_kernel<kFxSB> : fx_pack_kernel<kFxBS>;
+}
+
+// Sources per split, a power of two from a quarter tile up.  Measured on M_ss
+// and M_bb of 100 to 12,800 particles (152 SMs): with work enough, the
+// largest split that still gives 24 CTAs per SM, so that the last CTAs to
+// finish idle the chip for little of the launch (4096 blobs: 128 sources 232
+// us, 256 240, 1024 287; 12,800 segments: 1024 sources 3.92 ms, 128 3.95);
+// below that whole tiles while they give 13 (3000 segments: 128 262 us, 64
+// 275), then half and quarter tiles, whose CTAs have less to do than to set
+// up (962 segments: 64 55 us, 32 59; 642: 32 33 us, 64 37, 128 43).
+static int fx_chunk(int groups, int n_src, int sm_count, int most_splits)
+{
+    const auto splits = [&](long long chunk) { return ((long long)n_src + chunk - 1) / chunk; };
+    const auto ctas = [&](long long chunk) { return (double)groups * (double)splits(chunk) / sm_count; };
+    long long chunk = kFxTile;
+    if (ctas(kFxTile) >= 24.0)
+        while (ctas(2 * chunk) >= 24.0) chunk *= 2;
+    else if (ctas(kFxTile) < 13.0)
+        chunk = ctas(kFxTile / 2) >= 2.7 ? kFxTile / 2 : kFxTile / 4;
+    while (splits(chunk) > std::min(most_splits, 65535)) chunk *= 2;
+    return (int)std::min<long long>(chunk, 1 << 30);
+}
+
+static cudaError_t launch_fx(const void *fn, dim3 grid, int block, void **params, cudaStream_t stream, bool pdl)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelExC(&cfg, fn, params);
+}
+
+int fx_splits(int n_tgt, int n_src, int sm_count)
+{
+    if (n_tgt <= 0 || n_src <= 0) return 1;
+    const int chunk = fx_chunk((n_tgt + 31) / 32, n_src, sm_count, 1 << 20);
+    return (n_src + chunk - 1) / chunk;
+}
+
+gmi_status launch_pair_fx(const FxPairSum &s, int *launched)
+{
+    *launched = 0;
+    if (s.splits_out) *s.splits_out = 1;
+    if (s.n_tgt <= 0) return GMI_OK;
+    const int nout = nout_of(s.kind);
+    if (s.n_src <= 0) {
+        if (!s.accumulate)
+            GMI_CUDA_TRY(cudaMemsetAsync(s.out, 0, (size_t)s.n_tgt * nout * sizeof(double), s.stream));
+        return GMI_OK;
+    }
+    FxLaunch a{};
+    if (!fx_consts(s.kind, s.as, s.ab, s.mu, &a.K)) {
+        set_last_error_msg("launch_pair_fx: radii outside the fixed-point formats");
+        return GMI_ERR_ARG;
+    }
+    PairConsts c;
+    fill_consts(c, s.as, s.as, s.ab, s.mu);
+    a.eq = EqualK<double>{c.eq[0], c.eq[1], c.eq[2], c.eq[3], c.eq[4], c.eq[5], c.eq[6], c.eq[7], c.eq[8]};
+    a.uq = UnequalK<double>{c.uq[0], c.uq[1], c.uq[2], c.uq[3], c.uq[4],  c.uq[5], c.uq[6],
+                            c.uq[7], c.uq[8], c.uq[9], c.uq[10], c.uq[11], c.uq[12]};
+    const int groups = (s.n_tgt + 31) / 32;
+    const size_t per_split = (size_t)s.n_tgt * nout * sizeof(double);
+    int most = (int)std::min<size_t>(s.partial_bytes / per_split, 1 << 20);
+    if (s.max_splits > 0) most = std::min(most, s.max_splits);
+    a.chunk = fx_chunk(groups, s.n_src, s.sm_count, std::max(1, most));
+    const int splits = (s.n_src + a.chunk - 1) / a.chunk;
+    a.xt = s.xt;
+    a.xs = s.xs;
+    a.fs = s.fs;
+    a.rec = static_cast<const unsigned long long *>(s.rec);
+    a.tgt_start = s.tgt_start;
+    a.n_tgt = s.n_tgt;
+    a.n_src = s.n_src;
+    a.out = s.out;
+    a.partial = splits > 1 ? s.partial : nullptr;
+    a.tickets = s.splits_out ? nullptr : s.tickets;
+    a.accumulate = s.accumulate;
+    a.err = s.err;
+    a.skip = s.skip;
+    a.wait_ns = s.wait_ns;
+    int n = s.n_src;
+    unsigned long long *rec = static_cast<unsigned long long *>(s.rec);
+    void *pack_params[] = {const_cast<double **>(&a.xs), const_cast<double **>(&a.fs), &n, &a.K, &rec, &a.skip};
+    GMI_CUDA_TRY(launch_fx(reinterpret_cast<const void *>(pack_fn(s.kind)), dim3((n + kFxTile - 1) / kFxTile), kFxTile,
+                           pack_params, s.stream, s.pdl != 0));
+    void *params[] = {&a};
+    GMI_CUDA_TRY(launch_fx(reinterpret_cast<const void *>(pair_fn(s.kind)), dim3(groups, splits), kFxTpb, params,
+                           s.stream, s.pdl != 0));
+    *launched = 2;
+    if (s.splits_out) *s.splits_out = splits;
+    return GMI_OK;
+}
+
+}  // namespace gmi

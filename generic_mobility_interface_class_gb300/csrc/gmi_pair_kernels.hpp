@@ -61,6 +61,13 @@ gmi_status launch_pair(gmi_context *ctx, int kind, const void *tgt_rec, int tgt_
                        int n_src, const PairConsts &k, double *out, int accumulate,
                        const PairShape *force_shape = nullptr);
 
+// The same from positions and loads (AoS FP64): the reference-shaped sums of
+// the C ABI and the solver.  xt: the n_all_tgt positions of the target set;
+// as, ab: segment and blob radius (kinds within one set: its radius twice).
+gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt, int tgt_start, int n_tgt,
+                    const double *xs, const double *fs, int n_src, double as, double ab, double mu, double *out,
+                    int accumulate);
+
 gmi_status launch_barrier(gmi_context *ctx, const BarrierLaunch &a);
 
 // Whether a kernel exists for this shape, kind and precision, and whether the

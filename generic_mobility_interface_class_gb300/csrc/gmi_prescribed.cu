@@ -561,23 +561,17 @@ gmi_status prescribed_solve(gmi_solver *s, const double *body_x, const double *b
     ctx->launches += 2;
     GMI_CUDA_TRY(cudaGetLastError());
 
-    PairConsts kss, ksb, kbb;
-    fill_consts(kss, s->cfg.rseg, s->cfg.rseg, s->cfg.rseg, s->cfg.mu);
-    fill_consts(ksb, s->cfg.rseg, s->cfg.rseg, s->cfg.rblob, s->cfg.mu);
-    fill_consts(kbb, s->cfg.rblob, s->cfg.rblob, s->cfg.rblob, s->cfg.mu);
+    const double as = s->cfg.rseg, ab = s->cfg.rblob, mu = s->cfg.mu;
     DeviceApply matvec = [&](const double *in, double *out) -> gmi_status {
         pk_expand<<<blocks(S), kTpb, 0, st>>>(S, in, pw->f6);
         ctx->launches++;
         // segments with their forces; M_ss onto segments, M_bs onto blobs
-        GMI_TRY(pack_records(ctx, s->x_segs, pw->f6, 6, S, ctx->rec_src));
-        GMI_TRY(launch_pair(ctx, kSS, ctx->rec_src.ptr, 0, S, ctx->rec_src.ptr, S, kss, s->v_segs, 0));
-        GMI_TRY(pack_records(ctx, s->x_blobs, nullptr, 0, B, ctx->rec_tgt));
-        GMI_TRY(launch_pair(ctx, kBS, ctx->rec_tgt.ptr, 0, B, ctx->rec_src.ptr, S, ksb, s->v_blobs, 0));
+        GMI_TRY(pair_sum(ctx, kSS, s->x_segs, S, 0, S, s->x_segs, pw->f6, S, as, as, mu, s->v_segs, 0));
+        GMI_TRY(pair_sum(ctx, kBS, s->x_blobs, B, 0, B, s->x_segs, pw->f6, S, as, ab, mu, s->v_blobs, 0));
         // blobs with their forces; M_bb onto blobs, M_sb onto segments
-        GMI_TRY(pack_records(ctx, s->x_blobs, in + 3 * (size_t)S, 3, B, ctx->rec_src));
-        GMI_TRY(launch_pair(ctx, kBB, ctx->rec_src.ptr, 0, B, ctx->rec_src.ptr, B, kbb, s->v_blobs, 1));
-        GMI_TRY(pack_records(ctx, s->x_segs, nullptr, 0, S, ctx->rec_tgt));
-        GMI_TRY(launch_pair(ctx, kSB, ctx->rec_tgt.ptr, 0, S, ctx->rec_src.ptr, B, ksb, s->v_segs, 1));
+        const double *fb = in + 3 * (size_t)S;
+        GMI_TRY(pair_sum(ctx, kBB, s->x_blobs, B, 0, B, s->x_blobs, fb, B, ab, ab, mu, s->v_blobs, 1));
+        GMI_TRY(pair_sum(ctx, kSB, s->x_segs, S, 0, S, s->x_blobs, fb, B, as, ab, mu, s->v_segs, 1));
         pk_rows<false><<<blocks(S + B), kTpb, 0, st>>>(z, in, s->v_segs, s->v_blobs, s->x_segs, s->body_x, s->R,
                                                        s->refs, seg_mob, blob_mob, in + uoff, pw->vel_dir, pw->fil7,
                                                        nullptr, out);

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "gmi_context.hpp"
+#include "gmi_fx_kernels.hpp"
 #include "gmi_pair_kernels.hpp"
 #include "gmi_solver_device.cuh"
 #include "gmi_solver_internal.hpp"
@@ -649,7 +650,7 @@ __global__ void __launch_bounds__(kSBlobs) s2_precond_blobs_kernel(
     z[3 * i] = o[0];
     z[3 * i + 1] = o[1];
     z[3 * i + 2] = o[2];
-    pack_record(rec, (int)i, xb + 3 * i, o, f64);
+    if (rec != nullptr) pack_record(rec, (int)i, xb + 3 * i, o, f64);
 }
 
 // Column sums out[i * ostride] = sum over b < count of p[i * stride + b],
@@ -1136,10 +1137,8 @@ static gmi_status system_matrix_mult(gmi_solver *s, const double *in, double *ou
 {
     const int nb = s->B;
     gmi_context *ctx = s->ctx;
-    GMI_TRY(pack_records(ctx, s->x_blobs, in, 3, nb, ctx->rec_src));
-    PairConsts k;
-    fill_consts(k, s->cfg.rblob, s->cfg.rblob, s->cfg.rblob, s->cfg.mu);
-    GMI_TRY(launch_pair(ctx, kBB, ctx->rec_src.ptr, 0, nb, ctx->rec_src.ptr, nb, k, s->mbb, 0));
+    GMI_TRY(pair_sum(ctx, kBB, s->x_blobs, nb, 0, nb, s->x_blobs, in, nb, s->cfg.rblob, s->cfg.rblob, s->cfg.mu,
+                     s->mbb, 0));
     GMI_TRY(kt_sums(s, in));
     sysmult_finish_kernel<<<grid_for(nb + 6 * s->W), 256, 0, ctx->stream>>>(s->W, s->cfg.nblob, s->mbb, in + 3 * nb,
                                                                            s->sums, s->R, s->refs, out);
@@ -1269,10 +1268,12 @@ static gmi_status enqueue_arnoldi_step(gmi_solver *s, cudaGraphConditionalHandle
                              nblob, s->Q, ld, s->w, (const double *)s->R, (const double *)s->refs,
                              (const double *)s->ktk_rot, (const double *)s->mob_rot, (const double *)s->ktkf_rot,
                              minv, s->z, part, (const double *)s->st_scal, tk, (const GmresCtl *)s->ctl));
+    // FP64: the fixed-point pair sum packs its own records from z
+    const bool fx = f64 && std::getenv("GMI_GM_PAIR") == nullptr && fx_supported(kBB, s->cfg.rblob, s->cfg.rblob, s->cfg.mu);
     GMI_CUDA_TRY(launch_step(pdl, s2_precond_blobs_kernel, dim3((nblob + kSBlobs - 1) / kSBlobs, W), dim3(kSBlobs),
                              0, st, W, nblob, (const double *)s->Q, ld, (const double *)s->R,
-                             (const double *)s->refs, minv, (const double *)s->x_blobs, s->z, s->gm_rec,
-                             f64 ? 1 : 0, (const GmresCtl *)s->ctl));
+                             (const double *)s->refs, minv, (const double *)s->x_blobs, s->z,
+                             fx ? (void *)nullptr : s->gm_rec, f64 ? 1 : 0, (const GmresCtl *)s->ctl));
     ExplicitPairEnv env{};
     env.stream = st;
     env.partial = s->gm_partial;
@@ -1309,7 +1310,30 @@ static gmi_status enqueue_arnoldi_step(gmi_solver *s, cudaGraphConditionalHandle
     fill_consts(k, s->cfg.rblob, s->cfg.rblob, s->cfg.rblob, s->cfg.mu);
     int splits = 1;
     env.splits_out = &splits;  // S3 adds the split partials
-    GMI_TRY(launch_pair_into(env, kBB, f64, s->gm_rec, 0, nb, s->gm_rec, nb, k, s->mbb, 0));
+    if (fx) {
+        FxPairSum p{};
+        p.stream = st;
+        p.sm_count = ctx->sm_count;
+        p.kind = kBB;
+        p.xt = p.xs = s->x_blobs;
+        p.fs = s->z;
+        p.n_tgt = p.n_src = nb;
+        p.as = p.ab = s->cfg.rblob;
+        p.mu = s->cfg.mu;
+        p.out = s->mbb;
+        p.rec = s->gm_rec;
+        p.partial = s->gm_partial;
+        p.partial_bytes = s->gm_partial_bytes;
+        p.err = ctx->d_err;
+        p.skip = &s->ctl->done;
+        p.splits_out = &splits;
+        p.pdl = pdl ? 1 : 0;
+        p.wait_ns = ctx->wait_ns;
+        int launched_fx = 0;
+        GMI_TRY(launch_pair_fx(p, &launched_fx));
+    } else {
+        GMI_TRY(launch_pair_into(env, kBB, f64, s->gm_rec, 0, nb, s->gm_rec, nb, k, s->mbb, 0));
+    }
     GMI_CUDA_TRY(launch_step(pdl, s3_finish_project_kernel, dim3(L.nblk), dim3(kSTpb), 0, st, W, nblob,
                              (const double *)s->mbb, (const double *)s->gm_partial, splits, (const double *)s->z,
                              (const double *)s->R, (const double *)s->refs, s->w, (const double *)s->Q, ld, n, P,
@@ -1854,28 +1878,15 @@ gmi_status solver_place_blobs(gmi_solver *s, const double *body_x, const double 
 static gmi_status seg_pair(gmi_solver *s, int kind)
 {
     gmi_context *ctx = s->ctx;
-    PairConsts k;
-    if (kind == kSS) {
-        GMI_TRY(pack_records(ctx, s->x_segs, s->f_segs, 6, s->S, ctx->rec_src));
-        fill_consts(k, s->cfg.rseg, s->cfg.rseg, s->cfg.rseg, s->cfg.mu);
-        return launch_pair(ctx, s->cfg.wall ? kSSWall : kSS, ctx->rec_src.ptr, 0, s->S, ctx->rec_src.ptr, s->S, k,
-                           s->v_segs, 0);
-    }
-    if (kind == kBS) {
-        GMI_TRY(pack_records(ctx, s->x_blobs, nullptr, 0, s->B, ctx->rec_tgt));
-        GMI_TRY(pack_records(ctx, s->x_segs, s->f_segs, 6, s->S, ctx->rec_src));
-        fill_consts(k, s->cfg.rseg, s->cfg.rseg, s->cfg.rblob, s->cfg.mu);
-        return launch_pair(ctx, kBS, ctx->rec_tgt.ptr, 0, s->B, ctx->rec_src.ptr, s->S, k, s->v_blobs, 0);
-    }
-    if (kind == kSB) {
-        GMI_TRY(pack_records(ctx, s->x_segs, nullptr, 0, s->S, ctx->rec_tgt));
-        GMI_TRY(pack_records(ctx, s->x_blobs, s->f_blobs, 3, s->B, ctx->rec_src));
-        fill_consts(k, s->cfg.rseg, s->cfg.rseg, s->cfg.rblob, s->cfg.mu);
-        return launch_pair(ctx, kSB, ctx->rec_tgt.ptr, 0, s->S, ctx->rec_src.ptr, s->B, k, s->v_segs, 1);
-    }
-    GMI_TRY(pack_records(ctx, s->x_blobs, s->f_blobs, 3, s->B, ctx->rec_src));
-    fill_consts(k, s->cfg.rblob, s->cfg.rblob, s->cfg.rblob, s->cfg.mu);
-    return launch_pair(ctx, kBB, ctx->rec_src.ptr, 0, s->B, ctx->rec_src.ptr, s->B, k, s->v_blobs, 0);
+    const double as = s->cfg.rseg, ab = s->cfg.rblob, mu = s->cfg.mu;
+    if (kind == kSS)
+        return pair_sum(ctx, s->cfg.wall ? kSSWall : kSS, s->x_segs, s->S, 0, s->S, s->x_segs, s->f_segs, s->S, as, as,
+                        mu, s->v_segs, 0);
+    if (kind == kBS)
+        return pair_sum(ctx, kBS, s->x_blobs, s->B, 0, s->B, s->x_segs, s->f_segs, s->S, as, ab, mu, s->v_blobs, 0);
+    if (kind == kSB)
+        return pair_sum(ctx, kSB, s->x_segs, s->S, 0, s->S, s->x_blobs, s->f_blobs, s->B, as, ab, mu, s->v_segs, 1);
+    return pair_sum(ctx, kBB, s->x_blobs, s->B, 0, s->B, s->x_blobs, s->f_blobs, s->B, ab, ab, mu, s->v_blobs, 0);
 }
 
 static gmi_status h2d(gmi_solver *s, double *d, const double *h, size_t count)
@@ -2090,7 +2101,8 @@ gmi_status gmi_solver_create(const gmi_solver_config *cfg, gmi_solver **out)
         s->ctl = reinterpret_cast<GmresCtl *>(ctl_mem);
         TRY_OR_DIE(dalloc(s, &rec_mem, 12 * B));
         s->gm_rec = rec_mem;
-        const size_t max_splits = (B + 127) / 128 + 1;
+        // one tile per split, or (fixed-point sum, few blobs) a quarter of one
+        const size_t max_splits = B <= 4096 ? (B + 31) / 32 + 1 : (B + 127) / 128 + 1;
         TRY_OR_DIE(dalloc(s, &part_mem, max_splits * 3 * B));
         s->gm_partial = part_mem;
         s->gm_partial_bytes = max_splits * 3 * B * sizeof(double);

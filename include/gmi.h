@@ -7,7 +7,8 @@
  * point takes plain pointers and sizes, returns a gmi_status, and never
  * exits the process.  Device pointers are marked _d; host pointers _h.
  *
- * Precision: GMI_FP64 evaluates the pair sums in FP64 like the reference;
+ * Precision: GMI_FP64 evaluates the pair sums to FP64 accuracy (the wall in
+ * FP64 like the reference, the free-space sums in 64-bit fixed point);
  * GMI_FP32C evaluates them in FP32 with double-float source positions and
  * compensated (two-sum) accumulation, and returns FP64 results; GMI_DF64
  * (blob-blob only) carries every step of the pair formula as a double-float
@@ -37,7 +38,7 @@ typedef enum gmi_status {
 } gmi_status;
 
 typedef enum gmi_precision {
-    GMI_FP64 = 0,  /* reference arithmetic */
+    GMI_FP64 = 0,  /* the reference's accuracy */
     GMI_FP32C = 1, /* FP32 pair math, compensated accumulation, FP64 I/O */
     GMI_DF64 = 2   /* double-float (FP32 hi/lo pairs) pair math, ~1e-13, FP64 I/O;
                       gmi_Mbb_mult only (other pair sums return GMI_ERR_ARG) */
@@ -161,6 +162,8 @@ GMI_API gmi_status gmi_barrier_forces(gmi_context *ctx, double *f_segs_d, double
 
 /* Autotuner: time the candidate launch shapes of one pair kernel for the
  * given sizes on the context's GPU and keep the fastest for later calls.
+ * In FP64 without a wall there is one kernel, which sizes its own splits: the
+ * call only drops a pinned shape.
  * kind: 0 = ss, 1 = ss wall, 2 = bb, 3 = sb, 4 = bs. */
 GMI_API gmi_status gmi_autotune(gmi_context *ctx, int kind, int num_targets, int num_sources);
 /* The launch shape the context will use for this kernel and size:

@@ -1,0 +1,114 @@
+"""The fixed-point pair arithmetic (csrc/gmi_pairs_fx.cuh) against the FP64
+oracle, on the host: the formulas are plain integer C++ there and on the GPU.
+
+Tolerance: a term of the fixed-point sum is rounded at 2^-56 of its load, so
+the difference is the oracle's own, whose sums of n FP64 terms are each within
+n 2^-53 of the terms' size; n 2^-52 of the largest velocity is allowed.
+"""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT, rel_err
+
+KINDS = {"ss": 0, "bb": 2, "sb": 3, "bs": 4}
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fx") / "fx_host.so")
+    csrc = os.path.join(ROOT, "generic_mobility_interface_class_gb300", "csrc")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-x", "c++", "-I", csrc,
+                    os.path.join(ROOT, "tests", "fx_host.cpp"), "-o", so], check=True)
+    lib = ctypes.CDLL(so)
+    d, p = ctypes.c_double, ctypes.c_void_p
+    lib.fx_host_sum.argtypes = [ctypes.c_int, ctypes.c_int, p, ctypes.c_int, p, p, d, d, d, p]
+    return lib
+
+
+def fx_sum(lib, kind, xt, xs, f, a, b, mu=1.0):
+    xt, xs, f = (np.ascontiguousarray(v) for v in (xt, xs, f))
+    out = np.zeros((len(xt), 6 if kind in ("ss", "sb") else 3))
+    status = lib.fx_host_sum(KINDS[kind], len(xt), xt.ctypes.data, len(xs), xs.ctypes.data, f.ctypes.data, a, b, mu,
+                             out.ctypes.data)
+    return status, out
+
+
+def oracle_sum(rpy, kind, xt, xs, f, a, b, mu=1.0):
+    if kind == "ss":
+        return rpy.mss(xs, f, a, mu)
+    if kind == "bb":
+        return rpy.mbb(xs, f, a, mu)
+    if kind == "sb":
+        return rpy.msb(xt, xs, f, a, b, mu)
+    return rpy.mbs(xt, xs, f, a, b, mu)
+
+
+def in_range(xt, xs, radius):
+    """Positions lie within 512 U of the first source rounded to 256 U, U the
+    largest power of two not above the radius."""
+    u = 2.0 ** np.floor(np.log2(radius))
+    origin = np.rint(xs[0] / (256 * u)) * (256 * u)
+    return max(np.abs(xt - origin).max(), np.abs(xs - origin).max()) < 512 * u
+
+
+def cloud(kind, layout, n, a, seed):
+    rng = np.random.default_rng(seed)
+    size = {"far": 100.0, "dense": 3.0, "wide": 250.0, "near_copies": 20.0}[layout] * a
+    xs = rng.uniform(-size, size, size=(n, 3))
+    if layout == "near_copies":  # coincident particles, and pairs 2^-1 .. 2^-58 radii apart
+        for i in range(0, n - 1, 3):
+            xs[i + 1] = xs[i] + a * np.ldexp(rng.normal(size=3), -(i % 58)) * (i % 9 > 0)
+    f = rng.normal(size=(n, 6 if kind in ("ss", "bs") else 3))
+    xt = xs if kind in ("ss", "bb") else np.concatenate([xs[:20], rng.uniform(-size, size, size=(30, 3))])
+    return xt, xs, f
+
+
+@pytest.mark.parametrize("layout", ["far", "dense", "wide", "near_copies"])
+@pytest.mark.parametrize("kind,a,b", [("ss", 1.0, 1.0), ("ss", 1.999, 1.999), ("ss", 1e-3, 1e-3), ("bb", 1.0, 1.0),
+                                      ("bb", 0.75, 0.75), ("sb", 1.0, 1.0), ("sb", 1.0, 2.0), ("sb", 1.3, 0.7),
+                                      ("bs", 1.0, 1.0), ("bs", 0.5, 1.0), ("bs", 1.0, 0.6)])
+def test_fixed_point_sums_against_oracle(host, oracle_built, kind, a, b, layout):
+    n = 333
+    xt, xs, f = cloud(kind, layout, n, max(a, b), seed=5)
+    status, got = fx_sum(host, kind, xt, xs, f, a, b, mu=1.7)
+    if not in_range(xt, xs, min(a, b)):
+        assert status == 2
+        return
+    assert status == 0
+    want = oracle_sum(oracle_built, kind, xt, xs, f, a, b, 1.7)
+    for block in range(0, want.shape[1], 3):
+        assert rel_err(got[:, block:block + 3], want[:, block:block + 3]) < n * 2.0 ** -52
+
+
+@pytest.mark.parametrize("kind", ["ss", "bb"])
+def test_loads_of_very_different_sizes(host, oracle_built, kind):
+    """Loads from 1e-9 to 1e9 in one tile, zero loads, and a whole tile of zeros."""
+    n = 400
+    xt, xs, f = cloud(kind, "far", n, 1.0, seed=6)
+    f *= 10.0 ** np.random.default_rng(7).uniform(-9, 9, size=(n, 1))
+    f[5] = 0.0
+    f[128:256] = 0.0
+    status, got = fx_sum(host, kind, xt, xs, f, 1.0, 1.0)
+    assert status == 0
+    assert rel_err(got, oracle_sum(oracle_built, kind, xt, xs, f, 1.0, 1.0)) < n * 2.0 ** -52
+
+
+def test_translation_and_range(host, oracle_built):
+    """Far from the origin the positions stay exact; a cloud too wide, loads
+    too large or not finite, and radii too different are reported."""
+    xt, xs, f = cloud("ss", "far", 200, 1.0, seed=8)
+    for shift in (1e3, 1e6, 1e9):
+        x = xs + shift * np.array([1.0, -0.7, 0.3])
+        status, got = fx_sum(host, "ss", x, x, f, 1.0, 1.0)
+        assert status == 0
+        assert rel_err(got, oracle_built.mss(x, f)) < 200 * 2.0 ** -52
+    assert fx_sum(host, "ss", 8 * xs, 8 * xs, f, 1.0, 1.0)[0] == 2
+    for bad in (np.nan, np.inf, 1e300):
+        g = f.copy()
+        g[17, 4] = bad
+        assert fx_sum(host, "ss", xs, xs, g, 1.0, 1.0)[0] == 2
+    assert fx_sum(host, "sb", xs, xs, f[:, :3], 1.0, 2.1)[0] == 1

@@ -1,0 +1,107 @@
+"""The fixed-point pair kernel (FP64 precision, no wall) at the edges of its
+tiles, splits and formats, against the FP64 oracle.
+
+Tolerance: as test_pairs_fx_cpu.py, n 2^-52 of the largest velocity (the
+oracle's own rounding over n terms), and 2^-50 at least.
+"""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def T(a):
+    return torch.as_tensor(np.ascontiguousarray(a), device="cuda")
+
+
+def N(t):
+    return t.detach().cpu().numpy()
+
+
+def tol(n):
+    return max(n * 2.0 ** -52, 2.0 ** -50)
+
+
+def cloud(n, seed):
+    rng = np.random.default_rng(seed)
+    x = rng.uniform(0.0, 2.6 * max(n, 8) ** (1 / 3), size=(n, 3))
+    return x, rng.normal(size=(n, 6))
+
+
+def check_all(ctx, rpy, xs, fs, xb, fb, b=1.3, bound=None):
+    bound = tol(len(xs) + len(xb)) if bound is None else bound
+    assert rel_err(N(ctx.mss(T(xs), T(fs))), rpy.mss(xs, fs)) < bound
+    assert rel_err(N(ctx.mbb(T(xb), T(fb))), rpy.mbb(xb, fb)) < bound
+    v = np.random.default_rng(1).normal(size=(len(xs), 6))
+    got = T(v)
+    ctx.msb(T(xs), T(xb), T(fb), got, a_blob=b)
+    assert rel_err(N(got), rpy.msb(xs, xb, fb, 1.0, b, v_in=v)) < bound
+    assert rel_err(N(ctx.mbs(T(xb), T(xs), T(fs), a_blob=b)), rpy.mbs(xb, xs, fs, 1.0, b)) < bound
+
+
+@pytest.mark.parametrize("ns,nb", [(1, 1), (31, 2), (32, 33), (33, 127), (127, 128), (129, 257), (320, 642),
+                                   (963, 1281), (3001, 2047)])
+def test_sizes_against_oracle(gpu_ctx, oracle_built, ns, nb):
+    xs, fs = cloud(ns, 3)
+    xb, fb = cloud(nb, 4)
+    gpu_ctx.set_precision(0)
+    check_all(gpu_ctx, oracle_built, xs, fs, xb, fb[:, :3])
+
+
+def test_tiles_outside_the_formats(gpu_ctx, oracle_built):
+    """A particle far out (its tile, and it as a target, in FP64), a huge load
+    (its tile), the others beside them in fixed point."""
+    xs, fs = cloud(700, 5)
+    xb, fb = cloud(500, 6)
+    xs[300] += 5000.0
+    xb[60] -= 2.0e5
+    fs[40, 2] = 1e295
+    gpu_ctx.set_precision(0)
+    check_all(gpu_ctx, oracle_built, xs, fs, xb, fb[:, :3])
+
+
+def test_not_finite_loads_and_positions(gpu_ctx, oracle_built):
+    """A NaN load reaches every target, an infinite one too; a NaN position
+    its own row and, as a source, all."""
+    xs, fs = cloud(300, 7)
+    gpu_ctx.set_precision(0)
+    bad = fs.copy()
+    bad[200, 1] = np.nan
+    assert np.isnan(N(gpu_ctx.mss(T(xs), T(bad)))[:, :3]).all()
+    bad[200, 1] = np.inf
+    assert not np.isfinite(N(gpu_ctx.mss(T(xs), T(bad)))[:, :3]).any()
+    x = xs.copy()
+    x[10, 0] = np.nan
+    assert np.isnan(N(gpu_ctx.mss(T(x), T(fs)))).all()
+
+
+def test_slices_and_radii_ratio(gpu_ctx, oracle_built):
+    """Target slices that start inside a group of 32, and radii whose ratio
+    the formats do not hold (the FP64 kernels)."""
+    rpy = oracle_built
+    xs, fs = cloud(900, 8)
+    xb, fb = cloud(400, 9)
+    gpu_ctx.set_precision(0)
+    got = N(gpu_ctx.mss(T(xs), T(fs), start=45, num=333))
+    assert rel_err(got, rpy.mss(xs, fs)[45:378]) < tol(900)
+    for b in (0.5, 2.0, 0.3, 5.0):
+        check_all(gpu_ctx, rpy, xs, fs, xb, fb[:, :3], b=b)
+
+
+def test_pinned_fp64_shape_keeps_its_kernel(gmi_lib, oracle_built):
+    """A shape pinned in FP64 runs the FP64 kernel of that shape."""
+    from generic_mobility_interface_class_gb300.mobility import Context
+    xs, fs = cloud(700, 10)
+    with Context(0) as ctx:
+        auto = N(ctx.mss(T(xs), T(fs)))
+        ctx.set_shape(0, 700, 700, 64, 1, 3, 1)
+        assert ctx.tuned_shape(0, 700, 700) == (64, 1, 3, True)
+        pinned = N(ctx.mss(T(xs), T(fs)))
+        assert rel_err(pinned, auto) < tol(700)
+        ctx.autotune(0, 700, 700)
+        assert ctx.tuned_shape(0, 700, 700)[3]
+        np.testing.assert_array_equal(N(ctx.mss(T(xs), T(fs))), auto)
