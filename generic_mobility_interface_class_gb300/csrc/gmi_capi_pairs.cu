@@ -258,8 +258,8 @@ gmi_status gmi_autotune(gmi_context *ctx, int kind, int num_targets, int num_sou
     GMI_ARG_CHECK(num_targets > 0 && num_sources > 0, "gmi_autotune: sizes must be positive");
     gmi_status st = select_device(ctx);
     if (st != GMI_OK) return st;
-    if (ctx->precision == GMI_FP64 && kind != kSSWall) {
-        // one kernel, which sizes its own splits: nothing to time
+    if (ctx->precision == GMI_FP64) {
+        // one kernel a kind, which sizes its own splits: nothing to time
         PairShape fx;
         fx.tt = 1;
         fx.packed = 0;

@@ -28,7 +28,7 @@ struct PairShape {
     int tt = 2;        // targets per thread
     int splits = 0;    // source splits; 0 = choose from the SM count
     int packed = -1;   // two sources per thread step (FP32, no wall): 1 yes, 0 no, -1 where available
-    bool fx = false;   // the fixed-point kernel (FP64, no wall), which chooses its own splits
+    bool fx = false;   // FP64: the fixed-point or the wall kernel, which choose their own splits
 };
 
 enum PairKind : int { kSS = 0, kSSWall = 1, kBB = 2, kSB = 3, kBS = 4 };

@@ -27,6 +27,7 @@
 #include "gmi_df.cuh"
 #include "gmi_fx_kernels.hpp"
 #include "gmi_pair_kernels.hpp"
+#include "gmi_wall_kernel.hpp"
 
 namespace gmi {
 
@@ -1738,57 +1739,72 @@ gmi_status launch_pair(gmi_context *ctx, int kind, const void *tgt_rec, int tgt_
 }
 
 // One pair sum of positions and loads in the reference's layouts, by the
-// kernel of the context's precision.  FP64 without a wall takes the
-// fixed-point kernel, at every size: against the FP64 kernels M_ss of 320
+// kernel of the context's precision.  FP64 takes the wall kernel or, without a
+// wall, the fixed-point kernel, at every size: against the FP64 kernels M_ss of 320
 // segments went from 61 to 22.5 us, of 12,800 from 20.4 to 3.9 ms, M_bb of
-// 4096 blobs from 1222 to 231 us.  The FP64 kernels keep the wall, radii that
-// the fixed-point formats do not hold, and shapes pinned by gmi_set_shape.
+// 4096 blobs from 1222 to 231 us.  The FP64 kernels keep radii that the
+// fixed-point formats do not hold, and shapes pinned by gmi_set_shape.
 gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt, int tgt_start, int n_tgt,
                     const double *xs, const double *fs, int n_src, double as, double ab, double mu, double *out,
                     int accumulate)
 {
-    if (ctx->precision == GMI_FP64 && fx_supported(kind, as, ab, mu)) {
-        const auto it = ctx->tuned.find(TuneKey{kind, GMI_FP64, n_tgt, n_src});
-        if (it == ctx->tuned.end() || it->second.fx) {
-            FxPairSum s{};
-            s.max_splits = fx_splits(n_tgt, n_src, ctx->sm_count);
-            // one buffer: tickets, records, partial sums (a first call then
-            // allocates once: 30 us each)
-            const auto round = [](size_t b) { return (b + 255) / 256 * 256; };
-            const size_t tickets = std::max<size_t>(round(((size_t)std::max(n_tgt, 0) + 31) / 32 * sizeof(int)), 65536);
-            const size_t records = round((size_t)std::max(n_src, 0) * fx_record_bytes(kind));
-            s.partial_bytes = s.max_splits > 1 ? (size_t)s.max_splits * n_tgt * nout_of(kind) * sizeof(double) : 0;
-            const size_t had = ctx->fx.bytes;
-            GMI_TRY(ctx->fx.reserve(std::max(tickets, ctx->fx_tickets) + records + s.partial_bytes));
-            if (ctx->fx.bytes != had || tickets > ctx->fx_tickets) {
-                GMI_CUDA_TRY(cudaMemsetAsync(ctx->fx.ptr, 0, tickets, ctx->stream));
-                ctx->fx_tickets = tickets;
-            }
-            unsigned char *mem = static_cast<unsigned char *>(ctx->fx.ptr);
-            s.tickets = reinterpret_cast<int *>(mem);
-            s.rec = mem + ctx->fx_tickets;
-            s.partial = reinterpret_cast<double *>(mem + ctx->fx_tickets + records);
-            s.stream = ctx->stream;
-            s.sm_count = ctx->sm_count;
-            s.kind = kind;
-            s.xt = xt;
+    const auto it = ctx->tuned.find(TuneKey{kind, ctx->precision, n_tgt, n_src});
+    const bool pinned = it != ctx->tuned.end() && !it->second.fx;
+    const bool wall = kind == kSSWall;
+    if (ctx->precision == GMI_FP64 && !pinned && n_tgt > 0 && n_src > 0 && (wall || fx_supported(kind, as, ab, mu))) {
+        // one buffer: tickets, records, partial sums (a first call then
+        // allocates once: 30 us each)
+        const int splits = wall ? wall_splits(n_tgt, n_src, ctx->sm_count) : fx_splits(n_tgt, n_src, ctx->sm_count);
+        const auto round = [](size_t b) { return (b + 255) / 256 * 256; };
+        const size_t tickets = std::max<size_t>(round(((size_t)n_tgt + 31) / 32 * sizeof(int)), 65536);
+        const size_t records = wall ? 0 : round((size_t)n_src * fx_record_bytes(kind));
+        const size_t partial = splits > 1 ? (size_t)splits * n_tgt * nout_of(kind) * sizeof(double) : 0;
+        const size_t had = ctx->fx.bytes;
+        GMI_TRY(ctx->fx.reserve(std::max(tickets, ctx->fx_tickets) + records + partial));
+        if (ctx->fx.bytes != had || tickets > ctx->fx_tickets) {
+            ctx->fx_tickets = std::max(tickets, ctx->fx_tickets);
+            GMI_CUDA_TRY(cudaMemsetAsync(ctx->fx.ptr, 0, ctx->fx_tickets, ctx->stream));
+        }
+        unsigned char *mem = static_cast<unsigned char *>(ctx->fx.ptr);
+        if (wall) {
+            WallSum s{};
+            s.x = xs;
+            s.f = fs;
             s.tgt_start = tgt_start;
             s.n_tgt = n_tgt;
-            s.xs = xs;
-            s.fs = fs;
             s.n_src = n_src;
-            s.as = as;
-            s.ab = ab;
-            s.mu = mu;
             s.out = out;
-            s.accumulate = accumulate;
-            s.err = ctx->d_err;
-            s.wait_ns = ctx->wait_ns;
-            int launched = 0;
-            const gmi_status st = launch_pair_fx(s, &launched);
-            ctx->launches += launched;
-            return st;
+            s.tickets = reinterpret_cast<int *>(mem);
+            s.partial = reinterpret_cast<double *>(mem + ctx->fx_tickets);
+            ctx->launches++;
+            return launch_wall_fp64(ctx->stream, ctx->sm_count, s);
         }
+        FxPairSum s{};
+        s.max_splits = splits;
+        s.partial_bytes = partial;
+        s.tickets = reinterpret_cast<int *>(mem);
+        s.rec = mem + ctx->fx_tickets;
+        s.partial = reinterpret_cast<double *>(mem + ctx->fx_tickets + records);
+        s.stream = ctx->stream;
+        s.sm_count = ctx->sm_count;
+        s.kind = kind;
+        s.xt = xt;
+        s.tgt_start = tgt_start;
+        s.n_tgt = n_tgt;
+        s.xs = xs;
+        s.fs = fs;
+        s.n_src = n_src;
+        s.as = as;
+        s.ab = ab;
+        s.mu = mu;
+        s.out = out;
+        s.accumulate = accumulate;
+        s.err = ctx->d_err;
+        s.wait_ns = ctx->wait_ns;
+        int launched = 0;
+        const gmi_status st = launch_pair_fx(s, &launched);
+        ctx->launches += launched;
+        return st;
     }
     const int nf = (kind == kBB || kind == kSB) ? 3 : 6;
     const bool same = kind == kSS || kind == kSSWall || kind == kBB;

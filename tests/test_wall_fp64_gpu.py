@@ -1,0 +1,33 @@
+"""The FP64 wall kernel at the edges of its target groups and source splits,
+against the FP64 oracle.
+
+Tolerance: a pair's coefficients come from some 40 rounded operations whose
+terms are up to about ten times the pair's own velocity near the wall, so
+2^-44 of the largest velocity.
+"""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def T(a):
+    return torch.as_tensor(np.ascontiguousarray(a), device="cuda")
+
+
+@pytest.mark.parametrize("n", [1, 4, 31, 33, 129, 320, 1281, 2999])
+def test_wall_sizes_against_oracle(gpu_ctx, oracle_built, n):
+    rng = np.random.default_rng(n)
+    side = 3.0 * max(n, 4) ** (1 / 3)
+    x = rng.uniform(0.0, side, size=(n, 3)) + np.array([0.0, 0.0, 1.05])
+    f = rng.normal(size=(n, 6))
+    gpu_ctx.set_precision(0)
+    want = oracle_built.mss_wall(x, f)
+    assert rel_err(gpu_ctx.mss_wall(T(x), T(f)).cpu().numpy(), want) < 2.0 ** -44
+    if n > 300:  # a slice of the targets, not on a group's edge
+        got = gpu_ctx.mss_wall(T(x), T(f), start=37, num=211).cpu().numpy()
+        assert rel_err(got, want[37:248]) < 2.0 ** -44
