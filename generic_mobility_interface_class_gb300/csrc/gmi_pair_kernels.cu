@@ -527,9 +527,9 @@ constexpr int kTilePairs = kTile / 2;
 
 template <int KIND>
 __device__ __forceinline__ void pair2_apply(float2 dx, float2 dy, float2 dz, const float2 *F,
-                                            const KernelConsts<float> &K, float2 *p, float2 *m)
+                                            const KernelConsts<float> &K, const SSCoeffs &self, float2 *p, float2 *m)
 {
-    if constexpr (KIND == kSS) pair2_ss(dx, dy, dz, F, K.eq, p, m);
+    if constexpr (KIND == kSS) pair2_ss(dx, dy, dz, F, K.eq, self, p, m);
     if constexpr (KIND == kBB) pair2_bb(dx, dy, dz, F, K.eq, p);
     if constexpr (KIND == kSB) pair2_sb(dx, dy, dz, F, K.uq, p, m);
     if constexpr (KIND == kBS) pair2_bs(dx, dy, dz, F, K.uq, p, m);
@@ -579,6 +579,8 @@ __global__ void __launch_bounds__(TPB) rpy_pair2_kernel(const __grid_constant__ 
     const float load_scale = (KIND == kSB || KIND == kBS) ? K.uq.f8pm : K.eq.f8pm;
     const float *tgt_rec = reinterpret_cast<const float *>(args.tgt_rec);
     float2 th[TT][3], tl[TT][3];  // target position (hi, lo), both lanes
+    SSCoeffs self{};
+    if constexpr (KIND == kSS) self = ss_self2(K.eq);
     int ti[TT];
     float2 p[TT][NOUT], m[TT][NOUT];
     float hi[TT][NOUT], lo[TT][NOUT];
@@ -651,7 +653,7 @@ __global__ void __launch_bounds__(TPB) rpy_pair2_kernel(const __grid_constant__ 
                 const float2 dx = add2(add2(th[k][0], nxh), add2(tl[k][0], nxl));
                 const float2 dy = add2(add2(th[k][1], nyh), add2(tl[k][1], nyl));
                 const float2 dz = add2(add2(th[k][2], nzh), add2(tl[k][2], nzl));
-                pair2_apply<KIND>(dx, dy, dz, F, K, p[k], m[k]);
+                pair2_apply<KIND>(dx, dy, dz, F, K, self, p[k], m[k]);
             }
         }
         // tile sum of both lanes, plus minus minus, folded by two-sum

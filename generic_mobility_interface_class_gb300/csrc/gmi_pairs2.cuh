@@ -62,6 +62,15 @@ static __device__ __noinline__ SSCoeffs ss_near2(float r2, float ir, float dF, f
     return c;
 }
 
+// The self pair's coefficients, those of ss_near2 at r = 0 (dF = dT = 0, and
+// the others meet d = 0): taken once per thread.  Every target meets itself
+// once, in a step that ss_near2 made ten times as long as the others; 2501
+// segments (40 CTAs with a diagonal tile of 800) took 31 us, the last 15 for them.
+__device__ __forceinline__ SSCoeffs ss_self2(const EqualK<float> &k)
+{
+    return ss_near2(kTinyR2, rsq_raw(kTinyR2), 0.0f, 0.0f, k);
+}
+
 struct UnequalCoeffs {
     float A, Bd, Cd;
 };
@@ -78,7 +87,7 @@ static __device__ __noinline__ UnequalCoeffs unequal_near2(float r2, float ir, f
 // segment <- segment, 6 -> 6 (pair_ss).  F[0..2] force, F[3..5] torque.
 // p[0..2] / m[0..2]: velocity plus / minus parts, p[3..5] / m[3..5]: angular.
 __device__ __forceinline__ void pair2_ss(float2 dx, float2 dy, float2 dz, const float2 *F, const EqualK<float> &k,
-                                         float2 *p, float2 *m)
+                                         const SSCoeffs &self, float2 *p, float2 *m)
 {
     const float2 r2 = dist2(dx, dy, dz);
     const float2 ir = rsq2(r2);
@@ -94,11 +103,11 @@ __device__ __forceinline__ void pair2_ss(float2 dx, float2 dy, float2 dz, const 
     float2 Br = mul2(mul2(c3, ir2), mul2(bc2(1.5f), dT));      // 3 dT / (2 r^5)
     if (!(fminf(r2.x, r2.y) > k.four_a2)) {  // one test per step; near pairs are rare
         if (!(r2.x > k.four_a2)) {
-            const SSCoeffs c = ss_near2(r2.x, ir.x, dF.x, dT.x, k);
+            const SSCoeffs c = r2.x == kTinyR2 ? self : ss_near2(r2.x, ir.x, dF.x, dT.x, k);
             At.x = c.At; Bt.x = c.Bt; Ar.x = c.Ar; Br.x = c.Br; c3.x = c.c3;
         }
         if (!(r2.y > k.four_a2)) {
-            const SSCoeffs c = ss_near2(r2.y, ir.y, dF.y, dT.y, k);
+            const SSCoeffs c = r2.y == kTinyR2 ? self : ss_near2(r2.y, ir.y, dF.y, dT.y, k);
             At.y = c.At; Bt.y = c.Bt; Ar.y = c.Ar; Br.y = c.Br; c3.y = c.c3;
         }
     }
