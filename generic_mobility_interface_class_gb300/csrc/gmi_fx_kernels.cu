@@ -1,15 +1,15 @@
 // gmi_fx_kernels.cu -- the FP64-grade free-space pair sums (precision
 // GMI_FP64) in 64-bit fixed point.
 //
-// Two kernels per sum.  The pack kernel turns the sources into integer
+// Two kernels per sum, or one for small sums.  The pack kernel turns the sources into integer
 // records (gmi_pairs_fx.cuh), one CTA per tile of 128 with the tile's
 // exponent found by a block maximum.  In the pair kernel a CTA owns 32
 // targets, one per lane, and a contiguous slice ("split") of the sources,
 // staged tile by tile into shared memory by bulk copies; its four warps take
 // a quarter of each tile each, fold their integer sums into FP64 per tile
 // and meet in shared memory at the end.  32 targets per CTA rather than 128
-// let a few hundred targets reach every SM.  With several splits the last CTA
-// of a target group to finish adds the group's partial sums in split order.
+// let a few hundred targets reach every SM.  With several splits reduce_splits
+// adds the partial sums in split order.
 //
 // A tile whose loads or positions the formats do not hold (not finite, a load
 // beyond 2^+-900, a particle further than about 400 radii from the first
@@ -39,6 +39,7 @@ constexpr int kFxTile = 128;   // sources per tile: one exponent, one stage
 constexpr int kFxTpb = 128;    // four warps
 constexpr int kFxWarps = kFxTpb / 32;
 constexpr int kFxStages = 2;
+constexpr int kFxInlinePerSm = 4;  // CTAs per SM up to which a CTA packs its own sources
 constexpr int kFxBadTile = -0x7fffffff;  // in place of a tile's exponent: sum it in FP64
 static_assert(kFxTile == kFxWarps * kFxFold, "a warp's quarter of a tile is one fold");
 
@@ -55,7 +56,6 @@ struct FxLaunch {
     const unsigned long long *rec;
     int tgt_start, n_tgt, n_src, chunk;
     double *out, *partial;
-    int *tickets;  // non-null: the last CTA of a target group adds the partials
     int accumulate;
     unsigned *err;
     const int *skip;
@@ -65,68 +65,90 @@ struct FxLaunch {
     UnequalK<double> uq;
 };
 
+// One source on its way into a record: its position, its loads (torques over
+// U) and their exponent.
+template <int KIND> struct FxPacking {
+    long long X[3];
+    double F[FxTraits<KIND>::nf];
+    int e;
+};
+constexpr int kFxMark = 0x7fffffff;  // as an exponent: the formats do not hold this source
+
+template <int KIND>
+__device__ __forceinline__ FxPacking<KIND> fx_read_source(const double *__restrict__ x, const double *__restrict__ f,
+                                                          int i, const FxConsts &K)
+{
+    using Tr = FxTraits<KIND>;
+    FxPacking<KIND> p;
+    double mx = 0.0;
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        ok = fx_position(x[3 * (size_t)i + c], K.pos_scale, fx_origin(x[c], K.pos_scale), &p.X[c]) && ok;
+#pragma unroll
+    for (int c = 0; c < Tr::nf; ++c) {
+        p.F[c] = f[Tr::nf * (size_t)i + c] * (c < 3 ? 1.0 : K.inv_unit);
+        // the larger magnitude by its bits: a NaN or infinity stays the largest
+        mx = __longlong_as_double(max(__double_as_longlong(mx), __double_as_longlong(fabs(p.F[c]))));
+    }
+    ok = fx_load_exponent(mx, &p.e) && ok;
+    if (!ok) p.e = kFxMark;
+    return p;
+}
+
+// The largest exponent of a CTA of kFxTpb threads, one source each.
+__device__ __forceinline__ int fx_block_max(int e, int *wmax)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = e;
+    __syncthreads();
+    e = wmax[0];
+#pragma unroll
+    for (int w = 1; w < kFxWarps; ++w) e = max(e, wmax[w]);
+    return e;
+}
+
+// The record of a source in a tile whose largest exponent is E.
+template <int KIND>
+__device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E, unsigned long long *r)
+{
+    using Tr = FxTraits<KIND>;
+    const bool bad = E == kFxMark;
+    int gap = 0, used = 0;
+    if (!bad && p.e != kFxNoLoad) {
+        gap = min(E - p.e, kFxMaxGap);
+        used = E - gap;
+    }
+    const double scale = bad ? 0.0 : fx_exp2(-used);
+    const int meta = bad ? kFxBadTile : E == kFxNoLoad ? 0 : E;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        r[c] = (unsigned long long)p.X[c];
+        const fx l = fx_split(bad ? 0 : fx_from_double(p.F[c] * scale));
+        r[3 + c] = ((unsigned long long)(unsigned)l.hi << 32) | (unsigned)l.lo;
+    }
+    if constexpr (Tr::torque) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) r[6 + c] = bad ? 0ull : (unsigned long long)fx_from_double(p.F[3 + c] * scale);
+    }
+    r[Tr::meta] = ((unsigned long long)(unsigned)meta << 32) | (unsigned)gap;
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(kFxTile) fx_pack_kernel(const double *__restrict__ x, const double *__restrict__ f,
                                                           int n, FxConsts K, unsigned long long *__restrict__ rec,
                                                           const int *skip)
 {
-    using Tr = FxTraits<KIND>;
-    __shared__ int wmax[kFxTile / 32];
+    __shared__ int wmax[kFxWarps];
     pdl_wait_then_release();
     if (skip != nullptr && *skip != 0) return;
-    const int i = blockIdx.x * kFxTile + threadIdx.x, lane = threadIdx.x & 31;
-    long long X[3] = {0, 0, 0};
-    double F[Tr::nf];
-    int e = kFxNoLoad;
-    bool ok = true;
-#pragma unroll
-    for (int c = 0; c < Tr::nf; ++c) F[c] = 0.0;
-    if (i < n) {
-        double mx = 0.0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            ok = fx_position(x[3 * (size_t)i + c], K.pos_scale, fx_origin(x[c], K.pos_scale), &X[c]) && ok;
-#pragma unroll
-        for (int c = 0; c < Tr::nf; ++c) {
-            F[c] = f[Tr::nf * (size_t)i + c] * (c < 3 ? 1.0 : K.inv_unit);
-            // the larger magnitude by its bits: a NaN or infinity stays the largest
-            mx = __longlong_as_double(max(__double_as_longlong(mx), __double_as_longlong(fabs(F[c]))));
-        }
-        ok = fx_load_exponent(mx, &e) && ok;
-    }
-    // the tile's exponent, or its mark
-    int v = ok ? e : 0x7fffffff;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) wmax[threadIdx.x >> 5] = v;
-    __syncthreads();
-    int E = wmax[0];
-#pragma unroll
-    for (int w = 1; w < kFxTile / 32; ++w) E = max(E, wmax[w]);
-    if (i >= n) return;
-    int gap = 0, used = 0;
-    if (E == 0x7fffffff) {
-        E = kFxBadTile;
-#pragma unroll
-        for (int c = 0; c < Tr::nf; ++c) F[c] = 0.0;
-    } else if (E == kFxNoLoad) {
-        E = 0;
-    } else if (e != kFxNoLoad) {
-        gap = min(E - e, kFxMaxGap);
-        used = E - gap;
-    }
-    const double scale = fx_exp2(-used);
-    unsigned long long *r = rec + (size_t)i * Tr::words;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        r[c] = (unsigned long long)X[c];
-        const fx l = fx_split(fx_from_double(F[c] * scale));
-        r[3 + c] = ((unsigned long long)(unsigned)l.hi << 32) | (unsigned)l.lo;
-    }
-    if (Tr::torque)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) r[6 + c] = (unsigned long long)fx_from_double(F[3 + c] * scale);
-    r[Tr::meta] = ((unsigned long long)(unsigned)E << 32) | (unsigned)gap;
+    const int i = blockIdx.x * kFxTile + threadIdx.x;
+    FxPacking<KIND> p;
+    p.e = kFxNoLoad;
+    if (i < n) p = fx_read_source<KIND>(x, f, i, K);
+    const int E = fx_block_max(p.e, wmax);
+    if (i < n) fx_write_record<KIND>(p, E, rec + (size_t)i * FxTraits<KIND>::words);
 }
 
 struct FxSum {
@@ -187,7 +209,9 @@ __device__ __forceinline__ void bulk_load(void *smem_dst, const void *src, unsig
                  : "memory");
 }
 
-template <int KIND>
+// kInline: no pack kernel ran; the split is at most one tile, whose records the
+// CTA makes itself.
+template <int KIND, bool kInline>
 __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(const __grid_constant__ FxLaunch a)
 {
     using Tr = FxTraits<KIND>;
@@ -195,19 +219,21 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
     __shared__ __align__(128) unsigned long long ring[kFxStages][kFxTile * Tr::words];
     __shared__ double red[kFxWarps][NOUT][33];
     __shared__ uint64_t bars[kFxStages];
-    __shared__ int is_last;
+    __shared__ int wmax[kFxWarps];
 
     pdl_wait();
     if (a.skip != nullptr && *a.skip != 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int j_begin = blockIdx.y * a.chunk, j_end = min(j_begin + a.chunk, a.n_src);
     const int ntiles = (j_end - j_begin + kFxTile - 1) / kFxTile;
-    if (tid == 0) {
+    if (!kInline) {
+        if (tid == 0) {
 #pragma unroll
-        for (int s = 0; s < kFxStages; ++s) mbar_init(&bars[s], 1);
-        fence_mbar_init();
+            for (int s = 0; s < kFxStages; ++s) mbar_init(&bars[s], 1);
+            fence_mbar_init();
+        }
+        __syncthreads();
     }
-    __syncthreads();
     int issued = 0;  // tiles requested so far (meaningful on thread 0)
     const auto request = [&](int t) {
         const int j0 = j_begin + t * kFxTile;
@@ -215,8 +241,17 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
         mbar_arrive_expect_tx(&bars[t % kFxStages], bytes);
         bulk_load(ring[t % kFxStages], a.rec + (size_t)j0 * Tr::words, bytes, &bars[t % kFxStages]);
     };
-    if (tid == 0)
+    if (!kInline && tid == 0)
         for (; issued < kFxStages && issued < ntiles; ++issued) request(issued);
+    if (kInline) {
+        FxPacking<KIND> p;
+        p.e = kFxNoLoad;
+        const int i = j_begin + tid;
+        if (i < j_end) p = fx_read_source<KIND>(a.xs, a.fs, i, a.K);
+        const int E = fx_block_max(p.e, wmax);
+        if (i < j_end) fx_write_record<KIND>(p, E, ring[0] + tid * Tr::words);
+        __syncthreads();
+    }
 
     const int group0 = blockIdx.x * 32;
     const int ti = a.tgt_start + min(group0 + lane, a.n_tgt - 1);
@@ -234,13 +269,15 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
     int t = 0;
     for (; t < ntiles; ++t) {
         const int s = t % kFxStages;
-        const bool arrived = mbar_wait_bounded(&bars[s], (t / kFxStages) & 1, a.wait_ns);
-        if (__syncthreads_or(!arrived)) {
-            timed_out = true;
-            break;
+        if (!kInline) {
+            const bool arrived = mbar_wait_bounded(&bars[s], (t / kFxStages) & 1, a.wait_ns);
+            if (__syncthreads_or(!arrived)) {
+                timed_out = true;
+                break;
+            }
+            // every thread has finished tile t - 1: its stage can be refilled
+            if (tid == 0 && t >= 1 && issued < ntiles) request(issued++);
         }
-        // every thread has finished tile t - 1: its stage can be refilled
-        if (tid == 0 && t >= 1 && issued < ntiles) request(issued++);
         const int j0 = j_begin + t * kFxTile, jn = min(kFxTile, j_end - j0);
         const int per = (jn + kFxWarps - 1) / kFxWarps, b = min(warp * per, jn), e = min(b + per, jn);
         const unsigned long long *tile = ring[s];
@@ -264,12 +301,13 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
         for (int c = 0; c < NOUT; ++c) tot[c] += fx_fold(H[c], L[c], (c < 3 ? a.K.vscale : a.K.wscale) * scale);
     }
 
-    if (timed_out && tid == 0) {
-        // the sums are invalid, which the error word reports; the CTA still
-        // takes its turn at the ticket, so that the next launch finds zeros
-        atomicOr(a.err, kDevErrWaitTimeout);
-        // let the copies still in flight land (bounded) before the CTA exits
-        for (int u = t; u < issued; ++u) (void)mbar_wait_bounded(&bars[u % kFxStages], (u / kFxStages) & 1);
+    if (timed_out) {
+        if (tid == 0) {
+            atomicOr(a.err, kDevErrWaitTimeout);
+            // let the copies still in flight land (bounded) before the CTA exits
+            for (int u = t; u < issued; ++u) (void)mbar_wait_bounded(&bars[u % kFxStages], (u / kFxStages) & 1);
+        }
+        return;
     }
 
 #pragma unroll
@@ -285,20 +323,6 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
         else
             a.out[base + o] = a.accumulate ? a.out[base + o] + v : v;
     }
-    if (a.partial == nullptr || a.tickets == nullptr) return;
-    // the last split of this target group adds the group's partial sums
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) is_last = atomicAdd(a.tickets + blockIdx.x, 1) == (int)gridDim.y - 1;
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    for (int o = tid; o < nt * NOUT; o += kFxTpb) {
-        double v = a.accumulate ? a.out[base + o] : 0.0;
-        for (int p = 0; p < (int)gridDim.y; ++p) v += __ldcg(a.partial + p * count + base + o);
-        a.out[base + o] = v;
-    }
-    if (tid == 0) a.tickets[blockIdx.x] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -318,10 +342,10 @@ bool fx_supported(int kind, double as, double ab, double mu)
 using FxPairFn = void (*)(FxLaunch);
 using FxPackFn = void (*)(const double *, const double *, int, FxConsts, unsigned long long *, const int *);
 
-static FxPairFn pair_fn(int kind)
+template <bool kInline> static FxPairFn pair_fn(int kind)
 {
-    return kind == kSS ? rpy_fx_kernel<kFxSS> : kind == kBB ? rpy_fx_kernel<kFxBB>
-         : kind == kSB ? rpy_fx_kernel<kFxSB> : rpy_fx_kernel<kFxBS>;
+    return kind == kSS ? rpy_fx_kernel<kFxSS, kInline> : kind == kBB ? rpy_fx_kernel<kFxBB, kInline>
+         : kind == kSB ? rpy_fx_kernel<kFxSB, kInline> : rpy_fx_kernel<kFxBS, kInline>;
 }
 static FxPackFn pack_fn(int kind)
 {
@@ -329,14 +353,15 @@ static FxPackFn pack_fn(int kind)
          : kind == kSB ? fx_pack_kernel<kFxSB> : fx_pack_kernel<kFxBS>;
 }
 
-// Sources per split, a power of two from a quarter tile up.  Measured on M_ss
-// and M_bb of 100 to 12,800 particles (152 SMs): with work enough, the
-// largest split that still gives 24 CTAs per SM, so that the last CTAs to
-// finish idle the chip for little of the launch (4096 blobs: 128 sources 232
-// us, 256 240, 1024 287; 12,800 segments: 1024 sources 3.92 ms, 128 3.95);
-// below that whole tiles while they give 13 (3000 segments: 128 262 us, 64
-// 275), then half and quarter tiles, whose CTAs have less to do than to set
-// up (962 segments: 64 55 us, 32 59; 642: 32 33 us, 64 37, 128 43).
+// Sources per split, a power of two.  Measured on M_ss and M_bb of 60 to
+// 12,800 particles (152 SMs): with work enough, the largest split that still
+// gives 24 CTAs per SM, so that the last CTAs to finish idle the chip for
+// little of the launch (4096 blobs: 128 sources 232 us, 256 240, 1024 287;
+// 12,800 segments: 1024 sources 3.92 ms, 128 3.95); below that whole tiles
+// while they give 13 (3000 segments: 128 262 us, 64 275), then parts of a tile,
+// whose CTAs have less to do than to set up: 64 or 32 (962 segments: 64 49 us,
+// 32 51; 642: 32 29 us, 64 33, 128 39), and 16 or 8 while the CTAs still find an
+// SM each (100 blobs: 8 10.3 us, 32 12.3; 320 segments: 32 20.5 us, 8 24.6).
 static int fx_chunk(int groups, int n_src, int sm_count, int most_splits)
 {
     const auto splits = [&](long long chunk) { return ((long long)n_src + chunk - 1) / chunk; };
@@ -345,23 +370,9 @@ static int fx_chunk(int groups, int n_src, int sm_count, int most_splits)
     if (ctas(kFxTile) >= 24.0)
         while (ctas(2 * chunk) >= 24.0) chunk *= 2;
     else if (ctas(kFxTile) < 13.0)
-        chunk = ctas(kFxTile / 2) >= 2.7 ? kFxTile / 2 : kFxTile / 4;
+        chunk = ctas(64) >= 2.7 ? 64 : ctas(8) <= 1.2 ? 8 : ctas(16) <= 1.2 ? 16 : 32;
     while (splits(chunk) > std::min(most_splits, 65535)) chunk *= 2;
     return (int)std::min<long long>(chunk, 1 << 30);
-}
-
-static cudaError_t launch_fx(const void *fn, dim3 grid, int block, void **params, cudaStream_t stream, bool pdl)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(block);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelExC(&cfg, fn, params);
 }
 
 int fx_splits(int n_tgt, int n_src, int sm_count)
@@ -407,21 +418,29 @@ gmi_status launch_pair_fx(const FxPairSum &s, int *launched)
     a.n_src = s.n_src;
     a.out = s.out;
     a.partial = splits > 1 ? s.partial : nullptr;
-    a.tickets = s.splits_out ? nullptr : s.tickets;
     a.accumulate = s.accumulate;
     a.err = s.err;
     a.skip = s.skip;
     a.wait_ns = s.wait_ns;
-    int n = s.n_src;
-    unsigned long long *rec = static_cast<unsigned long long *>(s.rec);
-    void *pack_params[] = {const_cast<double **>(&a.xs), const_cast<double **>(&a.fs), &n, &a.K, &rec, &a.skip};
-    GMI_CUDA_TRY(launch_fx(reinterpret_cast<const void *>(pack_fn(s.kind)), dim3((n + kFxTile - 1) / kFxTile), kFxTile,
-                           pack_params, s.stream, s.pdl != 0));
-    void *params[] = {&a};
-    GMI_CUDA_TRY(launch_fx(reinterpret_cast<const void *>(pair_fn(s.kind)), dim3(groups, splits), kFxTpb, params,
-                           s.stream, s.pdl != 0));
-    *launched = 2;
-    if (s.splits_out) *s.splits_out = splits;
+    // a CTA packs its own sources where the packing kernel and its boundary
+    // (5 us) cost more than packing each tile once per target group
+    const bool packs_itself = a.chunk <= kFxTile && (long long)groups * splits <= kFxInlinePerSm * s.sm_count;
+    *launched = packs_itself ? 1 : 2;
+    if (!packs_itself)
+        GMI_CUDA_TRY(launch_chained(s.pdl != 0, pack_fn(s.kind), dim3((s.n_src + kFxTile - 1) / kFxTile), dim3(kFxTile),
+                                    s.stream, a.xs, a.fs, s.n_src, a.K, static_cast<unsigned long long *>(s.rec), a.skip));
+    GMI_CUDA_TRY(launch_chained(s.pdl != 0 || !packs_itself, packs_itself ? pair_fn<true>(s.kind) : pair_fn<false>(s.kind),
+                                dim3(groups, splits), dim3(kFxTpb), s.stream, a));
+    if (s.splits_out) {
+        *s.splits_out = splits;
+    } else if (splits > 1) {
+        // a kernel of its own: the last CTA of a target group adding the
+        // group's partials took 2 us longer (320 segments: 18.5, 16.4 us)
+        const int count = s.n_tgt * nout;
+        GMI_CUDA_TRY(launch_chained(true, reduce_splits, dim3((count + 255) / 256), dim3(256), s.stream, a.partial, splits,
+                                    count, a.out, a.accumulate, nullptr));
+        ++*launched;
+    }
     return GMI_OK;
 }
 

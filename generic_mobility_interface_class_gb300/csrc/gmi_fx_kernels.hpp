@@ -21,12 +21,11 @@ struct FxPairSum {
     void *rec;                     // n_src records of fx_record_bytes(kind)
     double *partial;               // split partial sums
     size_t partial_bytes;          // bounds the number of splits
-    int *tickets;                  // (n_tgt + 31) / 32 zeros, left zero
     unsigned *err;
     const int *skip;               // optional device flag: non-zero makes both kernels no-ops
     int *splits_out;               // optional: the caller adds the split partials (partial[p * 3 n_tgt + e],
                                    // p < *splits_out) itself; 1: the kernel wrote `out`
-    int pdl;                       // launch for programmatic dependent launch
+    int pdl;                       // the first kernel too may start while the previous one on the stream ends
     unsigned long long wait_ns;
     int max_splits;                // 0: no cap beyond the automatic choice
 };
@@ -36,7 +35,7 @@ bool fx_supported(int kind, double as, double ab, double mu);
 size_t fx_record_bytes(int kind);
 // The source splits of the automatic choice (it sizes `partial`).
 int fx_splits(int n_tgt, int n_src, int sm_count);
-// Packs the sources and sums; two launches (*launched counts them).
+// Packs the sources and sums, in one to three launches (*launched counts them).
 gmi_status launch_pair_fx(const FxPairSum &s, int *launched);
 
 }  // namespace gmi

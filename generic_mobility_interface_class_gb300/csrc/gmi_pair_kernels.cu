@@ -41,6 +41,7 @@ constexpr int kStages = 4;   // depth of the shared-memory ring
 __global__ void pack_records_f32(const double *__restrict__ x, const double *__restrict__ f, int nf, int n,
                                  float4 *__restrict__ rec)
 {
+    pdl_wait_then_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double px = x[3 * i], py = x[3 * i + 1], pz = x[3 * i + 2];
@@ -70,6 +71,7 @@ __global__ void pack_records_f32(const double *__restrict__ x, const double *__r
 __global__ void pack_records_df(const double *__restrict__ x, const double *__restrict__ f, int n,
                                 float4 *__restrict__ rec)
 {
+    pdl_wait_then_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const df2 px = df_from_double(x[3 * i] - x[0]), py = df_from_double(x[3 * i + 1] - x[1]),
@@ -89,6 +91,7 @@ __global__ void pack_records_df(const double *__restrict__ x, const double *__re
 __global__ void pack_records_f64(const double *__restrict__ x, const double *__restrict__ f, int nf, int n,
                                  double2 *__restrict__ rec)
 {
+    pdl_wait_then_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double f0 = 0, f1 = 0, f2 = 0, t0 = 0, t1 = 0, t2 = 0;
@@ -483,6 +486,7 @@ __global__ void __launch_bounds__(TPB) rpy_bb_df_kernel(const __grid_constant__ 
 __global__ void __launch_bounds__(128) rpy_bb_df_warp_kernel(const PairLaunch args, const float4 *__restrict__ src,
                                                              const DfBBConsts K)
 {
+    pdl_wait();
     const int t = (int)((blockIdx.x * 128u + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (t >= args.n_tgt) return;
     const float4 *tr = reinterpret_cast<const float4 *>(args.tgt_rec) + 3 * (size_t)(args.tgt_start + t);
@@ -575,12 +579,12 @@ __global__ void __launch_bounds__(TPB) rpy_pair2_kernel(const __grid_constant__ 
     }
 
     const KernelConsts<float> K = convert_consts<float>(args.k);
+    SSCoeffs self{};
+    if constexpr (KIND == kSS) self = ss_self2(K.eq);
     // loads enter the packed formulas times 1/(8 pi mu) (gmi_pairs2.cuh)
     const float load_scale = (KIND == kSB || KIND == kBS) ? K.uq.f8pm : K.eq.f8pm;
     const float *tgt_rec = reinterpret_cast<const float *>(args.tgt_rec);
     float2 th[TT][3], tl[TT][3];  // target position (hi, lo), both lanes
-    SSCoeffs self{};
-    if constexpr (KIND == kSS) self = ss_self2(K.eq);
     int ti[TT];
     float2 p[TT][NOUT], m[TT][NOUT];
     float hi[TT][NOUT], lo[TT][NOUT];
@@ -701,6 +705,7 @@ __global__ void __launch_bounds__(TPB) rpy_pair2_kernel(const __grid_constant__ 
 __global__ void reduce_splits(const double *__restrict__ partial, int splits, int count,
                               double *__restrict__ out, int accumulate, const int *skip)
 {
+    pdl_wait();
     if (skip != nullptr && *skip != 0) return;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
@@ -1341,7 +1346,8 @@ void fill_consts(PairConsts &c, double a_eq, double as, double ab, double mu)
     c.uq[12] = dmin;
 }
 
-gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int nf, int n, DeviceBuffer &buf)
+gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int nf, int n, DeviceBuffer &buf,
+                        bool chained)
 {
     if (ctx->precision == GMI_DF64) {
         if (nf != 3) {
@@ -1351,9 +1357,9 @@ gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int 
         gmi_status st = buf.reserve(n > 0 ? (size_t)n * kRecLen * sizeof(float) : 16);
         if (st != GMI_OK) return st;
         if (n == 0) return GMI_OK;
-        pack_records_df<<<(n + 255) / 256, 256, 0, ctx->stream>>>(x, f, n, static_cast<float4 *>(buf.ptr));
+        GMI_CUDA_TRY(launch_chained(chained, pack_records_df, dim3((n + 255) / 256), dim3(256), ctx->stream, x, f, n,
+                                    static_cast<float4 *>(buf.ptr)));
         ctx->launches++;
-        GMI_CUDA_TRY(cudaGetLastError());
         return GMI_OK;
     }
     const bool f64 = ctx->precision == GMI_FP64;
@@ -1364,11 +1370,12 @@ gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int 
     const int tpb = 256;
     const int grid = (n + tpb - 1) / tpb;
     if (f64)
-        pack_records_f64<<<grid, tpb, 0, ctx->stream>>>(x, f, nf, n, static_cast<double2 *>(buf.ptr));
+        GMI_CUDA_TRY(launch_chained(chained, pack_records_f64, dim3(grid), dim3(tpb), ctx->stream, x, f, nf, n,
+                                    static_cast<double2 *>(buf.ptr)));
     else
-        pack_records_f32<<<grid, tpb, 0, ctx->stream>>>(x, f, nf, n, static_cast<float4 *>(buf.ptr));
+        GMI_CUDA_TRY(launch_chained(chained, pack_records_f32, dim3(grid), dim3(tpb), ctx->stream, x, f, nf, n,
+                                    static_cast<float4 *>(buf.ptr)));
     ctx->launches++;
-    GMI_CUDA_TRY(cudaGetLastError());
     return GMI_OK;
 }
 
@@ -1588,9 +1595,9 @@ static gmi_status launch_bb_df(gmi_context *ctx, const void *tgt_rec, int tgt_st
         a.out = out;
         a.accumulate = accumulate;
         const unsigned ctas = (unsigned)(((long long)n_tgt * 32 + 127) / 128);
-        rpy_bb_df_warp_kernel<<<ctas, 128, 0, ctx->stream>>>(a, static_cast<const float4 *>(src_rec), K);
+        GMI_CUDA_TRY(launch_chained(true, rpy_bb_df_warp_kernel, dim3(ctas), dim3(128), ctx->stream, a,
+                                    static_cast<const float4 *>(src_rec), K));
         ctx->launches++;
-        GMI_CUDA_TRY(cudaGetLastError());
         return GMI_OK;
     }
     void *fn = reinterpret_cast<void *>(&rpy_bb_df_kernel<kDfTpb>);
@@ -1628,14 +1635,13 @@ static gmi_status launch_bb_df(gmi_context *ctx, const void *tgt_rec, int tgt_st
     gmi_status st = make_record_map(ctx, &map, src_rec, n_src, false);
     if (st != GMI_OK) return st;
     void *params[] = {&map, &a, &K};
-    GMI_CUDA_TRY(cudaLaunchKernel(fn, dim3(n_tgt_ctas, splits), dim3(kDfTpb), params, smem, ctx->stream));
+    GMI_CUDA_TRY(launch_fn(fn, dim3(n_tgt_ctas, splits), dim3(kDfTpb), params, smem, ctx->stream, true));
     ctx->launches++;
     if (splits > 1) {
         const int count = n_tgt * 3;
-        reduce_splits<<<(count + 255) / 256, 256, 0, ctx->stream>>>(a.partial, splits, count, out, accumulate,
-                                                                    nullptr);
+        GMI_CUDA_TRY(launch_chained(true, reduce_splits, dim3((count + 255) / 256), dim3(256), ctx->stream, a.partial,
+                                    splits, count, out, accumulate, nullptr));
         ctx->launches++;
-        GMI_CUDA_TRY(cudaGetLastError());
     }
     return GMI_OK;
 }
@@ -1687,7 +1693,7 @@ gmi_status launch_pair(gmi_context *ctx, int kind, const void *tgt_rec, int tgt_
         a.accumulate = accumulate;
         a.err = ctx->d_err;
         a.wait_ns = ctx->wait_ns;
-        const gmi_status ws = launch_warp(ctx->stream, kind, f64, shape.tt, a, src_rec);
+        const gmi_status ws = launch_warp(ctx->stream, kind, f64, shape.tt, a, src_rec, true);
         if (ws == GMI_OK) ctx->launches++;
         return ws;
     }
@@ -1728,14 +1734,13 @@ gmi_status launch_pair(gmi_context *ctx, int kind, const void *tgt_rec, int tgt_
     void *params[] = {&map, &a};
     dim3 grid(n_tgt_ctas, splits);
     const size_t smem_run = (kShapes[sidx].packed != 0 && chunk <= kTile) ? ring_bytes_single_tile() : smem;
-    GMI_CUDA_TRY(cudaLaunchKernel(fn, grid, dim3(tpb), params, smem_run, ctx->stream));
+    GMI_CUDA_TRY(launch_fn(fn, grid, dim3(tpb), params, smem_run, ctx->stream, true));
     ctx->launches++;
     if (splits > 1) {
         const int count = n_tgt * nout;
-        reduce_splits<<<(count + 255) / 256, 256, 0, ctx->stream>>>(a.partial, splits, count, out, accumulate,
-                                                                    nullptr);
+        GMI_CUDA_TRY(launch_chained(true, reduce_splits, dim3((count + 255) / 256), dim3(256), ctx->stream, a.partial,
+                                    splits, count, out, accumulate, nullptr));
         ctx->launches++;
-        GMI_CUDA_TRY(cudaGetLastError());
     }
     return GMI_OK;
 }
@@ -1754,20 +1759,14 @@ gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt,
     const bool pinned = it != ctx->tuned.end() && !it->second.fx;
     const bool wall = kind == kSSWall;
     if (ctx->precision == GMI_FP64 && !pinned && n_tgt > 0 && n_src > 0 && (wall || fx_supported(kind, as, ab, mu))) {
-        // one buffer: tickets, records, partial sums (a first call then
-        // allocates once: 30 us each)
+        // one buffer for records and partial sums: a first call allocates once
+        // (30 us each)
         const int splits = wall ? wall_splits(n_tgt, n_src, ctx->sm_count) : fx_splits(n_tgt, n_src, ctx->sm_count);
-        const auto round = [](size_t b) { return (b + 255) / 256 * 256; };
-        const size_t tickets = std::max<size_t>(round(((size_t)n_tgt + 31) / 32 * sizeof(int)), 65536);
-        const size_t records = wall ? 0 : round((size_t)n_src * fx_record_bytes(kind));
+        const size_t records = wall ? 0 : ((size_t)n_src * fx_record_bytes(kind) + 255) / 256 * 256;
         const size_t partial = splits > 1 ? (size_t)splits * n_tgt * nout_of(kind) * sizeof(double) : 0;
-        const size_t had = ctx->fx.bytes;
-        GMI_TRY(ctx->fx.reserve(std::max(tickets, ctx->fx_tickets) + records + partial));
-        if (ctx->fx.bytes != had || tickets > ctx->fx_tickets) {
-            ctx->fx_tickets = std::max(tickets, ctx->fx_tickets);
-            GMI_CUDA_TRY(cudaMemsetAsync(ctx->fx.ptr, 0, ctx->fx_tickets, ctx->stream));
-        }
+        GMI_TRY(ctx->fx.reserve(records + partial));
         unsigned char *mem = static_cast<unsigned char *>(ctx->fx.ptr);
+        int launched = 0;
         if (wall) {
             WallSum s{};
             s.x = xs;
@@ -1776,17 +1775,16 @@ gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt,
             s.n_tgt = n_tgt;
             s.n_src = n_src;
             s.out = out;
-            s.tickets = reinterpret_cast<int *>(mem);
-            s.partial = reinterpret_cast<double *>(mem + ctx->fx_tickets);
-            ctx->launches++;
-            return launch_wall_fp64(ctx->stream, ctx->sm_count, s);
+            s.partial = reinterpret_cast<double *>(mem);
+            const gmi_status st = launch_wall_fp64(ctx->stream, ctx->sm_count, s, &launched);
+            ctx->launches += launched;
+            return st;
         }
         FxPairSum s{};
         s.max_splits = splits;
         s.partial_bytes = partial;
-        s.tickets = reinterpret_cast<int *>(mem);
-        s.rec = mem + ctx->fx_tickets;
-        s.partial = reinterpret_cast<double *>(mem + ctx->fx_tickets + records);
+        s.rec = mem;
+        s.partial = reinterpret_cast<double *>(mem + records);
         s.stream = ctx->stream;
         s.sm_count = ctx->sm_count;
         s.kind = kind;
@@ -1803,7 +1801,6 @@ gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt,
         s.accumulate = accumulate;
         s.err = ctx->d_err;
         s.wait_ns = ctx->wait_ns;
-        int launched = 0;
         const gmi_status st = launch_pair_fx(s, &launched);
         ctx->launches += launched;
         return st;
@@ -1813,7 +1810,7 @@ gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt,
     PairConsts k;
     fill_consts(k, as, as, ab, mu);
     if (!same) GMI_TRY(pack_records(ctx, xt, nullptr, 0, n_all_tgt, ctx->rec_tgt));
-    GMI_TRY(pack_records(ctx, xs, fs, nf, n_src, ctx->rec_src));
+    GMI_TRY(pack_records(ctx, xs, fs, nf, n_src, ctx->rec_src, !same));
     return launch_pair(ctx, kind, same ? ctx->rec_src.ptr : ctx->rec_tgt.ptr, tgt_start, n_tgt, ctx->rec_src.ptr, n_src,
                        k, out, accumulate);
 }

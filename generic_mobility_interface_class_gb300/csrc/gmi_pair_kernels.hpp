@@ -53,7 +53,9 @@ void fill_consts(PairConsts &c, double a_eq, double a_seg, double a_blob, double
 
 // Pack AoS FP64 positions (and forces with nf = 3 or 6 components, or none
 // when f == nullptr) into the context's record format for its precision.
-gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int nf, int n, DeviceBuffer &buf);
+// `chained`: launch_chained after an earlier kernel of the same call.
+gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int nf, int n, DeviceBuffer &buf,
+                        bool chained = false);
 
 // One pair sum: out[nout*(i)] (=|+=) sum_j M(i, j) F_j for targets
 // [tgt_start, tgt_start + n_tgt).  force_shape overrides the tuned shape.
@@ -97,6 +99,10 @@ struct ExplicitPairEnv {
     int max_splits;              // cap on the source splits (0: none beyond the automatic choice)
 };
 
+// out[i] (=|+=) the sum over splits of partial[p * count + i], in split order
+// (a no-op when skip is given and set).
+__global__ void reduce_splits(const double *partial, int splits, int count, double *out, int accumulate,
+                              const int *skip);
 size_t record_bytes(bool f64);
 gmi_status pack_records_into(cudaStream_t stream, bool f64, const double *x, const double *f, int nf, int n,
                              void *dst);

@@ -12,12 +12,12 @@
 //
 // A CTA owns 32 targets, one per lane; its four warps take a quarter each of
 // a slice of the sources ("split"), sized so that every SM gets the same
-// number of CTAs to within a few per cent.  The last CTA of a target group to
-// finish adds the group's partial sums in split order.  One launch, no packing.
+// number of CTAs to within a few per cent; reduce_splits adds the splits.
 // 1280 segments: 1287 us (two targets per warp, 160 CTAs on 152 SMs, so 8 of
 // them set the time) -> 480 us, at the pipe's rate for these instructions.
 #include <algorithm>
 
+#include "gmi_pair_kernels.hpp"
 #include "gmi_wall_kernel.hpp"
 
 namespace gmi {
@@ -123,7 +123,6 @@ __global__ void __launch_bounds__(kWallTpb) rpy_wall_kernel(const WallSum a, int
 {
     __shared__ __align__(16) double src[kWallTile][10];
     __shared__ double red[kWallWarps][6][33];
-    __shared__ int is_last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int j_begin = blockIdx.y * chunk, j_end = min(j_begin + chunk, a.n_src);
     const int group0 = blockIdx.x * 32, ti = a.tgt_start + min(group0 + lane, a.n_tgt - 1);
@@ -160,20 +159,6 @@ __global__ void __launch_bounds__(kWallTpb) rpy_wall_kernel(const WallSum a, int
         else
             a.out[base + o] = t;
     }
-    if (gridDim.y == 1) return;
-    // the last split of this target group adds the group's partial sums
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) is_last = atomicAdd(a.tickets + blockIdx.x, 1) == (int)gridDim.y - 1;
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    for (int o = tid; o < nt * 6; o += kWallTpb) {
-        double t = 0.0;
-        for (int p = 0; p < (int)gridDim.y; ++p) t += __ldcg(a.partial + p * count + base + o);
-        a.out[base + o] = t;
-    }
-    if (tid == 0) a.tickets[blockIdx.x] = 0;
 }
 
 // Sources per split: the smallest power of two from 4 (one source per warp)
@@ -194,11 +179,18 @@ int wall_splits(int n_tgt, int n_src, int sm_count)
     return (n_src + chunk - 1) / chunk;
 }
 
-gmi_status launch_wall_fp64(cudaStream_t stream, int sm_count, const WallSum &a)
+gmi_status launch_wall_fp64(cudaStream_t stream, int sm_count, const WallSum &a, int *launched)
 {
-    const int chunk = wall_chunk(a.n_tgt, a.n_src, sm_count);
-    rpy_wall_kernel<<<dim3((a.n_tgt + 31) / 32, (a.n_src + chunk - 1) / chunk), kWallTpb, 0, stream>>>(a, chunk);
+    const int chunk = wall_chunk(a.n_tgt, a.n_src, sm_count), splits = (a.n_src + chunk - 1) / chunk;
+    rpy_wall_kernel<<<dim3((a.n_tgt + 31) / 32, splits), kWallTpb, 0, stream>>>(a, chunk);
     GMI_CUDA_TRY(cudaGetLastError());
+    *launched = 1;
+    if (splits > 1) {
+        const int count = a.n_tgt * 6;
+        GMI_CUDA_TRY(launch_chained(true, reduce_splits, dim3((count + 255) / 256), dim3(256), stream, a.partial, splits,
+                                    count, a.out, 0, nullptr));
+        *launched = 2;
+    }
     return GMI_OK;
 }
 

@@ -12,10 +12,10 @@ struct WallSum {
     int tgt_start, n_tgt, n_src;
     double *out;
     double *partial;  // wall_splits() * 6 n_tgt values when there are several splits
-    int *tickets;     // (n_tgt + 31) / 32 zeros, left zero
 };
 
 int wall_splits(int n_tgt, int n_src, int sm_count);
-gmi_status launch_wall_fp64(cudaStream_t stream, int sm_count, const WallSum &a);
+// One or two launches (*launched counts them).
+gmi_status launch_wall_fp64(cudaStream_t stream, int sm_count, const WallSum &a, int *launched);
 
 }  // namespace gmi
