@@ -1003,41 +1003,51 @@ __global__ void barrier_reduce(BarrierLaunch a, int splits)
 // 1.1 (a_i + a_j) (cuda_functions.cu:1031-1046, 1121-1135).  With cells at
 // least as wide as the widest screen cutoff, a target's candidates lie in
 // the 27 cells around its own.  Cell (cx, cy, cz) of a particle's FP32 screen
-// position hashes to one of T = 2^k buckets, and a counting sort (count,
-// bucket offsets, scatter) lists each bucket's particles.  Each target
-// screens the particles of its 27 buckets exactly as barrier_kernel does
-// (the same FP32 test and exclusions), keeps its candidates in shared
-// memory, sorts them by index, drops repeats (two of its cells can share a
-// bucket), and adds their FP64 forces in ascending j in one accumulator: the
-// reference's per-target order, so each force is the reference's bit for
-// bit.  A target with more than kCellCand candidates goes to an overflow
-// list, which a warp-per-target all-pairs kernel finishes in the same order.
+// position hashes to one of T = 2^k >= 2N buckets of kCellSlots entries, each
+// an entry's screen position and index, filled by an atomic count: no scan, no
+// scatter, and a search reads entries without a look at the particle.
+//
+// What bounds it is latency: a search is a chain of dependent L2 reads.  One
+// thread per target walked its 27 buckets in turn, and the kernel took 61 us
+// at 12,800 segments and 4096 blobs.  Here a CTA takes 16 targets and deals
+// their 432 (target, bucket) pairs over its 128 threads, which screen the
+// entries exactly as barrier_kernel does (the same FP32 test and exclusions)
+// and append candidates to their target's list in shared memory.  The CTA then
+// evaluates all its candidates in FP64, one per thread, places each force by
+// the rank of its index among its target's (a repeat, from two cells that
+// share a bucket, is dropped), and one thread per target and component adds
+// them in ascending j: the reference's per-target order, so each force is the
+// reference's bit for bit.  A target with more than kCellCand candidates, or
+// with a bucket that overflowed, goes to an overflow list, which a
+// warp-per-target all-pairs kernel finishes in the same order.
+// 16,896 particles: 69 us of kernels and three memsets -> 25 us of four kernels,
+// the search 61 -> 16; a call from Python 93 -> 38 us, 30 of them on the host.
 // ---------------------------------------------------------------------------
 constexpr int kCellTpb = 128;
+constexpr int kCellTargets = 16;       // targets per CTA
+constexpr int kCellSlots = 16;         // entries per bucket
 constexpr int kCellCand = 40;          // candidates per target kept in shared memory
-constexpr int kCellScanTpb = 1024;
-constexpr int kCellScanTile = 4 * kCellScanTpb;  // buckets per CTA of the offset scan
+constexpr int kCellPackTpb = 256;
 constexpr int kCellMinParticles = 8192;          // fewer particles: the all-pairs kernel
+constexpr int kCellMaxBuckets = 1 << 22;
 
 struct CellList {
-    int T;              // buckets (a power of two, a multiple of kCellScanTile)
+    int T;              // buckets (a power of two)
     float cut_max;      // widest FP32 screen cutoff before the rounding margin
-    const unsigned *extent;
-    int *count;         // [T] particles per bucket (counted down again by the scatter)
-    int *local;         // [T] exclusive scan of count within its scan tile
-    int *tile_prefix;   // [T / kCellScanTile] particles before each scan tile
-    int *order;         // [N] particles by bucket
-    int *key;           // [N] each particle's bucket
+    float *block_max;   // [ceil(N / kCellPackTpb)] largest |coordinate| of each pack CTA
+    int blocks;
+    unsigned *extent;   // largest |coordinate| of all, as FP32 bits
+    int *count;         // [T] particles per bucket
+    float4 *slot;       // [T][kCellSlots] screen position and index (as bits)
     int *overflow;      // [1 + targets]: count, then the overflowed targets (launch-local indices)
-    int *ticket;        // [1] the scan's last-CTA ticket (zero between launches)
 };
 
 // cell width: the widest screen cutoff plus the rounding margin of the
 // screen (as barrier_kernel) with 1 % to spare, so that any pair the screen
 // can accept lies in adjacent cells whatever the rounding of x / h
-__device__ __forceinline__ float cell_inv_width(const CellList &c)
+__device__ __forceinline__ float cell_inv_width(const CellList &c, float extent)
 {
-    const float margin = 1.0e-6f * __uint_as_float(*c.extent);
+    const float margin = 1.0e-6f * extent;
     return 1.0f / ((c.cut_max + margin) * 1.01f);
 }
 __device__ __forceinline__ int cell_coord(float x, float inv_h) { return (int)floorf(x * inv_h); }
@@ -1046,115 +1056,80 @@ __device__ __forceinline__ int cell_bucket(int cx, int cy, int cz, int T)
     const unsigned h = ((unsigned)cx * 73856093u) ^ ((unsigned)cy * 19349663u) ^ ((unsigned)cz * 83492791u);
     return (int)(h & (unsigned)(T - 1));
 }
-__device__ __forceinline__ int cell_offset(const CellList &c, int b)
+
+// screen positions (as pack_screen_positions), each CTA's extent, and the
+// zeros that the next kernels count up from
+__global__ void __launch_bounds__(kCellPackTpb) cell_pack_kernel(CellList c, const double *__restrict__ xs, int S,
+                                                                 const double *__restrict__ xb, int B,
+                                                                 float4 *__restrict__ out)
 {
-    return __ldcg(c.local + b) + __ldcg(c.tile_prefix + b / kCellScanTile);
+    pdl_wait_then_release();
+    __shared__ unsigned wmax[kCellPackTpb / 32];
+    const int i = blockIdx.x * kCellPackTpb + threadIdx.x;
+    const double *p0 = S > 0 ? xs : xb;
+    float m = 0.0f;
+    if (i < S + B) {
+        const double *p = i < S ? xs + 3 * (size_t)i : xb + 3 * (size_t)(i - S);
+        const float rx = (float)(p[0] - p0[0]), ry = (float)(p[1] - p0[1]), rz = (float)(p[2] - p0[2]);
+        out[i] = make_float4(rx, ry, rz, 0.f);
+        m = fmaxf(fabsf(rx), fmaxf(fabsf(ry), fabsf(rz)));
+    }
+    for (int b = i; b < c.T; b += gridDim.x * kCellPackTpb) c.count[b] = 0;
+    if (i == 0) {
+        c.overflow[0] = 0;
+        *c.extent = 0u;
+    }
+    const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mb;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const unsigned w = threadIdx.x < kCellPackTpb / 32 ? wmax[threadIdx.x] : 0u;
+        const unsigned all = __reduce_max_sync(0xffffffffu, w);
+        if (threadIdx.x == 0) c.block_max[blockIdx.x] = __uint_as_float(all);
+    }
 }
 
-__global__ void cell_keys_kernel(CellList c, const float4 *__restrict__ screen, int N)
+// every particle into its bucket; each CTA first takes the extent over the
+// pack kernel's CTAs (the first writes it for the kernels that follow)
+__global__ void __launch_bounds__(kCellPackTpb) cell_insert_kernel(CellList c, const float4 *__restrict__ screen, int N)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait_then_release();
+    __shared__ unsigned wmax[kCellPackTpb / 32];
+    unsigned mb = 0u;  // non-negative FP32 bits order like the values
+    for (int b = threadIdx.x; b < c.blocks; b += kCellPackTpb) mb = max(mb, __float_as_uint(c.block_max[b]));
+    mb = __reduce_max_sync(0xffffffffu, mb);
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mb;
+    __syncthreads();
+    mb = wmax[0];
+#pragma unroll
+    for (int w = 1; w < kCellPackTpb / 32; ++w) mb = max(mb, wmax[w]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *c.extent = mb;
+    const int i = blockIdx.x * kCellPackTpb + threadIdx.x;
     if (i >= N) return;
-    const float inv_h = cell_inv_width(c);
+    const float inv_h = cell_inv_width(c, __uint_as_float(mb));
     const float4 p = screen[i];
     const int b = cell_bucket(cell_coord(p.x, inv_h), cell_coord(p.y, inv_h), cell_coord(p.z, inv_h), c.T);
-    c.key[i] = b;
-    atomicAdd(c.count + b, 1);
+    const int k = atomicAdd(c.count + b, 1);
+    if (k < kCellSlots) c.slot[(size_t)b * kCellSlots + k] = make_float4(p.x, p.y, p.z, __int_as_float(i));
 }
 
-// Exclusive scan of the bucket counts: each CTA scans one tile of
-// kCellScanTile buckets (four per thread) into local[] and writes its total;
-// the last CTA to finish scans the totals into tile_prefix[].
-__global__ void __launch_bounds__(kCellScanTpb) cell_scan_kernel(CellList c)
-{
-    __shared__ int warp_tot[kCellScanTpb / 32];
-    __shared__ int is_last;
-    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    const int base = blockIdx.x * kCellScanTile + 4 * t;
-    const int4 v = *reinterpret_cast<const int4 *>(c.count + base);
-    const int own = v.x + v.y + v.z + v.w;
-    int incl = own;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) warp_tot[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-        int w = warp_tot[lane];
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        warp_tot[lane] = w;  // inclusive over warps
-    }
-    __syncthreads();
-    const int before = incl - own + (wid > 0 ? warp_tot[wid - 1] : 0);
-    int4 e;
-    e.x = before;
-    e.y = before + v.x;
-    e.z = e.y + v.y;
-    e.w = e.z + v.z;
-    *reinterpret_cast<int4 *>(c.local + base) = e;
-    if (t == kCellScanTpb - 1) {
-        c.tile_prefix[blockIdx.x] = before + own;  // the tile's total, scanned below
-        __threadfence();
-        is_last = atomicAdd(c.ticket, 1) == (int)gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    // the last CTA: exclusive scan of the gridDim.x (<= kCellScanTpb) tile totals
-    const int n = gridDim.x;
-    const int tot = t < n ? __ldcg(c.tile_prefix + t) : 0;
-    int x = tot;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    __syncthreads();
-    if (lane == 31) warp_tot[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        int w = warp_tot[lane];
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        warp_tot[lane] = w;
-    }
-    __syncthreads();
-    if (t < n) c.tile_prefix[t] = x - tot + (wid > 0 ? warp_tot[wid - 1] : 0);
-    if (t == 0) *c.ticket = 0;
-}
-
-__global__ void cell_scatter_kernel(CellList c, int N)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const int b = c.key[i];
-    const int slot = atomicSub(c.count + b, 1) - 1;
-    c.order[cell_offset(c, b) + slot] = i;
-}
-
-// The FP64 force of one accepted pair, as barrier_flush: zero outside the
-// exact cutoff.
-__device__ __forceinline__ void barrier_pair(const BarrierLaunch &a, int j, double xi, double yi, double zi,
-                                             double a_tgt, double &g0, double &g1, double &g2)
+// The FP64 force of one accepted pair, as barrier_flush, in the two factors
+// that a sum takes it by: (x, y, z) i, zero outside the exact cutoff.
+struct BarrierTerm {
+    double x, y, z, i;
+};
+__device__ __forceinline__ BarrierTerm barrier_term(const BarrierLaunch &a, int j, double xi, double yi, double zi,
+                                                    double a_tgt)
 {
     const bool src_seg = j < a.S;
     const double asum = a_tgt + (src_seg ? a.rseg : a.rblob);
     const double *pj = src_seg ? a.xs + 3 * (size_t)j : a.xb + 3 * (size_t)(j - a.S);
     const double ddx = xi - pj[0], ddy = yi - pj[1], ddz = zi - pj[2];
     const double dist = sqrt(ddx * ddx + ddy * ddy + ddz * ddz);
-    if (dist < 1.1 * asum) {
-        double cc = fmin(1.0, 1.0 - (10.0 / asum) * (dist - asum));
-        cc = a.scale * cc * cc * cc * cc;
-        const double idist = 1.0 / dist;
-        g0 += cc * ddx * idist;
-        g1 += cc * ddy * idist;
-        g2 += cc * ddz * idist;
-    }
+    if (!(dist < 1.1 * asum)) return BarrierTerm{0.0, 0.0, 0.0, 0.0};
+    double cc = fmin(1.0, 1.0 - (10.0 / asum) * (dist - asum));
+    cc = a.scale * cc * cc * cc * cc;
+    return BarrierTerm{cc * ddx, cc * ddy, cc * ddz, 1.0 / dist};
 }
 
 // a target's launch-local index -> its global particle index, position and
@@ -1222,59 +1197,96 @@ __device__ __forceinline__ void barrier_cutoffs(const BarrierLaunch &a, bool seg
 
 __global__ void __launch_bounds__(kCellTpb) barrier_cell_kernel(BarrierLaunch a, CellList c)
 {
-    __shared__ int cand[kCellCand * kCellTpb];  // candidate e of thread t at [e * kCellTpb + t]
-    const int ntg = a.num_segs + (a.wall ? 0 : a.num_blobs);
-    const int local = blockIdx.x * blockDim.x + threadIdx.x;
-    if (local >= ntg) return;
-    const int N = a.S + a.B;
-    const BarrierTarget t = barrier_target(a, local);
-    const float4 pf = a.screen[t.gi];
-    float c2_s, c2_b;
-    barrier_cutoffs(a, t.seg, c2_s, c2_b);
-    const float inv_h = cell_inv_width(c);
-    const int cx = cell_coord(pf.x, inv_h), cy = cell_coord(pf.y, inv_h), cz = cell_coord(pf.z, inv_h);
-    int n = 0;
-    bool over = false;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) {
-                const int b = cell_bucket(cx + dx, cy + dy, cz + dz, c.T);
-                const int beg = cell_offset(c, b), end = b + 1 < c.T ? cell_offset(c, b + 1) : N;
-                for (int p = beg; p < end; ++p) {
-                    const int j = __ldcg(c.order + p);
-                    if (!barrier_candidate(a, t, pf, c2_s, c2_b, j, a.screen[j])) continue;
-                    if (n < kCellCand)
-                        cand[n * kCellTpb + threadIdx.x] = j;
-                    else
-                        over = true;
-                    ++n;
-                }
-            }
-    if (over) {
-        const int pos = atomicAdd(c.overflow, 1);
-        c.overflow[1 + pos] = local;
-        return;
+    pdl_wait_then_release();
+    __shared__ float4 pos[kCellTargets];
+    __shared__ int3 cell[kCellTargets];
+    __shared__ int n_cand[kCellTargets], start[kCellTargets + 1], n_kept[kCellTargets];
+    __shared__ int cand[kCellTargets][kCellCand];
+    __shared__ __align__(16) BarrierTerm force[kCellTargets][kCellCand];
+    const int ntg = a.num_segs + (a.wall ? 0 : a.num_blobs), tid = threadIdx.x;
+    const int local0 = blockIdx.x * kCellTargets, nt = min(kCellTargets, ntg - local0);
+    if (tid < nt) {
+        const int local = local0 + tid;
+        const int gi = local < a.num_segs ? a.start_seg + local : a.S + a.start_blob + (local - a.num_segs);
+        const float inv_h = cell_inv_width(c, __uint_as_float(*c.extent));
+        const float4 p = a.screen[gi];
+        pos[tid] = p;
+        cell[tid] = make_int3(cell_coord(p.x, inv_h), cell_coord(p.y, inv_h), cell_coord(p.z, inv_h));
+        n_cand[tid] = n_kept[tid] = 0;
     }
-    // ascending j (insertion sort of a handful), repeats dropped below
-    for (int e = 1; e < n; ++e) {
-        const int v = cand[e * kCellTpb + threadIdx.x];
-        int f = e - 1;
-        while (f >= 0 && cand[f * kCellTpb + threadIdx.x] > v) {
-            cand[(f + 1) * kCellTpb + threadIdx.x] = cand[f * kCellTpb + threadIdx.x];
-            --f;
+    __syncthreads();
+    // a target's 27 buckets, one (target, bucket) pair per thread and turn
+    for (int it = tid; it < nt * 27; it += kCellTpb) {
+        const int t = it / 27, nb = it - 27 * t;
+        const int3 q = cell[t];
+        const int b = cell_bucket(q.x + nb % 3 - 1, q.y + nb / 3 % 3 - 1, q.z + nb / 9 - 1, c.T);
+        const float4 *slots = c.slot + (size_t)b * kCellSlots;
+        const int held = __ldcg(c.count + b);
+        const float4 ahead = __ldcg(slots);  // with the count: an empty bucket's entry is not used
+        if (held == 0) continue;
+        if (held > kCellSlots) {
+            atomicAdd(&n_cand[t], kCellCand + 1);
+            continue;
         }
-        cand[(f + 1) * kCellTpb + threadIdx.x] = v;
+        BarrierTarget tg;
+        const int local = local0 + t;
+        tg.seg = local < a.num_segs;
+        tg.gi = tg.seg ? a.start_seg + local : a.S + a.start_blob + (local - a.num_segs);
+        float c2_s, c2_b;
+        barrier_cutoffs(a, tg.seg, c2_s, c2_b);
+        const float4 pf = pos[t];
+        for (int k = 0; k < held; ++k) {
+            const float4 e = k == 0 ? ahead : __ldcg(slots + k);
+            const int j = __float_as_int(e.w);
+            if (!barrier_candidate(a, tg, pf, c2_s, c2_b, j, e)) continue;
+            const int at = atomicAdd(&n_cand[t], 1);
+            if (at < kCellCand) cand[t][at] = j;
+        }
     }
-    const double a_tgt = t.seg ? a.rseg : a.rblob;
-    double g0 = 0.0, g1 = 0.0, g2 = barrier_wall_z(a, t);
-    int prev = -1;
-    for (int e = 0; e < n; ++e) {
-        const int j = cand[e * kCellTpb + threadIdx.x];
-        if (j == prev) continue;
-        prev = j;
-        barrier_pair(a, j, t.x, t.y, t.z, a_tgt, g0, g1, g2);
+    __syncthreads();
+    if (tid == 0) {
+        int at = 0;
+        for (int t = 0; t < nt; ++t) {
+            start[t] = at;
+            at += n_cand[t] > kCellCand ? 0 : n_cand[t];
+        }
+        start[nt] = at;
     }
-    barrier_store(a, t, local, g0, g1, g2);
+    if (tid < nt && n_cand[tid] > kCellCand) c.overflow[1 + atomicAdd(c.overflow, 1)] = local0 + tid;
+    __syncthreads();
+    // the candidates' forces, each at its index's rank
+    for (int f = tid; f < start[nt]; f += kCellTpb) {
+        int t = 0;
+        while (f >= start[t + 1]) ++t;
+        const int e = f - start[t], n = n_cand[t], j = cand[t][e];
+        int rank = 0, repeats = 0;
+        for (int o = 0; o < n; ++o) {
+            const int jo = cand[t][o];
+            repeats += jo == j && o < e;
+            bool first = jo < j;  // counted once, however often it is in the list
+            for (int r = 0; first && r < o; ++r) first = cand[t][r] != jo;
+            rank += first;
+        }
+        if (repeats) continue;
+        const BarrierTarget tg = barrier_target(a, local0 + t);
+        force[t][rank] = barrier_term(a, j, tg.x, tg.y, tg.z, tg.seg ? a.rseg : a.rblob);
+        atomicAdd(&n_kept[t], 1);
+    }
+    __syncthreads();
+    for (int o = tid; o < 3 * nt; o += kCellTpb) {
+        const int t = o / 3, comp = o - 3 * t, local = local0 + t;
+        if (n_cand[t] > kCellCand) continue;
+        double g = 0.0;
+        if (comp == 2 && a.wall) g = barrier_wall_z(a, barrier_target(a, local));
+        for (int e = 0; e < n_kept[t]; ++e) {
+            const BarrierTerm &f = force[t][e];
+            g = fma(comp == 0 ? f.x : comp == 1 ? f.y : f.z, f.i, g);
+        }
+        if (local < a.num_segs)
+            a.f_segs[6 * (size_t)(a.start_seg + local) + comp] += g;
+        else
+            a.f_blobs_rep[3 * (size_t)(local - a.num_segs) + comp] = g;
+    }
 }
 
 // Targets with more candidates than the cell kernel keeps: one warp each,
@@ -1282,6 +1294,7 @@ __global__ void __launch_bounds__(kCellTpb) barrier_cell_kernel(BarrierLaunch a,
 // ascending j by lane 0 (the lanes evaluate their own source's force).
 __global__ void __launch_bounds__(128) barrier_overflow_kernel(BarrierLaunch a, CellList c)
 {
+    pdl_wait_then_release();
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * (blockDim.x >> 5);
     const int N = a.S + a.B;
@@ -1299,7 +1312,12 @@ __global__ void __launch_bounds__(128) barrier_overflow_kernel(BarrierLaunch a, 
             const bool cand = j < N && barrier_candidate(a, t, pf, c2_s, c2_b, j, a.screen[j]);
             unsigned mask = __ballot_sync(0xffffffffu, cand);
             double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-            if (cand) barrier_pair(a, j, t.x, t.y, t.z, a_tgt, v0, v1, v2);
+            if (cand) {
+                const BarrierTerm f = barrier_term(a, j, t.x, t.y, t.z, a_tgt);
+                v0 = f.x * f.i;
+                v1 = f.y * f.i;
+                v2 = f.z * f.i;
+            }
             while (mask) {
                 const int src = __ffs(mask) - 1;
                 mask &= mask - 1;
@@ -1844,44 +1862,41 @@ gmi_status launch_barrier(gmi_context *ctx, const BarrierLaunch &in)
         if (st != GMI_OK) return st;
         a.partial = static_cast<double *>(ctx->partial.ptr);
     }
-    GMI_CUDA_TRY(cudaMemsetAsync(a.extent, 0, sizeof(unsigned), ctx->stream));
-    pack_screen_positions<<<(N + 255) / 256, 256, 0, ctx->stream>>>(a.xs, a.S, a.xb, a.B, a.screen, a.extent);
-    ctx->launches++;
     // the cell list from kCellMinParticles particles (GMI_BARRIER_CELLS=0
-    // never, =1 always), up to the scan's 4 M buckets
+    // never, =1 always), up to kCellMaxBuckets buckets
     const char *cells_env = std::getenv("GMI_BARRIER_CELLS");
     const bool cells = cells_env ? cells_env[0] != '0' : N >= kCellMinParticles;
-    int T = kCellScanTile;
-    while (T < 2 * N) T *= 2;
-    if (cells && T / kCellScanTile <= kCellScanTpb) {
+    int T = 4096;
+    while (T < 2 * N && T < kCellMaxBuckets) T *= 2;
+    if (cells && T >= 2 * N) {
         a.partial = nullptr;
-        const size_t tiles = (size_t)T / kCellScanTile;
-        const size_t ints = 4 + 2 * (size_t)T + ((tiles + 3) & ~(size_t)3) + 2 * (size_t)N + 1 + (size_t)ntg;
-        st = ctx->cells.reserve(ints * sizeof(int));
+        const int blocks = (N + kCellPackTpb - 1) / kCellPackTpb;
+        const auto round = [](size_t n) { return (n + 3) & ~(size_t)3; };
+        const size_t words = 4 * (size_t)T * kCellSlots + (size_t)T + round(blocks) + 4 + 1 + (size_t)ntg;
+        st = ctx->cells.reserve(words * sizeof(int));
         if (st != GMI_OK) return st;
         CellList c{};
-        int *base = static_cast<int *>(ctx->cells.ptr);
         c.T = T;
         c.cut_max = std::max(a.cut_ss, std::max(a.cut_sb, a.cut_bb));
         c.extent = a.extent;
-        c.ticket = base;
-        c.count = base + 4;
-        c.local = c.count + T;
-        c.tile_prefix = c.local + T;
-        c.key = c.tile_prefix + ((tiles + 3) & ~(size_t)3);
-        c.order = c.key + N;
-        c.overflow = c.order + N;
-        GMI_CUDA_TRY(cudaMemsetAsync(base, 0, (4 + (size_t)T) * sizeof(int), ctx->stream));
-        GMI_CUDA_TRY(cudaMemsetAsync(c.overflow, 0, sizeof(int), ctx->stream));
-        cell_keys_kernel<<<(N + 255) / 256, 256, 0, ctx->stream>>>(c, a.screen, N);
-        cell_scan_kernel<<<(unsigned)tiles, kCellScanTpb, 0, ctx->stream>>>(c);
-        cell_scatter_kernel<<<(N + 255) / 256, 256, 0, ctx->stream>>>(c, N);
-        barrier_cell_kernel<<<(ntg + kCellTpb - 1) / kCellTpb, kCellTpb, 0, ctx->stream>>>(a, c);
-        barrier_overflow_kernel<<<ctx->sm_count, 128, 0, ctx->stream>>>(a, c);
-        ctx->launches += 5;
+        c.blocks = blocks;
+        c.slot = static_cast<float4 *>(ctx->cells.ptr);
+        c.count = reinterpret_cast<int *>(c.slot + (size_t)T * kCellSlots);
+        c.block_max = reinterpret_cast<float *>(c.count + T);
+        c.overflow = c.count + T + round(blocks);
+        cell_pack_kernel<<<blocks, kCellPackTpb, 0, ctx->stream>>>(c, a.xs, a.S, a.xb, a.B, a.screen);
+        GMI_CUDA_TRY(launch_chained(true, cell_insert_kernel, dim3(blocks), dim3(kCellPackTpb), ctx->stream, c, a.screen,
+                                    N));
+        GMI_CUDA_TRY(launch_chained(true, barrier_cell_kernel, dim3((ntg + kCellTargets - 1) / kCellTargets),
+                                    dim3(kCellTpb), ctx->stream, a, c));
+        GMI_CUDA_TRY(launch_chained(true, barrier_overflow_kernel, dim3(ctx->sm_count), dim3(128), ctx->stream, a, c));
+        ctx->launches += 4;
         GMI_CUDA_TRY(cudaGetLastError());
         return GMI_OK;
     }
+    GMI_CUDA_TRY(cudaMemsetAsync(a.extent, 0, sizeof(unsigned), ctx->stream));
+    pack_screen_positions<<<(N + 255) / 256, 256, 0, ctx->stream>>>(a.xs, a.S, a.xb, a.B, a.screen, a.extent);
+    ctx->launches++;
     barrier_kernel<<<dim3(tgt_ctas, splits), kBarrierTpb, 0, ctx->stream>>>(a);
     ctx->launches++;
     if (splits > 1) {

@@ -124,7 +124,9 @@ class Context:
         """fs_inout[:, :3] += segment repulsion (in place); returns blob repulsion."""
         S, B = xs.shape[0], xb.shape[0]
         if fb_out is None:
-            fb_out = torch.zeros((max(B, 1), 3), dtype=torch.float64, device=xs.device)
+            # with a wall the kernels leave the blobs' rows as they are; without one they write them all
+            make = torch.zeros if wall else torch.empty
+            fb_out = make((max(B, 1), 3), dtype=torch.float64, device=xs.device)
         check(self.lib.gmi_barrier_forces(
             self.handle, _dev(fs_inout, S, 6, "f_segs") if S else None,
             fb_out.data_ptr() if B else None,
