@@ -1,28 +1,33 @@
 // gmi_fx_kernels.cu -- the FP64-grade free-space pair sums (precision
 // GMI_FP64) in 64-bit fixed point.
 //
-// Two kernels per sum, or one for small sums.  The pack kernel turns the sources into integer
-// records (gmi_pairs_fx.cuh), one CTA per tile of 128 with the tile's
-// exponent found by a block maximum.  In the pair kernel a CTA owns 32
-// targets, one per lane, and a contiguous slice ("split") of the sources,
-// staged tile by tile into shared memory by bulk copies; its four warps take
-// a quarter of each tile each, fold their integer sums into FP64 per tile
-// and meet in shared memory at the end.  32 targets per CTA rather than 128
-// let a few hundred targets reach every SM.  With several splits reduce_splits
-// adds the partial sums in split order.
+// Two kernels per sum, or one for small sums.  The pack kernel turns the
+// sources into integer records (gmi_pairs_fx.cuh), one CTA per block of 512
+// with the block's exponent found by a block maximum.  In the pair kernel a CTA
+// owns 32 targets, one per lane, and a contiguous slice ("split") of the
+// sources, staged in tiles of 128 into shared memory by bulk copies; its four
+// warps take a quarter of each tile each, fold their integer sums into FP64 once
+// per block and meet in shared memory at the end.  32 targets per CTA rather than
+// 128 let a few hundred targets reach every SM.  With several splits
+// reduce_splits_tree adds the partial sums.
 //
-// A tile whose loads or positions the formats do not hold (not finite, a load
+// A block whose loads or positions the formats do not hold (not finite, a load
 // beyond 2^+-900, a particle further than about 400 radii from the first
 // source) is marked by the pack kernel, and its pairs, and all pairs of a
 // warp with such a target, are summed in FP64 from the original arrays.
 //
-// What bounds it: the integer pipes.  M_ss executes about 530 instructions a
-// pair and warp (210 on the FMA pipe, 146 of them 32x32 -> 64-bit, 290 on the
-// ALU) at 1.8 cycles each, whatever the split and the occupancy; the FP64
-// kernel executed 65 FP64 instructions at 76 cycles each.  12,800 segments:
-// 20.4 -> 3.9 ms (87 flop a pair: 0.70 -> 3.7 TFLOP/s); 4096 blobs: 1222 ->
-// 231 us; 12,800 segments with 4096 blobs, both ways: 9.7 -> 1.8 ms.  Error
-// against exact sums at 12,800 segments: 1.4e-15 -> 3.1e-16.
+// What bounds it: instruction issue, M_ss about 470 instructions a pair and warp
+// (61 wide integer multiplies, 140 FP32, 200 integer) at 1.5 cycles each; the
+// FP64 kernel executed 65 FP64 instructions at 76 cycles each.  Integer limbs
+// alone (530 instructions, 146 of them wide multiplies) took 1.8 cycles each.
+// FP64 kernel -> integer limbs -> limb and FP32 (this one):
+//   12,800 segments                  20.4 -> 3.90 -> 2.81 ms  (5.1 TFLOP/s at 87 flop a pair)
+//   4096 blobs                       1223 -> 229 -> 188 us
+//   12,800 segments, 4096 blobs,
+//   both ways                        9.72 -> 1.80 -> 1.40 ms
+// Error against extended precision (2-norm, mean of four draws), FP64 kernel ->
+// this: 60 to 700 segments 0.86 to 1.02 of it, 1500 segments 2.9e-16 -> 1.9e-16;
+// 50 to 1200 blobs 0.7 to 0.96; 100 segments on 60 blobs 2.1e-16 -> 2.1e-16.
 #include <algorithm>
 
 #include "gmi_fx_kernels.hpp"
@@ -35,25 +40,26 @@ namespace gmi {
 static_assert((int)kFxSS == (int)kSS && (int)kFxBB == (int)kBB && (int)kFxSB == (int)kSB && (int)kFxBS == (int)kBS,
               "FxKind follows PairKind");
 
-constexpr int kFxTile = 128;   // sources per tile: one exponent, one stage
+constexpr int kFxTile = 128;   // sources per tile: one stage
+constexpr int kFxBlock = 512;  // sources per block: one exponent, one fold
 constexpr int kFxTpb = 128;    // four warps
 constexpr int kFxWarps = kFxTpb / 32;
 constexpr int kFxStages = 2;
 constexpr int kFxInlinePerSm = 4;  // CTAs per SM up to which a CTA packs its own sources
-constexpr int kFxBadTile = -0x7fffffff;  // in place of a tile's exponent: sum it in FP64
-static_assert(kFxTile == kFxWarps * kFxFold, "a warp's quarter of a tile is one fold");
+constexpr int kFxBadTile = -(1 << 22);  // in place of a block's exponent: sum it in FP64
+static_assert(kFxBlock == kFxWarps * kFxFold && kFxBlock % kFxTile == 0, "a warp's quarter of a block is one fold");
 
 template <int KIND> struct FxTraits {
     static constexpr bool torque = KIND == kFxSS || KIND == kFxBS;
     static constexpr int nout = (KIND == kFxSS || KIND == kFxSB) ? 6 : 3;
     static constexpr int nf = torque ? 6 : 3;
-    static constexpr int words = torque ? 10 : 8;  // 64-bit words per record: X F [T] {gap, E} [pad]
-    static constexpr int meta = torque ? 9 : 6;
+    // 16-byte quarters per record: X0 X1 | X2 F0.h F0.hf | F0.lf F1 | F2 meta | T0 T1 | T2 pad
+    static constexpr int quads = torque ? 6 : 4;
 };
 
 struct FxLaunch {
     const double *xt, *xs, *fs;
-    const unsigned long long *rec;
+    const int4 *rec;
     int tgt_start, n_tgt, n_src, chunk;
     double *out, *partial;
     int accumulate;
@@ -96,8 +102,8 @@ __device__ __forceinline__ FxPacking<KIND> fx_read_source(const double *__restri
     return p;
 }
 
-// The largest exponent of a CTA of kFxTpb threads, one source each.
-__device__ __forceinline__ int fx_block_max(int e, int *wmax)
+// The largest exponent of a CTA of NW warps, one source per thread.
+template <int NW> __device__ __forceinline__ int fx_block_max(int e, int *wmax)
 {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
@@ -105,13 +111,13 @@ __device__ __forceinline__ int fx_block_max(int e, int *wmax)
     __syncthreads();
     e = wmax[0];
 #pragma unroll
-    for (int w = 1; w < kFxWarps; ++w) e = max(e, wmax[w]);
+    for (int w = 1; w < NW; ++w) e = max(e, wmax[w]);
     return e;
 }
 
-// The record of a source in a tile whose largest exponent is E.
+// The record of a source in a block whose largest exponent is E.
 template <int KIND>
-__device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E, unsigned long long *r)
+__device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E, int4 *r)
 {
     using Tr = FxTraits<KIND>;
     const bool bad = E == kFxMark;
@@ -121,34 +127,38 @@ __device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E,
         used = E - gap;
     }
     const double scale = bad ? 0.0 : fx_exp2(-used);
-    const int meta = bad ? kFxBadTile : E == kFxNoLoad ? 0 : E;
+    const int tile = bad ? kFxBadTile : E == kFxNoLoad ? 0 : E;
+    const auto lo = [](long long v) { return (int)(unsigned)v; };
+    const auto hi = [](long long v) { return (int)(v >> 32); };
+    fxop F[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        r[c] = (unsigned long long)p.X[c];
-        const fx l = fx_split(bad ? 0 : fx_from_double(p.F[c] * scale));
-        r[3 + c] = ((unsigned long long)(unsigned)l.hi << 32) | (unsigned)l.lo;
-    }
+    for (int c = 0; c < 3; ++c) F[c] = bad ? fxop{0, 0.0f, 0.0f} : fx_from_double(p.F[c] * scale);
+    r[0] = make_int4(lo(p.X[0]), hi(p.X[0]), lo(p.X[1]), hi(p.X[1]));
+    r[1] = make_int4(lo(p.X[2]), hi(p.X[2]), F[0].h, __float_as_int(F[0].hf));
+    r[2] = make_int4(__float_as_int(F[0].lf), F[1].h, __float_as_int(F[1].hf), __float_as_int(F[1].lf));
+    r[3] = make_int4(F[2].h, __float_as_int(F[2].hf), __float_as_int(F[2].lf), (int)((unsigned)tile << 8) | gap);
     if constexpr (Tr::torque) {
+        long long T[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) r[6 + c] = bad ? 0ull : (unsigned long long)fx_from_double(p.F[3 + c] * scale);
+        for (int c = 0; c < 3; ++c) T[c] = bad ? 0 : fx_rint(p.F[3 + c] * scale * 4611686018427387904.0);
+        r[4] = make_int4(lo(T[0]), hi(T[0]), lo(T[1]), hi(T[1]));
+        r[5] = make_int4(lo(T[2]), hi(T[2]), 0, 0);
     }
-    r[Tr::meta] = ((unsigned long long)(unsigned)meta << 32) | (unsigned)gap;
 }
 
 template <int KIND>
-__global__ void __launch_bounds__(kFxTile) fx_pack_kernel(const double *__restrict__ x, const double *__restrict__ f,
-                                                          int n, FxConsts K, unsigned long long *__restrict__ rec,
-                                                          const int *skip)
+__global__ void __launch_bounds__(kFxBlock) fx_pack_kernel(const double *__restrict__ x, const double *__restrict__ f,
+                                                          int n, FxConsts K, int4 *__restrict__ rec, const int *skip)
 {
-    __shared__ int wmax[kFxWarps];
+    __shared__ int wmax[kFxBlock / 32];
     pdl_wait_then_release();
     if (skip != nullptr && *skip != 0) return;
-    const int i = blockIdx.x * kFxTile + threadIdx.x;
+    const int i = blockIdx.x * kFxBlock + threadIdx.x;
     FxPacking<KIND> p;
     p.e = kFxNoLoad;
     if (i < n) p = fx_read_source<KIND>(x, f, i, K);
-    const int E = fx_block_max(p.e, wmax);
-    if (i < n) fx_write_record<KIND>(p, E, rec + (size_t)i * FxTraits<KIND>::words);
+    const int E = fx_block_max<kFxBlock / 32>(p.e, wmax);
+    if (i < n) fx_write_record<KIND>(p, E, rec + (size_t)i * FxTraits<KIND>::quads);
 }
 
 struct FxSum {
@@ -175,27 +185,27 @@ static __device__ __noinline__ FxSum fx_sum_fp64(const FxLaunch &a, int ti, int 
     return s;
 }
 
-__device__ __forceinline__ fx fx_limbs(unsigned long long w) { return fx{(int)(w >> 32), (int)(unsigned)w}; }
-
-template <int KIND> __device__ __forceinline__ FxSource fx_load_source(const unsigned long long *p)
+__device__ __forceinline__ long long fx_word(int lo, int hi)
 {
-    const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p);
-    const ulonglong2 a = q[0], b = q[1], c = q[2];
+    return (long long)(((unsigned long long)(unsigned)hi << 32) | (unsigned)lo);
+}
+
+template <int KIND> __device__ __forceinline__ FxSource fx_load_source(const int4 *q)
+{
+    const int4 a = q[0], b = q[1], c = q[2], d = q[3];
     FxSource s;
-    s.X[0] = (long long)a.x;
-    s.X[1] = (long long)a.y;
-    s.X[2] = (long long)b.x;
-    s.F[0] = fx_limbs(b.y);
-    s.F[1] = fx_limbs(c.x);
-    s.F[2] = fx_limbs(c.y);
+    s.X[0] = fx_word(a.x, a.y);
+    s.X[1] = fx_word(a.z, a.w);
+    s.X[2] = fx_word(b.x, b.y);
+    s.F[0] = fxop{b.z, __int_as_float(b.w), __int_as_float(c.x)};
+    s.F[1] = fxop{c.y, __int_as_float(c.z), __int_as_float(c.w)};
+    s.F[2] = fxop{d.x, __int_as_float(d.y), __int_as_float(d.z)};
+    s.gap = d.w & 255;
     if constexpr (FxTraits<KIND>::torque) {
-        const ulonglong2 d = q[3], e = q[4];
-        s.T[0] = (long long)d.x;
-        s.T[1] = (long long)d.y;
-        s.T[2] = (long long)e.x;
-        s.gap = (int)(unsigned)e.y;
-    } else {
-        s.gap = (int)(unsigned)p[FxTraits<KIND>::meta];
+        const int4 e = q[4], f = q[5];
+        s.T[0] = fx_word(e.x, e.y);
+        s.T[1] = fx_word(e.z, e.w);
+        s.T[2] = fx_word(f.x, f.y);
     }
     return s;
 }
@@ -209,14 +219,19 @@ __device__ __forceinline__ void bulk_load(void *smem_dst, const void *src, unsig
                  : "memory");
 }
 
+// CTAs per SM that the registers are held to.  M_ss: 3 2.80 ms (12,800
+// segments), 4 2.85; M_bb: 6 185 us (4096 blobs), 5 189, 7 190, 4 194; both
+// ways between the two: 4 1.37 ms, 3 1.42, 5 1.40.
+template <int KIND> constexpr int kFxCtas = KIND == kFxSS ? 3 : KIND == kFxBB ? 6 : 4;
+
 // kInline: no pack kernel ran; the split is at most one tile, whose records the
 // CTA makes itself.
 template <int KIND, bool kInline>
-__global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(const __grid_constant__ FxLaunch a)
+__global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __grid_constant__ FxLaunch a)
 {
     using Tr = FxTraits<KIND>;
     constexpr int NOUT = Tr::nout;
-    __shared__ __align__(128) unsigned long long ring[kFxStages][kFxTile * Tr::words];
+    __shared__ __align__(128) int4 ring[kFxStages][kFxTile * Tr::quads];
     __shared__ double red[kFxWarps][NOUT][33];
     __shared__ uint64_t bars[kFxStages];
     __shared__ int wmax[kFxWarps];
@@ -237,9 +252,9 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
     int issued = 0;  // tiles requested so far (meaningful on thread 0)
     const auto request = [&](int t) {
         const int j0 = j_begin + t * kFxTile;
-        const unsigned bytes = (unsigned)min(kFxTile, j_end - j0) * (Tr::words * 8u);
+        const unsigned bytes = (unsigned)min(kFxTile, j_end - j0) * (Tr::quads * 16u);
         mbar_arrive_expect_tx(&bars[t % kFxStages], bytes);
-        bulk_load(ring[t % kFxStages], a.rec + (size_t)j0 * Tr::words, bytes, &bars[t % kFxStages]);
+        bulk_load(ring[t % kFxStages], a.rec + (size_t)j0 * Tr::quads, bytes, &bars[t % kFxStages]);
     };
     if (!kInline && tid == 0)
         for (; issued < kFxStages && issued < ntiles; ++issued) request(issued);
@@ -248,8 +263,8 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
         p.e = kFxNoLoad;
         const int i = j_begin + tid;
         if (i < j_end) p = fx_read_source<KIND>(a.xs, a.fs, i, a.K);
-        const int E = fx_block_max(p.e, wmax);
-        if (i < j_end) fx_write_record<KIND>(p, E, ring[0] + tid * Tr::words);
+        const int E = fx_block_max<kFxWarps>(p.e, wmax);
+        if (i < j_end) fx_write_record<KIND>(p, E, ring[0] + tid * Tr::quads);
         __syncthreads();
     }
 
@@ -266,6 +281,8 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
     for (int c = 0; c < NOUT; ++c) tot[c] = 0.0;
 
     bool timed_out = false;
+    FxAcc<NOUT> acc;
+    fx_clear(acc);
     int t = 0;
     for (; t < ntiles; ++t) {
         const int s = t % kFxStages;
@@ -280,25 +297,26 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
         }
         const int j0 = j_begin + t * kFxTile, jn = min(kFxTile, j_end - j0);
         const int per = (jn + kFxWarps - 1) / kFxWarps, b = min(warp * per, jn), e = min(b + per, jn);
-        const unsigned long long *tile = ring[s];
-        const int E = (int)(tile[Tr::meta] >> 32);
-        if (E == kFxBadTile || !warp_ok) {
+        const int4 *tile = ring[s];
+        const int E = tile[3].w >> 8;
+        if (E == kFxBadTile || !warp_ok) {  // the whole block
             const FxSum r = fx_sum_fp64<KIND>(a, ti, j0 + b, j0 + e);
 #pragma unroll
             for (int c = 0; c < NOUT; ++c) tot[c] += r.v[c];
             continue;
         }
-        long long H[NOUT], L[NOUT];
-#pragma unroll
-        for (int c = 0; c < NOUT; ++c) H[c] = L[c] = 0;
+        for (int j = b; j < e;) {
+            const int stop = min(j + kFxSettle[KIND], e);
 #pragma unroll 1
-        for (int j = b; j < e; ++j) {
-            const FxSource src = fx_load_source<KIND>(tile + j * Tr::words);
-            fx_pair<KIND>(X, src, a.K, H, L);
+            for (; j < stop; ++j) fx_pair<KIND>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc);
+            fx_settle(acc);
         }
-        const double scale = fx_exp2(E);
+        if (t + 1 == ntiles || (j0 + kFxTile) % kFxBlock == 0) {  // the block's last tile here
+            const double scale = fx_exp2(E);
 #pragma unroll
-        for (int c = 0; c < NOUT; ++c) tot[c] += fx_fold(H[c], L[c], (c < 3 ? a.K.vscale : a.K.wscale) * scale);
+            for (int c = 0; c < NOUT; ++c) tot[c] += fx_fold(acc, c, (c < 3 ? a.K.vscale : a.K.wscale) * scale, a.K.vscale_fix);
+            fx_clear(acc);
+        }
     }
 
     if (timed_out) {
@@ -328,10 +346,10 @@ __global__ void __launch_bounds__(kFxTpb, KIND == kFxSS ? 4 : 1) rpy_fx_kernel(c
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-static int words_of(int kind) { return (kind == kSS || kind == kBS) ? 10 : 8; }
+static int quads_of(int kind) { return (kind == kSS || kind == kBS) ? 6 : 4; }
 static int nout_of(int kind) { return (kind == kBB || kind == kBS) ? 3 : 6; }
 
-size_t fx_record_bytes(int kind) { return (size_t)words_of(kind) * 8; }
+size_t fx_record_bytes(int kind) { return (size_t)quads_of(kind) * 16; }
 
 bool fx_supported(int kind, double as, double ab, double mu)
 {
@@ -340,7 +358,7 @@ bool fx_supported(int kind, double as, double ab, double mu)
 }
 
 using FxPairFn = void (*)(FxLaunch);
-using FxPackFn = void (*)(const double *, const double *, int, FxConsts, unsigned long long *, const int *);
+using FxPackFn = void (*)(const double *, const double *, int, FxConsts, int4 *, const int *);
 
 template <bool kInline> static FxPairFn pair_fn(int kind)
 {
@@ -353,24 +371,22 @@ static FxPackFn pack_fn(int kind)
          : kind == kSB ? fx_pack_kernel<kFxSB> : fx_pack_kernel<kFxBS>;
 }
 
-// Sources per split, a power of two.  Measured on M_ss and M_bb of 60 to
+// Sources per split, a power of two.  Measured on M_ss and M_bb of 200 to
 // 12,800 particles (152 SMs): with work enough, the largest split that still
 // gives 24 CTAs per SM, so that the last CTAs to finish idle the chip for
-// little of the launch (4096 blobs: 128 sources 232 us, 256 240, 1024 287;
-// 12,800 segments: 1024 sources 3.92 ms, 128 3.95); below that whole tiles
-// while they give 13 (3000 segments: 128 262 us, 64 275), then parts of a tile,
-// whose CTAs have less to do than to set up: 64 or 32 (962 segments: 64 49 us,
-// 32 51; 642: 32 29 us, 64 33, 128 39), and 16 or 8 while the CTAs still find an
-// SM each (100 blobs: 8 10.3 us, 32 12.3; 320 segments: 32 20.5 us, 8 24.6).
+// little of the launch (4096 segments: 128 sources 339 us, 1024 407; 12,800:
+// 1024 sources 2.79 ms, 128 2.86, 2048 2.82); below that a tile, down to 1.5
+// CTAs per SM (2000 segments: 128 111 us, 64 117; 962: 41 against 49); then
+// parts of a tile, whose CTAs have less to do than to set up (642: 32 28 us,
+// 64 29, 128 33), and 16 or 8 while the CTAs still find an SM each (200: 16
+// 16.5 us, 8 and 32 18.5; 320: 32 18.5 us, 16 20.5, 8 24.6).
 static int fx_chunk(int groups, int n_src, int sm_count, int most_splits)
 {
     const auto splits = [&](long long chunk) { return ((long long)n_src + chunk - 1) / chunk; };
     const auto ctas = [&](long long chunk) { return (double)groups * (double)splits(chunk) / sm_count; };
     long long chunk = kFxTile;
-    if (ctas(kFxTile) >= 24.0)
-        while (ctas(2 * chunk) >= 24.0) chunk *= 2;
-    else if (ctas(kFxTile) < 13.0)
-        chunk = ctas(64) >= 2.7 ? 64 : ctas(8) <= 1.2 ? 8 : ctas(16) <= 1.2 ? 16 : 32;
+    while (ctas(2 * chunk) >= 24.0) chunk *= 2;
+    if (ctas(kFxTile) < 1.5) chunk = ctas(64) >= 2.0 ? 64 : ctas(8) <= 0.5 ? 8 : ctas(16) <= 1.0 ? 16 : 32;
     while (splits(chunk) > std::min(most_splits, 65535)) chunk *= 2;
     return (int)std::min<long long>(chunk, 1 << 30);
 }
@@ -412,7 +428,7 @@ gmi_status launch_pair_fx(const FxPairSum &s, int *launched)
     a.xt = s.xt;
     a.xs = s.xs;
     a.fs = s.fs;
-    a.rec = static_cast<const unsigned long long *>(s.rec);
+    a.rec = static_cast<const int4 *>(s.rec);
     a.tgt_start = s.tgt_start;
     a.n_tgt = s.n_tgt;
     a.n_src = s.n_src;
@@ -427,8 +443,8 @@ gmi_status launch_pair_fx(const FxPairSum &s, int *launched)
     const bool packs_itself = a.chunk <= kFxTile && (long long)groups * splits <= kFxInlinePerSm * s.sm_count;
     *launched = packs_itself ? 1 : 2;
     if (!packs_itself)
-        GMI_CUDA_TRY(launch_chained(s.pdl != 0, pack_fn(s.kind), dim3((s.n_src + kFxTile - 1) / kFxTile), dim3(kFxTile),
-                                    s.stream, a.xs, a.fs, s.n_src, a.K, static_cast<unsigned long long *>(s.rec), a.skip));
+        GMI_CUDA_TRY(launch_chained(s.pdl != 0, pack_fn(s.kind), dim3((s.n_src + kFxBlock - 1) / kFxBlock), dim3(kFxBlock),
+                                    s.stream, a.xs, a.fs, s.n_src, a.K, static_cast<int4 *>(s.rec), a.skip));
     GMI_CUDA_TRY(launch_chained(s.pdl != 0 || !packs_itself, packs_itself ? pair_fn<true>(s.kind) : pair_fn<false>(s.kind),
                                 dim3(groups, splits), dim3(kFxTpb), s.stream, a));
     if (s.splits_out) {

@@ -714,6 +714,26 @@ __global__ void reduce_splits(const double *__restrict__ partial, int splits, in
     out[e] = s;
 }
 
+// The same for the FP64 sums, whose splits are many and short: eight at a time
+// as a tree, so that eight loads are in flight and an eighth of the additions
+// round at the size of the whole sum.  Error of M_ss above the wall at 300
+// segments (75 splits) against extended precision: 3.3e-16 in order, 2.2e-16.
+__global__ void __launch_bounds__(64) reduce_splits_tree(const double *__restrict__ partial, int splits, int count,
+                                                         double *__restrict__ out, int accumulate)
+{
+    pdl_wait();
+    const int e = blockIdx.x * 64 + threadIdx.x;
+    if (e >= count) return;
+    double s = 0.0;
+    for (int p0 = 0; p0 < splits; p0 += 8) {
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = p0 + k < splits ? partial[(size_t)(p0 + k) * count + e] : 0.0;
+        s += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
+    out[e] = accumulate ? out[e] + s : s;
+}
+
 // ---------------------------------------------------------------------------
 // 2b. small problems (up to a few thousand sources): one warp per TPW
 // targets, its 32 lanes stride over the sources with direct vector loads
@@ -1766,8 +1786,8 @@ gmi_status launch_pair(gmi_context *ctx, int kind, const void *tgt_rec, int tgt_
 // One pair sum of positions and loads in the reference's layouts, by the
 // kernel of the context's precision.  FP64 takes the wall kernel or, without a
 // wall, the fixed-point kernel, at every size: against the FP64 kernels M_ss of 320
-// segments went from 61 to 22.5 us, of 12,800 from 20.4 to 3.9 ms, M_bb of
-// 4096 blobs from 1222 to 231 us.  The FP64 kernels keep radii that the
+// segments went from 61 to 16.4 us, of 12,800 from 20.4 to 2.81 ms, M_bb of
+// 4096 blobs from 1223 to 188 us.  The FP64 kernels keep radii that the
 // fixed-point formats do not hold, and shapes pinned by gmi_set_shape.
 gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt, int tgt_start, int n_tgt,
                     const double *xs, const double *fs, int n_src, double as, double ab, double mu, double *out,

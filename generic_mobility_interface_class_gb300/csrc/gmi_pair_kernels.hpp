@@ -103,6 +103,7 @@ struct ExplicitPairEnv {
 // (a no-op when skip is given and set).
 __global__ void reduce_splits(const double *partial, int splits, int count, double *out, int accumulate,
                               const int *skip);
+__global__ void reduce_splits_tree(const double *partial, int splits, int count, double *out, int accumulate);
 size_t record_bytes(bool f64);
 gmi_status pack_records_into(cudaStream_t stream, bool f64, const double *x, const double *f, int nf, int n,
                              void *dst);

@@ -1,6 +1,5 @@
 // gmi_pairs_fx.cuh -- the RPY pair sums in the fixed-point arithmetic of
-// gmi_fx.cuh: FP64-grade results (a term is rounded at 2^-56 of its source's
-// load) on the integer multiply pipe.
+// gmi_fx.cuh: FP64-grade results on the integer and FP32 pipes.
 //
 // Units.  U is the largest power of two not above the smaller radius.
 // Positions are 64-bit integers of 2^-51 U relative to an origin near the
@@ -9,17 +8,22 @@
 // lies in [1, 3.47).  A source's loads share one exponent: force components
 // and torque components over U are fractions of 2^e.  Sums are formed in
 // units of 2^e / (8 pi mu U) (velocity) and 2^e / (8 pi mu U^2) (angular
-// velocity):
-//   far:  v = 2^-k  [ A F + B (d'.F) d' + C T''x d' ]
-//         w = 2^-2k [ -C/2 T'' + Br (d'.T'') d' + C F x d' ],   T'' = 2^-k T
+// velocity), with the unit vector e' = d' / r' and T'' = 2^-k T:
+//   far:  v = 2^-k  [ A F + B (e'.F) e' + C T'' x e' ]
+//         w = 2^-2k [ Ar T'' + Br (e'.T'') e' + C F x e' ]
+//         A = (1 + t)/r', B = (1 - 3t)/r', t = (as^2 + ab^2)/(3 r^2),
+//         C = 1/r'^2, Ar = -1/(2 r'^3), Br = 3/(2 r'^3)
 //   near: the same without the powers of two, with the near-field scalars.
 // The formulas are those of gmi_pairs.cuh, which cites the reference kernels.
+// d' has scale 29, everything after it is below 2 and has scale 30, and every
+// term of v and w scale 60.
 //
-// Accumulation.  A term P (2^-56) enters as its limbs times 2^(26 - s), s the
-// term's shift (k or 2k plus the source's exponent gap, at most 26): two
-// integer multiply-adds instead of a variable shift and a three-word add,
-// and nothing is rounded.  |P| < 8, so 32 terms keep both 64-bit
-// accumulators below 2^62; the caller folds them into FP64 by then.
+// Accumulation.  A term's integer part enters by its two words times
+// 2^(24 - s), s the term's shift (k or 2k plus the source's exponent gap, at
+// most 24): two integer multiply-adds instead of a variable shift and a
+// three-word add.  Its FP32 part enters an FP32 sum, which fx_settle adds to a
+// compensated one every kFxSettle terms.  |term| < 8, so 128 terms keep the
+// 64-bit accumulators in range; the caller folds them into FP64 by then.
 #pragma once
 
 #include <math.h>
@@ -29,9 +33,13 @@
 namespace gmi {
 
 constexpr int kFxPosBits = 51;     // position quantum 2^-51 U
-constexpr int kFxAccBits = 26;     // a term without shift enters times 2^26
-constexpr int kFxMaxGap = 8;       // exponent gap of a source within its tile
-constexpr int kFxFold = 32;        // terms between folds
+constexpr int kFxAccBits = 24;     // a term without shift enters times 2^24
+constexpr int kFxMaxGap = 6;       // exponent gap of a source within its block
+constexpr int kFxFold = 128;       // terms between folds
+// Terms between fx_settle: the running FP32 parts are a quarter of the error
+// of a few hundred particles' sum; every 4 instead of 8 takes 1.3 % longer.
+// The blobs' sum over segments has the largest terms next to its total.
+constexpr int kFxSettle[5] = {4, 4, 4, 4, 2};  // by FxKind
 constexpr double kFxPosLimit = 1152921504606845952.0;  // 2^60 - 2^10: |position| stays below
 
 enum FxKind : int { kFxSS = 0, kFxBB = 2, kFxSB = 3, kFxBS = 4 };  // as PairKind
@@ -40,30 +48,41 @@ struct FxConsts {
     double pos_scale;          // 2^51 / U
     double unit, inv_unit;     // U, 1/U
     double vscale, wscale;     // 1/(8 pi mu U), 1/(8 pi mu U^2)
+    double vscale_fix;         // their common relative error: exact = rounded * (1 + fix)
     double as, ab, inv_as;     // radii (equal kinds: both the one radius)
     double a0, ar0;            // near field: 4U/(3a) (unequal: 4U/(3 as ab)), (U/a)^3
-    fx k3;                     // far field: (as^2 + ab^2) / (3 U^2)
-    long long t4;              // near up to r^2 = t4 U^2 (2^-56): (as + ab)^2
-    long long a_zero;          // A at r = 0: 4U / (3 max(as, ab))
-    long long bb_b;            // blob-blob near field: (U/a)^2 / 8
-    fx bb_a1;                  // and 3 (U/a)^2 / 8
+    fxop k3;                   // far field: (as^2 + ab^2) / (3 U^2)
+    long long t4;              // near up to r^2 = t4 U^2 (2^-58): (as + ab)^2
+    fxop a_zero, ar_zero;      // at r = 0: A = 4U / (3 max(as, ab)), Ar = (U/a)^3
+    fxop bb_b;                 // blob-blob near field: (U/a)^2, an eighth of it at scale 33
 };
 
 struct FxSource {
     long long X[3];
-    fx F[3];
-    long long T[3];  // torques over U, 2^-60
-    int gap;         // the tile's exponent less the source's, <= kFxMaxGap
+    fxop F[3];
+    long long T[3];  // torques over U, 2^-62
+    int gap;         // the block's exponent less the source's, <= kFxMaxGap
 };
 
-GMI_FX_HD long long fx_from_double(double v)  // 2^-60, |v| < 8
+// One target's accumulators, in 2^(-60 - 24) of the block's unit: H 2^32 + L,
+// and the FP32 parts x, settled into xh + xl.
+template <int N> struct FxAcc {
+    long long H[N];
+    unsigned long long L[N];
+    float x[N], xh[N], xl[N];
+};
+
+GMI_FX_HD long long fx_rint(double v)
 {
 #ifdef __CUDA_ARCH__
-    return __double2ll_rn(v * 1152921504606846976.0);
+    return __double2ll_rn(v);
 #else
-    return (long long)llrint(v * 1152921504606846976.0);
+    return (long long)llrint(v);
 #endif
 }
+
+// v (|v| < 2) as a value of scale 30
+GMI_FX_HD fxop fx_from_double(double v) { return fx_split(fx_rint(v * 4611686018427387904.0)); }
 
 GMI_FX_HD double fx_exp2(int e)  // 2^e, -1022 <= e <= 1023
 {
@@ -75,56 +94,59 @@ GMI_FX_HD double fx_exp2(int e)  // 2^e, -1022 <= e <= 1023
     return c.d;
 }
 
-// The scalars of one pair in 2^-60: A of F, B of (d'.F) d', C of the cross
-// products, Ar of T'', Br of (d'.T'') d'.
+// The scalars of one pair: A of F, B of (e'.F) e', C of the cross products, Ar
+// of T'', Br of (e'.T'') e'.
 struct FxScalars {
-    long long A, B, C, Ar, Br;
+    fxop A, B, C, Ar, Br;
 };
 
-// Near-field scalars of the segment kinds in FP64 (few pairs get here):
-// r' and 1/r'^2 from the fixed-point separation, 2^k U the separation's unit.
+// Near-field scalars of the segment kinds in FP64 (few pairs get here), at r = ru U.
 template <int KIND>
 #ifdef __CUDACC__
 __host__ __device__ __noinline__
 #endif
-FxScalars fx_near_scalars(long long r2, long long ir, int k, const FxConsts &K)
+FxScalars fx_near_scalars(double ru, const FxConsts &K)
 {
-    const double ird = (double)ir * (1.0 / 1152921504606846976.0);
-    const double rp = (double)r2 * (1.0 / 72057594037927936.0) * ird;  // r'
-    const double ru = rp * fx_exp2(k);             // r / U
-    const double ir2 = ird * ird;
+    const fxop none{0, 0.0f, 0.0f};
     FxScalars s;
     if (KIND == kFxSS) {
         const double rho = ru * K.unit * K.inv_as, q = rho * (1.0 / 32.0), rho3 = rho * rho * rho;
         s.A = fx_from_double(K.a0 - K.a0 * 9.0 * q);
-        s.B = fx_from_double(K.a0 * 3.0 * q * ir2);
+        s.B = fx_from_double(K.a0 * 3.0 * q);
         s.Ar = fx_from_double(K.ar0 * (1.0 - 27.0 * q + (5.0 / 64.0) * rho3));
-        s.Br = fx_from_double(K.ar0 * (9.0 * q - (3.0 / 64.0) * rho3) * ir2);
-        s.C = fx_from_double(0.5 * K.ar0 * ru * (1.0 - 12.0 * q) * ird);
+        s.Br = fx_from_double(K.ar0 * (9.0 * q - (3.0 / 64.0) * rho3));
+        s.C = fx_from_double(0.5 * K.ar0 * ru * (1.0 - 12.0 * q));
         return s;
     }
-    s.Ar = s.Br = 0;
+    s.Ar = s.Br = none;
     const double r = ru * K.unit, dm = K.as - K.ab;
     if (r > fabs(dm)) {
         const double i3 = 1.0 / (32.0 * r * r * r), dm2 = dm * dm, r2d = r * r;
         const double t = dm2 + 3.0 * r2d, b = dm2 - r2d, u = dm + r;
         const double p = K.ab * K.ab + 2.0 * K.ab * (r + K.as) - 3.0 * (K.as - r) * (K.as - r);
         s.A = fx_from_double(K.a0 * (0.5 * (K.as + K.ab) - t * t * i3));
-        s.B = fx_from_double(K.a0 * 3.0 * b * b * i3 * ir2);
-        s.C = fx_from_double(K.unit * K.unit * u * u * p / (16.0 * K.ab * K.as * K.as * K.as * r2d) * ird);
+        s.B = fx_from_double(K.a0 * 3.0 * b * b * i3);
+        s.C = fx_from_double(K.unit * K.unit * u * u * p / (16.0 * K.ab * K.as * K.as * K.as * r2d));
     } else {
-        const double amax = K.as > K.ab ? K.as : K.ab;
-        s.A = fx_from_double(K.unit * 4.0 / (3.0 * amax));
-        s.B = 0;
-        s.C = K.as > K.ab ? fx_from_double(K.unit * K.unit * r / (K.as * K.as * K.as) * ird) : 0;
+        s.A = K.a_zero;
+        s.B = none;
+        s.C = K.as > K.ab ? fx_from_double(K.unit * K.unit * r / (K.as * K.as * K.as)) : none;
     }
     return s;
 }
 
-// One source's contribution to one target's accumulators (H: 2^32, L: 1, both
-// times 2^(-56 - 26) of the tile's unit).
-template <int KIND>
-GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K, long long *H, long long *L)
+// (h, x) 2^k, by shifts (k <= 1)
+GMI_FX_HD fxsum fx_scale(fxsum s, int k)
+{
+    const int dn = k < -62 ? 62 : -k;
+    s.h = k > 0 ? (long long)((unsigned long long)s.h << k) : s.h >> dn;
+    s.x *= fx_as_float((127 + (k < -126 ? -126 : k)) << 23);
+    return s;
+}
+
+// One source's contribution to one target's accumulators.
+template <int KIND, int N>
+GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K, FxAcc<N> &acc)
 {
     constexpr bool kTorque = KIND == kFxSS || KIND == kFxBS;  // sources carry torques
     constexpr bool kAngular = KIND == kFxSS || KIND == kFxSB; // targets turn
@@ -147,122 +169,138 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
         }
         zero = mx == 0;
         if (zero) D[0] = 1;
-        sl = zero ? 60 : fx_clzll(mx) - 3;
+        sl = zero ? 61 : fx_clzll(mx) - 2;
     } else {
-        sl = fx_clz((unsigned)m) - 3;  // the leading bit moves to 2^60 (one place off for a negative power of two)
+        sl = fx_clz((unsigned)m) - 2;  // the leading bit moves to 2^61 (one place off for a negative power of two)
     }
-    const int k = 60 - kFxPosBits - sl;
-    fx d[3];
-    for (int c = 0; c < 3; ++c) d[c] = fx_split((long long)((unsigned long long)D[c] << sl));
-    // r'^2 in 2^-56
-    fxacc s{0, 0};
+    const int k = 61 - kFxPosBits - sl;
+    fxop d[3];
+    for (int c = 0; c < 3; ++c) d[c] = fx_split((long long)((unsigned long long)D[c] << sl));  // scale 29
+    fxsum s{0, 0.0f};  // r'^2, scale 58
     for (int c = 0; c < 3; ++c) {
-        s.h = fx_madw(d[c].hi, d[c].hi, s.h);
-        s.x = fx_madw(d[c].hi, d[c].lo, s.x);
+        s.h = fx_madw(d[c].h, d[c].h, s.h);
+        s.x = fmaf(d[c].hf, d[c].lf, s.x);
     }
-    const long long r2 = s.h + (s.x >> 31);
-    const long long irq = fx_rsqrt(r2);
-    const fx ir = fx_split(irq);
+    s.x *= 2.0f;
+    const fxop ir = fx_rsqrt(s.h, s.x);  // 30
+    const bool near = k < 0 || (k <= 2 && s.h <= (K.t4 >> (2 * k)));
 
-    FxScalars g;
+    fxop e[3];
+    for (int c = 0; c < 3; ++c) e[c] = fx_product<29>(d[c], ir);
+
+    FxScalars g;  // far field
     int kk = k;
-    const bool near = k < 0 || (k <= 2 && r2 <= (K.t4 >> (2 * k)));
-    // far field: A = (1 + t)/r', B = (1 - 3t)/r'^3, t = (as^2 + ab^2)/(3 r^2)
     {
-        s = fxacc{fx_madw(ir.hi, ir.hi, 0), fx_madw(ir.hi, ir.lo, 0)};
-        const fx ir2 = fx_split((s.h << 4) + (s.x >> 27));
-        const long long c3 = fx_mul60(ir, ir2);
+        const fxop ir2 = fx_close<30>(fx_madw(ir.h, ir.h, 0), 2.0f * (ir.hf * ir.lf));
+        const fxsum u = fx_mul(K.k3, ir2);  // 28 + 30
         const int k2 = near ? 0 : 2 * k;
-        const fx t = fx_split(fx_mul60(K.k3, ir2) >> k2);
-        const fx c3f = fx_split(c3);
-        g.A = irq + fx_mul60(ir, t);
-        g.B = c3 - 3 * fx_mul60(c3f, t);
-        g.C = c3;
+        const fxop t = fx_close<28>(u.h >> k2, u.x * fx_as_float((127 - k2) << 23));
+        const fxop p = fx_product_low<30>(ir, t);
+        g.A = fx_add(ir, 1, p);
+        g.B = fx_add(ir, -3, p);
+        g.C = ir2;
         if (KIND == kFxSS) {
-            const long long c5 = fx_mul60(c3f, ir2);
-            g.Ar = -(c3 >> 1);
-            g.Br = c5 + (c5 >> 1);
+            const fxop c3 = fx_product<31>(ir, ir2);  // r'^-3 of scale 29, so half of it of scale 30
+            g.Ar = fx_neg(c3);
+            g.Br = fx_add(fxop{0, 0.0f, 0.0f}, 3, c3);
         }
     }
     if (near) {
         kk = 0;
         if (zero) {  // r -> 0
             g.A = K.a_zero;
-            g.B = g.Br = g.C = 0;
-            g.Ar = KIND == kFxSS ? fx_from_double(K.ar0) : 0;
+            g.B = g.Br = g.C = fxop{0, 0.0f, 0.0f};
+            g.Ar = K.ar_zero;
         } else if (KIND == kFxBB) {
-            // A = 4U/(3a) (1 - 9r/(32a)), B = (U/a)^2 2^k / (8 r')
-            const int rh = (int)(r2 >> 32);  // 2^-24
-            const long long rx = (long long)ir.lo * rh + (long long)((unsigned long long)(unsigned)r2 * (unsigned)ir.hi);
-            const long long rp = (((long long)ir.hi * rh) << 8) + (rx >> 24);  // r' = r'^2 / r'
-            const int dn = k < 0 ? (k < -62 ? 62 : -k) : 0, up = k < 0 ? 0 : k;
-            const fx ru = fx_split((rp << up) >> dn);  // r / U < 4
-            g.A = K.a_zero - fx_mul60(K.bb_a1, ru);
-            g.B = (fx_mul60(fx_split(K.bb_b), ir) << up) >> dn;
+            // B = (U/a)^2 r / (8 U), A = 4U/(3a) - 3 B
+            fxop r2 = fx_split(s.h);  // 26
+            r2.lf = fmaf(s.x, 1.0f / 4294967296.0f, r2.lf);
+            const fxop rp = fx_product<28>(r2, ir);           // r', 28
+            const fxsum u = fx_scale(fx_mul(K.bb_b, rp), k);  // 33 + 28
+            g.B = fx_close<31>(u.h, u.x);
+            g.A = fx_add(K.a_zero, -3, g.B);
         } else {
-            g = fx_near_scalars<KIND>(r2, irq, k, K);
+            const double ird = ((double)ir.h + (double)ir.lf * (1.0 / 4294967296.0)) * (1.0 / 1073741824.0);
+            const double r2 = ((double)s.h + (double)s.x * (1.0 / 4294967296.0)) * (1.0 / 288230376151711744.0);
+            g = fx_near_scalars<KIND>(r2 * ird * fx_exp2(k), K);
         }
     }
 
     // dot products and loads
-    fxacc q{0, 0};
-    for (int c = 0; c < 3; ++c) fx_mac(q, d[c], S.F[c]);
-    const fx dF = fx_split(fx_q60(q));
-    const fx A = fx_split(g.A), Bt = fx_split(fx_mul60(fx_split(g.B), dF));
-    fx T[3], cp[3], cn[3], Ar, Br;
-    if (kCross) {
-        const fx C = fx_split(g.C);
+    fxsum q{0, 0.0f};
+    for (int c = 0; c < 3; ++c) fx_mac(q, e[c], S.F[c]);
+    const fxop Bt = fx_product<30>(g.B, fx_close<30>(q.h, q.x));
+    fxop T[3], cp[3], cn[3], Br;
+    if (kCross)
         for (int c = 0; c < 3; ++c) {
-            cp[c] = fx_split(fx_mul60(C, d[c]));
-            cn[c] = fx{-cp[c].hi, ~cp[c].lo};  // -cp but for one unit of 2^-60 (and no -2^31 to negate)
+            cp[c] = fx_product<30>(e[c], g.C);
+            cn[c] = fx_neg(cp[c]);
         }
-    }
     if (kTorque)
         for (int c = 0; c < 3; ++c) T[c] = fx_split(S.T[c] >> kk);
     if (KIND == kFxSS) {
-        q = fxacc{0, 0};
-        for (int c = 0; c < 3; ++c) fx_mac(q, d[c], T[c]);
-        Ar = fx_split(g.Ar);
-        Br = fx_split(fx_mul60(fx_split(g.Br), fx_split(fx_q60(q))));
+        q = fxsum{0, 0.0f};
+        for (int c = 0; c < 3; ++c) fx_mac(q, e[c], T[c]);
+        Br = fx_product<30>(g.Br, fx_close<30>(q.h, q.x));
     }
-    const int mv = 1 << (kFxAccBits - S.gap - kk);
-    const int mw = 1 << (kFxAccBits - S.gap - 2 * kk);
-    constexpr long long kRoundP = 1ll << 31;  // of x's shift, and of the split of P
+    const int sv = S.gap + kk, sw = S.gap + 2 * kk;
+    const int mv = 1 << (kFxAccBits - sv), mw = 1 << (kFxAccBits - sw);
+    const float fv = fx_as_float((127 + kFxAccBits - 32 - sv) << 23);
+    const float fw = fx_as_float((127 + kFxAccBits - 32 - sw) << 23);
     for (int c = 0; c < 3; ++c) {
         const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
-        q = fxacc{kRoundP, kRoundP};
-        fx_mac(q, A, S.F[c]);
-        fx_mac(q, Bt, d[c]);
+        q = fx_mul(g.A, S.F[c]);
+        fx_mac(q, Bt, e[c]);
         if (kTorque) {
             fx_mac(q, T[c1], cp[c2]);
             fx_mac(q, T[c2], cn[c1]);
         }
-        const long long P = q.h + (q.x >> 32);
-        H[c] = fx_madw((int)(P >> 32), mv, H[c]);
-        L[c] = fx_madw((int)((unsigned)P ^ 0x80000000u), mv, L[c]);
+        acc.H[c] = fx_madw((int)(q.h >> 32), mv, acc.H[c]);
+        acc.L[c] = fx_madw_u((unsigned)q.h, (unsigned)mv, acc.L[c]);
+        acc.x[c] = fmaf(q.x, fv, acc.x[c]);
     }
     if (kAngular)
         for (int c = 0; c < 3; ++c) {
-            const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
-            q = fxacc{kRoundP, kRoundP};
-            if (KIND == kFxSS) {
-                fx_mac(q, Ar, T[c]);
-                fx_mac(q, Br, d[c]);
-            }
-            fx_mac(q, S.F[c1], cp[c2]);
+            const int c1 = (c + 1) % 3, c2 = (c + 2) % 3, o = N == 6 ? 3 + c : c;
+            q = fx_mul(S.F[c1], cp[c2]);
             fx_mac(q, S.F[c2], cn[c1]);
-            const long long P = q.h + (q.x >> 32);
-            H[3 + c] = fx_madw((int)(P >> 32), mw, H[3 + c]);
-            L[3 + c] = fx_madw((int)((unsigned)P ^ 0x80000000u), mw, L[3 + c]);
+            if (KIND == kFxSS) {
+                fx_mac(q, g.Ar, T[c]);
+                fx_mac(q, Br, e[c]);
+            }
+            acc.H[o] = fx_madw((int)(q.h >> 32), mw, acc.H[o]);
+            acc.L[o] = fx_madw_u((unsigned)q.h, (unsigned)mw, acc.L[o]);
+            acc.x[o] = fmaf(q.x, fw, acc.x[o]);
         }
 }
 
-// Accumulators to FP64 in final units: scale = vscale or wscale times the
-// tile's 2^E.
-GMI_FX_HD double fx_fold(long long H, long long L, double scale)
+template <int N> GMI_FX_HD void fx_clear(FxAcc<N> &a)
 {
-    const double s = scale * (1.0 / 72057594037927936.0) * (1.0 / (double)(1 << kFxAccBits));
-    return (double)H * (s * 4294967296.0) + (double)L * s;
+    for (int c = 0; c < N; ++c) {
+        a.H[c] = 0;
+        a.L[c] = 0;
+        a.x[c] = a.xh[c] = a.xl[c] = 0.0f;
+    }
+}
+
+// Knuth's two-sum of the running FP32 parts into the settled ones
+template <int N> GMI_FX_HD void fx_settle(FxAcc<N> &a)
+{
+    for (int c = 0; c < N; ++c) {
+        const float s = a.xh[c] + a.x[c], b = s - a.xh[c];
+        a.xl[c] += (a.xh[c] - (s - b)) + (a.x[c] - b);
+        a.xh[c] = s;
+        a.x[c] = 0.0f;
+    }
+}
+
+// One settled accumulator to FP64 in final units: scale = vscale or wscale
+// times the block's 2^E.
+template <int N> GMI_FX_HD double fx_fold(const FxAcc<N> &a, int c, double scale, double fix)
+{
+    const double s = scale * (1.0 / 1152921504606846976.0) * (1.0 / (double)(1 << kFxAccBits));
+    const double high = (double)a.H[c], low = (double)a.L[c] + ((double)a.xh[c] + (double)a.xl[c]);
+    return fma(high, s * 4294967296.0, fma(low, s, high * (s * 4294967296.0 * fix)));
 }
 
 // The constants of one kind; false where the formats do not hold them: the
@@ -274,23 +312,29 @@ inline bool fx_consts(int kind, double as, double ab, double mu, FxConsts *K)
     if (!(amin > 1e-60 && amax < 1e60 && mu > 1e-60 && mu < 1e60) || amax > 2.0 * amin) return false;
     int e;
     frexp(amin, &e);
-    const double U = ldexp(1.0, e - 1), f8 = 1.0 / (8.0 * 3.14159265358979323846264338327950288 * mu);
-    const double one = 1152921504606846976.0;  // 2^60
+    const double U = ldexp(1.0, e - 1);
+    // 8 pi mu in two parts: the one rounding that every velocity shares
+    const double pi = 3.14159265358979323846264338327950288, pi_low = 1.2246467991473532e-16;
+    const double d8 = 8.0 * pi * mu, d8_low = fma(8.0 * pi, mu, -d8) + 8.0 * pi_low * mu, f8 = 1.0 / d8;
     K->unit = U;
     K->inv_unit = 1.0 / U;
     K->pos_scale = ldexp(1.0, kFxPosBits) / U;
     K->vscale = f8 / U;
     K->wscale = f8 / (U * U);
+    K->vscale_fix = fma(-f8, d8, 1.0) - f8 * d8_low;
     K->as = as;
     K->ab = ab;
     K->inv_as = 1.0 / as;
     K->a0 = equal ? 4.0 * U / (3.0 * as) : 4.0 * U / (3.0 * as * ab);
     K->ar0 = (U / as) * (U / as) * (U / as);
-    K->k3 = fx_split((long long)llrint((as * as + ab * ab) / (3.0 * U * U) * one));
-    K->t4 = (long long)llrint((as + ab) * (as + ab) / (U * U) * 72057594037927936.0);
-    K->a_zero = (long long)llrint(4.0 * U / (3.0 * amax) * one);
-    K->bb_b = (long long)llrint(U * U / (8.0 * as * as) * one);
-    K->bb_a1 = fx_split((long long)llrint(3.0 * U * U / (8.0 * as * as) * one));
+    K->k3 = fx_split(fx_rint((as * as + ab * ab) / (3.0 * U * U) * 1152921504606846976.0));  // 28
+    K->t4 = fx_rint((as + ab) * (as + ab) / (U * U) * 288230376151711744.0);
+    // the self term is the largest of most sums: the quotient's remainder too
+    const double a3 = 3.0 * amax, a_zero = 4.0 * U / a3;
+    K->a_zero = fx_from_double(a_zero);
+    K->a_zero.lf += (float)((fma(-a_zero, a3, 4.0 * U) - a_zero * fma(3.0, amax, -a3)) / a3 * 4611686018427387904.0);
+    K->ar_zero = fx_from_double(K->ar0);
+    K->bb_b = fx_from_double(U * U / (as * as));
     return true;
 }
 
@@ -304,11 +348,7 @@ GMI_FX_HD bool fx_position(double x, double pos_scale, double origin, long long 
         *X = 0;
         return false;
     }
-#ifdef __CUDA_ARCH__
-    *X = fabs(t) < 4611686018427387904.0 ? __double2ll_rn(t) - (long long)origin : __double2ll_rn(rel);
-#else
-    *X = fabs(t) < 4611686018427387904.0 ? (long long)llrint(t) - (long long)origin : (long long)llrint(rel);
-#endif
+    *X = fabs(t) < 4611686018427387904.0 ? fx_rint(t) - (long long)origin : fx_rint(rel);
     return true;
 }
 

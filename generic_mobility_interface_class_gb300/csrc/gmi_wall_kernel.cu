@@ -12,7 +12,7 @@
 //
 // A CTA owns 32 targets, one per lane; its four warps take a quarter each of
 // a slice of the sources ("split"), sized so that every SM gets the same
-// number of CTAs to within a few per cent; reduce_splits adds the splits.
+// number of CTAs to within a few per cent; reduce_splits_tree adds the splits.
 // 1280 segments: 1287 us (two targets per warp, 160 CTAs on 152 SMs, so 8 of
 // them set the time) -> 480 us, at the pipe's rate for these instructions.
 #include <algorithm>
@@ -187,8 +187,8 @@ gmi_status launch_wall_fp64(cudaStream_t stream, int sm_count, const WallSum &a,
     *launched = 1;
     if (splits > 1) {
         const int count = a.n_tgt * 6;
-        GMI_CUDA_TRY(launch_chained(true, reduce_splits, dim3((count + 255) / 256), dim3(256), stream, a.partial, splits,
-                                    count, a.out, 0, nullptr));
+        GMI_CUDA_TRY(launch_chained(true, reduce_splits_tree, dim3((count + 63) / 64), dim3(64), stream, a.partial, splits,
+                                    count, a.out, 0));
         *launched = 2;
     }
     return GMI_OK;

@@ -13,7 +13,7 @@ static int sum(int nt, const double *xt, int ns, const double *xs, const double 
                double *out)
 {
     constexpr bool torque = KIND == kFxSS || KIND == kFxBS;
-    constexpr int nf = torque ? 6 : 3, nout = (KIND == kFxSS || KIND == kFxSB) ? 6 : 3, tile = 128;
+    constexpr int nf = torque ? 6 : 3, nout = (KIND == kFxSS || KIND == kFxSB) ? 6 : 3, tile = 512;
     FxConsts K;
     if (!fx_consts(KIND, as, ab, mu, &K)) return 1;
     std::vector<FxSource> src(ns);
@@ -35,8 +35,8 @@ static int sum(int nt, const double *xt, int ns, const double *xs, const double 
         src[j].gap = e[j] == kFxNoLoad ? 0 : std::min(E[j / tile] - e[j], kFxMaxGap);
         const double s = fx_exp2(e[j] == kFxNoLoad ? 0 : -(E[j / tile] - src[j].gap));
         for (int c = 0; c < 3; ++c) {
-            src[j].F[c] = fx_split(fx_from_double(f[nf * j + c] * s));
-            src[j].T[c] = torque ? fx_from_double(f[nf * j + nf - 3 + c] * K.inv_unit * s) : 0;
+            src[j].F[c] = fx_from_double(f[nf * j + c] * s);
+            src[j].T[c] = torque ? fx_rint(f[nf * j + nf - 3 + c] * K.inv_unit * s * 4611686018427387904.0) : 0;
         }
     }
     for (int i = 0; i < nt; ++i) {
@@ -45,10 +45,15 @@ static int sum(int nt, const double *xt, int ns, const double *xs, const double 
         for (int c = 0; c < 3; ++c)
             if (!fx_position(xt[3 * i + c], K.pos_scale, origin[c], &X[c])) return 2;
         for (int j0 = 0; j0 < ns; j0 += kFxFold) {
-            long long H[6] = {0, 0, 0, 0, 0, 0}, L[6] = {0, 0, 0, 0, 0, 0};
-            for (int j = j0; j < std::min(ns, j0 + kFxFold); ++j) fx_pair<KIND>(X, src[j], K, H, L);
+            FxAcc<nout> acc;
+            fx_clear(acc);
+            for (int j = j0; j < std::min(ns, j0 + kFxFold); ++j) {
+                fx_pair<KIND>(X, src[j], K, acc);
+                if ((j - j0) % kFxSettle[KIND] == kFxSettle[KIND] - 1) fx_settle(acc);
+            }
+            fx_settle(acc);
             const double s = fx_exp2(E[j0 / tile] == kFxNoLoad ? 0 : E[j0 / tile]);
-            for (int c = 0; c < nout; ++c) tot[c] += fx_fold(H[c], L[c], (c < 3 ? K.vscale : K.wscale) * s);
+            for (int c = 0; c < nout; ++c) tot[c] += fx_fold(acc, c, (c < 3 ? K.vscale : K.wscale) * s, K.vscale_fix);
         }
         for (int c = 0; c < nout; ++c) out[nout * i + c] = tot[c];
     }

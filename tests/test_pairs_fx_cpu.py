@@ -1,9 +1,10 @@
 """The fixed-point pair arithmetic (csrc/gmi_pairs_fx.cuh) against the FP64
-oracle, on the host: the formulas are plain integer C++ there and on the GPU.
+oracle, on the host: the formulas are plain C++ on integers and floats there and on
+the GPU.
 
-Tolerance: a term of the fixed-point sum is rounded at 2^-56 of its load, so
-the difference is the oracle's own, whose sums of n FP64 terms are each within
-n 2^-53 of the terms' size; n 2^-52 of the largest velocity is allowed.
+Tolerance: a term of the fixed-point sum is rounded at about 2^-55 of its load,
+so the difference is the oracle's own, whose sums of n FP64 terms are each
+within n 2^-53 of the terms' size; n 2^-52 of the largest velocity is allowed.
 """
 import ctypes
 import os

@@ -44,7 +44,7 @@ def check_all(ctx, rpy, xs, fs, xb, fb, b=1.3, bound=None):
 
 
 @pytest.mark.parametrize("ns,nb", [(1, 1), (31, 2), (32, 33), (33, 127), (127, 128), (129, 257), (320, 642),
-                                   (963, 1281), (3001, 2047)])
+                                   (511, 512), (513, 1025), (963, 1281), (3001, 2047), (1537, 4099)])
 def test_sizes_against_oracle(gpu_ctx, oracle_built, ns, nb):
     xs, fs = cloud(ns, 3)
     xb, fb = cloud(nb, 4)
