@@ -38,6 +38,17 @@ __device__ __forceinline__ void pdl_wait_then_release()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// f in FP64 by its bits.  The conversion instruction holds a warp's FP64 unit
+// for 95 cycles (measured; an FP64 addition for 76), these integer ones take
+// 11; denormals, infinities and NaN go through the conversion.
+__device__ __forceinline__ double widen(float f)
+{
+    const unsigned u = __float_as_uint(f), m = u << 1;
+    if (m - 0x01000000u >= 0xfe000000u && m != 0u) return (double)f;
+    const unsigned hi = (u & 0x80000000u) | (((u >> 3) & 0x0fffffffu) + 0x38000000u);
+    return m == 0u ? __hiloint2double((int)u, 0) : __hiloint2double((int)hi, (int)(u << 29));
+}
+
 // Upper bound for any spin on an mbarrier: by default 2 s of %globaltimer
 // (a context can set its own, gmi_context_set_wait_deadline; a launch passes
 // it by value, 0 meaning the default).  A wait that runs past it records

@@ -192,7 +192,7 @@ template <int NOUT> struct Acc<float, NOUT> {
             t[c] = 0.f;
         }
     }
-    __device__ double total(int c) const { return (double)hi[c] + (double)lo[c]; }
+    __device__ double total(int c) const { return widen(hi[c]) + widen(lo[c]); }
 };
 
 template <int KIND> struct KindTraits;
@@ -210,16 +210,18 @@ template <class R> struct KernelConsts {
     UnequalK<R> uq;
 };
 
-template <class R> __device__ __forceinline__ KernelConsts<R> convert_consts(const PairConsts &c)
+template <class R, bool kHost = true> __device__ __forceinline__ KernelConsts<R> convert_consts(const PairConsts &c)
 {
+    const auto eq = [&](int i) -> R { if constexpr (sizeof(R) == 4 && kHost) return c.eqf[i]; else return (R)c.eq[i]; };
+    const auto uq = [&](int i) -> R { if constexpr (sizeof(R) == 4 && kHost) return c.uqf[i]; else return (R)c.uq[i]; };
     KernelConsts<R> k;
-    k.eq.four_a2 = (R)c.eq[0]; k.eq.two_a2 = (R)c.eq[1]; k.eq.f8pm = (R)c.eq[2]; k.eq.f6pma = (R)c.eq[3];
-    k.eq.q32 = (R)c.eq[4]; k.eq.inv_a = (R)c.eq[5]; k.eq.f8pma3 = (R)c.eq[6]; k.eq.f16pma3 = (R)c.eq[7];
-    k.eq.q8 = (R)c.eq[8];
-    k.uq.sum2 = (R)c.uq[0]; k.uq.dmin2 = (R)c.uq[1]; k.uq.far_c = (R)c.uq[2]; k.uq.half_sum = (R)c.uq[3];
-    k.uq.f8pm = (R)c.uq[4]; k.uq.f6pmab = (R)c.uq[5]; k.uq.fmax = (R)c.uq[6]; k.uq.c_mid_den = (R)c.uq[7];
-    k.uq.ab = (R)c.uq[8]; k.uq.as = (R)c.uq[9]; k.uq.ab2 = (R)c.uq[10]; k.uq.inner_c = (R)c.uq[11];
-    k.uq.dmin = (R)c.uq[12];
+    k.eq.four_a2 = eq(0); k.eq.two_a2 = eq(1); k.eq.f8pm = eq(2); k.eq.f6pma = eq(3);
+    k.eq.q32 = eq(4); k.eq.inv_a = eq(5); k.eq.f8pma3 = eq(6); k.eq.f16pma3 = eq(7);
+    k.eq.q8 = eq(8);
+    k.uq.sum2 = uq(0); k.uq.dmin2 = uq(1); k.uq.far_c = uq(2); k.uq.half_sum = uq(3);
+    k.uq.f8pm = uq(4); k.uq.f6pmab = uq(5); k.uq.fmax = uq(6); k.uq.c_mid_den = uq(7);
+    k.uq.ab = uq(8); k.uq.as = uq(9); k.uq.ab2 = uq(10); k.uq.inner_c = uq(11);
+    k.uq.dmin = uq(12);
     return k;
 }
 
@@ -578,7 +580,9 @@ __global__ void __launch_bounds__(TPB) rpy_pair2_kernel(const __grid_constant__ 
         }
     }
 
-    const KernelConsts<float> K = convert_consts<float>(args.k);
+    // M_ss converts its constants here: as parameters they cost the long sums
+    // more than the conversions do (131,072 segments: 32.4 ms, 32.2 this way)
+    const KernelConsts<float> K = convert_consts<float, KIND != kSS>(args.k);
     SSCoeffs self{};
     if constexpr (KIND == kSS) self = ss_self2(K.eq);
     // loads enter the packed formulas times 1/(8 pi mu) (gmi_pairs2.cuh)
@@ -745,11 +749,34 @@ __global__ void __launch_bounds__(64) reduce_splits_tree(const double *__restric
 constexpr int kWarpCta = 128;  // threads per CTA of the warp kernel
 constexpr int kWarpFold = 32;
 
-__device__ __forceinline__ double warp_sum_d(double v)
+// The sums over the warp of v[0..NOUT) (3 or 6), component c = warp_sums_slot
+// of the lane: the halving tree of a shuffle reduction, every level of which
+// also halves the components a lane carries, so 8 additions in place of 30
+// (6 of 15 for three components).
+template <int NOUT> __device__ __forceinline__ double warp_sums(const double *v)
 {
+    constexpr int H = NOUT == 6 ? 4 : 2;
+    const unsigned full = 0xffffffffu;
+    const bool h16 = (threadIdx.x & 16) != 0, h8 = (threadIdx.x & 8) != 0, h4 = (threadIdx.x & 4) != 0;
+    double b[H];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
+    for (int j = 0; j < H; ++j) {
+        const double low = v[j], high = j + H < NOUT ? v[j + H] : 0.0;
+        b[j] = (h16 ? high : low) + __shfl_xor_sync(full, h16 ? low : high, 16);
+    }
+#pragma unroll
+    for (int j = 0; j < H / 2; ++j) b[j] = (h8 ? b[j + H / 2] : b[j]) + __shfl_xor_sync(full, h8 ? b[j] : b[j + H / 2], 8);
+    double s = NOUT == 6 ? (h4 ? b[1] : b[0]) + __shfl_xor_sync(full, h4 ? b[0] : b[1], 4)
+                         : b[0] + __shfl_xor_sync(full, b[0], 4);
+    s += __shfl_xor_sync(full, s, 2);
+    s += __shfl_xor_sync(full, s, 1);
+    return s;
+}
+// The component this lane's warp_sums holds, or -1 (one lane writes each).
+template <int NOUT> __device__ __forceinline__ int warp_sums_slot()
+{
+    const int lane = threadIdx.x & 31, step = NOUT == 6 ? 4 : 8;
+    return lane % step == 0 && lane / step < NOUT ? lane / step : -1;
 }
 
 template <int KIND, class R, int TPW>
@@ -790,11 +817,12 @@ __global__ void __launch_bounds__(kWarpCta) rpy_pair_warp_kernel(const PairLaunc
         acc[k].fold();
         double v[NOUT];
 #pragma unroll
-        for (int c = 0; c < NOUT; ++c) v[c] = warp_sum_d(acc[k].total(c));
-        if (lane == 0 && t0 + k < args.n_tgt) {
-            double *o = args.out + (size_t)(t0 + k) * NOUT;
-#pragma unroll
-            for (int c = 0; c < NOUT; ++c) o[c] = args.accumulate ? o[c] + v[c] : v[c];
+        for (int c = 0; c < NOUT; ++c) v[c] = acc[k].total(c);
+        const double sum = warp_sums<NOUT>(v);
+        const int c = warp_sums_slot<NOUT>();
+        if (c >= 0 && t0 + k < args.n_tgt) {
+            double *o = args.out + (size_t)(t0 + k) * NOUT + c;
+            *o = args.accumulate ? *o + sum : sum;
         }
     }
 }
@@ -1382,6 +1410,8 @@ void fill_consts(PairConsts &c, double a_eq, double as, double ab, double mu)
     c.uq[10] = ab * ab;
     c.uq[11] = (as > ab ? 1.0 : 0.0) / (8.0 * pi * mu * as * as * as);
     c.uq[12] = dmin;
+    for (int i = 0; i < 9; ++i) c.eqf[i] = (float)c.eq[i];
+    for (int i = 0; i < 13; ++i) c.uqf[i] = (float)c.uq[i];
 }
 
 gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int nf, int n, DeviceBuffer &buf,

@@ -7,9 +7,13 @@ namespace gmi {
 
 // Physical constants of one pair kind, precomputed on the host in FP64
 // (converted to the kernel's scalar type on the device).
+// The FP32 kernels' constants are rounded on the host: a warp's conversion
+// from FP64 takes as long as one of its FP64 instructions, and every warp of a
+// launch had 9 to 13 of them to make (4096 blobs: 2 us).
 struct PairConsts {
     double eq[9];   // equal radii: see EqualK
     double uq[13];  // segment/blob radii: see UnequalK
+    float eqf[9], uqf[13];
 };
 
 struct PairLaunch {
