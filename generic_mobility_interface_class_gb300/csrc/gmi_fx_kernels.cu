@@ -22,12 +22,16 @@
 // alone (530 instructions, 146 of them wide multiplies) took 1.8 cycles each.
 // FP64 kernel -> integer limbs -> limb and FP32 (this one):
 //   12,800 segments                  20.4 -> 3.90 -> 2.81 ms  (5.1 TFLOP/s at 87 flop a pair)
-//   4096 blobs                       1223 -> 229 -> 188 us
+//   4096 blobs                       1223 -> 229 -> 178 us
 //   12,800 segments, 4096 blobs,
-//   both ways                        9.72 -> 1.80 -> 1.40 ms
+//   both ways                        9.72 -> 1.80 -> 1.36 ms
+// Nothing outside the pair loop runs in FP64 (76 cycles an instruction, 95 a
+// conversion): positions and loads become integers, and sums FP64 numbers, by
+// integer instructions.  With FP64 there, 642 segments took 28.6 us (now 20.5),
+// 962 41.0 (34.8), 1669 blobs 55.3 (45.1), a solve of 962 particles 4.25 ms (3.80).
 // Error against extended precision (2-norm, mean of four draws), FP64 kernel ->
-// this: 60 to 700 segments 0.86 to 1.02 of it, 1500 segments 2.9e-16 -> 1.9e-16;
-// 50 to 1200 blobs 0.7 to 0.96; 100 segments on 60 blobs 2.1e-16 -> 2.1e-16.
+// this: 60 to 700 segments 0.81 to 0.96 of it, 1500 segments 2.9e-16 -> 1.9e-16;
+// 50 to 1200 blobs 0.65 to 0.95; segments on blobs and back 0.82 to 1.05.
 #include <algorithm>
 
 #include "gmi_fx_kernels.hpp"
@@ -71,8 +75,8 @@ struct FxLaunch {
     UnequalK<double> uq;
 };
 
-// One source on its way into a record: its position, its loads (torques over
-// U) and their exponent.
+// One source on its way into a record: its position, its loads and their
+// exponent (torques over U).
 template <int KIND> struct FxPacking {
     long long X[3];
     double F[FxTraits<KIND>::nf];
@@ -86,19 +90,16 @@ __device__ __forceinline__ FxPacking<KIND> fx_read_source(const double *__restri
 {
     using Tr = FxTraits<KIND>;
     FxPacking<KIND> p;
-    double mx = 0.0;
     bool ok = true;
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-        ok = fx_position(x[3 * (size_t)i + c], K.pos_scale, fx_origin(x[c], K.pos_scale), &p.X[c]) && ok;
+    for (int c = 0; c < 3; ++c) ok = fx_position(x[3 * (size_t)i + c], K, fx_origin(x[c], K), &p.X[c]) && ok;
+    p.e = kFxNoLoad;
 #pragma unroll
     for (int c = 0; c < Tr::nf; ++c) {
-        p.F[c] = f[Tr::nf * (size_t)i + c] * (c < 3 ? 1.0 : K.inv_unit);
-        // the larger magnitude by its bits: a NaN or infinity stays the largest
-        mx = __longlong_as_double(max(__double_as_longlong(mx), __double_as_longlong(fabs(p.F[c]))));
+        p.F[c] = f[Tr::nf * (size_t)i + c];
+        p.e = max(p.e, fx_exponent(p.F[c], c < 3 ? 0 : K.unit_exp));
     }
-    ok = fx_load_exponent(mx, &p.e) && ok;
-    if (!ok) p.e = kFxMark;
+    if (!ok || !fx_exponent_held(p.e)) p.e = kFxMark;
     return p;
 }
 
@@ -117,7 +118,7 @@ template <int NW> __device__ __forceinline__ int fx_block_max(int e, int *wmax)
 
 // The record of a source in a block whose largest exponent is E.
 template <int KIND>
-__device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E, int4 *r)
+__device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E, const FxConsts &K, int4 *r)
 {
     using Tr = FxTraits<KIND>;
     const bool bad = E == kFxMark;
@@ -126,13 +127,16 @@ __device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E,
         gap = min(E - p.e, kFxMaxGap);
         used = E - gap;
     }
-    const double scale = bad ? 0.0 : fx_exp2(-used);
     const int tile = bad ? kFxBadTile : E == kFxNoLoad ? 0 : E;
     const auto lo = [](long long v) { return (int)(unsigned)v; };
     const auto hi = [](long long v) { return (int)(v >> 32); };
     fxop F[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) F[c] = bad ? fxop{0, 0.0f, 0.0f} : fx_from_double(p.F[c] * scale);
+    for (int c = 0; c < 3; ++c) {
+        long long v;
+        fx_fixed(p.F[c], 62 - used, &v);
+        F[c] = bad ? fxop{0, 0.0f, 0.0f} : fx_split(v);
+    }
     r[0] = make_int4(lo(p.X[0]), hi(p.X[0]), lo(p.X[1]), hi(p.X[1]));
     r[1] = make_int4(lo(p.X[2]), hi(p.X[2]), F[0].h, __float_as_int(F[0].hf));
     r[2] = make_int4(__float_as_int(F[0].lf), F[1].h, __float_as_int(F[1].hf), __float_as_int(F[1].lf));
@@ -140,7 +144,10 @@ __device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E,
     if constexpr (Tr::torque) {
         long long T[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) T[c] = bad ? 0 : fx_rint(p.F[3 + c] * scale * 4611686018427387904.0);
+        for (int c = 0; c < 3; ++c) {
+            fx_fixed(p.F[3 + c], 62 - used - K.unit_exp, &T[c]);
+            if (bad) T[c] = 0;
+        }
         r[4] = make_int4(lo(T[0]), hi(T[0]), lo(T[1]), hi(T[1]));
         r[5] = make_int4(lo(T[2]), hi(T[2]), 0, 0);
     }
@@ -158,7 +165,7 @@ __global__ void __launch_bounds__(kFxBlock) fx_pack_kernel(const double *__restr
     p.e = kFxNoLoad;
     if (i < n) p = fx_read_source<KIND>(x, f, i, K);
     const int E = fx_block_max<kFxBlock / 32>(p.e, wmax);
-    if (i < n) fx_write_record<KIND>(p, E, rec + (size_t)i * FxTraits<KIND>::quads);
+    if (i < n) fx_write_record<KIND>(p, E, K, rec + (size_t)i * FxTraits<KIND>::quads);
 }
 
 struct FxSum {
@@ -232,7 +239,7 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
     using Tr = FxTraits<KIND>;
     constexpr int NOUT = Tr::nout;
     __shared__ __align__(128) int4 ring[kFxStages][kFxTile * Tr::quads];
-    __shared__ double red[kFxWarps][NOUT][33];
+    __shared__ long long red[2][kFxWarps][NOUT][33];
     __shared__ uint64_t bars[kFxStages];
     __shared__ int wmax[kFxWarps];
 
@@ -264,7 +271,7 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
         const int i = j_begin + tid;
         if (i < j_end) p = fx_read_source<KIND>(a.xs, a.fs, i, a.K);
         const int E = fx_block_max<kFxWarps>(p.e, wmax);
-        if (i < j_end) fx_write_record<KIND>(p, E, ring[0] + tid * Tr::quads);
+        if (i < j_end) fx_write_record<KIND>(p, E, a.K, ring[0] + tid * Tr::quads);
         __syncthreads();
     }
 
@@ -274,7 +281,7 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
     bool ok = true;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
-        ok = fx_position(a.xt[3 * (size_t)ti + c], a.K.pos_scale, fx_origin(a.xs[c], a.K.pos_scale), &X[c]) && ok;
+        ok = fx_position(a.xt[3 * (size_t)ti + c], a.K, fx_origin(a.xs[c], a.K), &X[c]) && ok;
     const bool warp_ok = __all_sync(0xffffffffu, ok);
     double tot[NOUT];
 #pragma unroll
@@ -283,6 +290,8 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
     bool timed_out = false;
     FxAcc<NOUT> acc;
     fx_clear(acc);
+    int E = 0;             // of the block in acc
+    bool earlier = false;  // tot holds something (the same in every thread)
     int t = 0;
     for (; t < ntiles; ++t) {
         const int s = t % kFxStages;
@@ -298,24 +307,27 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
         const int j0 = j_begin + t * kFxTile, jn = min(kFxTile, j_end - j0);
         const int per = (jn + kFxWarps - 1) / kFxWarps, b = min(warp * per, jn), e = min(b + per, jn);
         const int4 *tile = ring[s];
-        const int E = tile[3].w >> 8;
-        if (E == kFxBadTile || !warp_ok) {  // the whole block
+        const int Et = tile[3].w >> 8;
+        if (Et == kFxBadTile || !warp_ok) {  // the whole block
             const FxSum r = fx_sum_fp64<KIND>(a, ti, j0 + b, j0 + e);
 #pragma unroll
             for (int c = 0; c < NOUT; ++c) tot[c] += r.v[c];
+            earlier = true;
             continue;
         }
+        E = Et;
         for (int j = b; j < e;) {
             const int stop = min(j + kFxSettle[KIND], e);
 #pragma unroll 1
             for (; j < stop; ++j) fx_pair<KIND>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc);
             fx_settle(acc);
         }
-        if (t + 1 == ntiles || (j0 + kFxTile) % kFxBlock == 0) {  // the block's last tile here
-            const double scale = fx_exp2(E);
+        if (t + 1 < ntiles && (j0 + kFxTile) % kFxBlock == 0) {  // the block's last tile
 #pragma unroll
-            for (int c = 0; c < NOUT; ++c) tot[c] += fx_fold(acc, c, (c < 3 ? a.K.vscale : a.K.wscale) * scale, a.K.vscale_fix);
+            for (int c = 0; c < NOUT; ++c)
+                tot[c] += fx_value(fx_total(acc, c), E, c < 3 ? a.K.vscale : a.K.wscale, c < 3 ? a.K.vfix : a.K.wfix);
             fx_clear(acc);
+            earlier = true;
         }
     }
 
@@ -328,14 +340,46 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
         return;
     }
 
+    // the warps' sums of the last block meet as integers, so they are rounded
+    // once; earlier blocks' (of splits beyond one block) in FP64
 #pragma unroll
-    for (int c = 0; c < NOUT; ++c) red[warp][c][lane] = tot[c];
+    for (int c = 0; c < NOUT; ++c) {
+        const FxTotal v = fx_total(acc, c);
+        red[0][warp][c][lane] = v.a;
+        red[1][warp][c][lane] = v.b;
+    }
     __syncthreads();
     const int nt = min(32, a.n_tgt - group0);
     const size_t base = (size_t)group0 * NOUT, count = (size_t)a.n_tgt * NOUT;
-    for (int o = tid; o < nt * NOUT; o += kFxTpb) {
-        const int i = o / NOUT, c = o - i * NOUT;
-        const double v = (red[0][c][i] + red[1][c][i]) + (red[2][c][i] + red[3][c][i]);
+    constexpr int kPer = (32 * NOUT + kFxTpb - 1) / kFxTpb;
+    double sum[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int o = tid + k * kFxTpb, i = o / NOUT, c = o - i * NOUT;
+        if (o >= nt * NOUT) continue;
+        FxTotal v{0, 0};
+#pragma unroll
+        for (int w = 0; w < kFxWarps; ++w) {
+            v.a += red[0][w][c][i];
+            v.b += red[1][w][c][i];
+        }
+        sum[k] = fx_value(v, E, c < 3 ? a.K.vscale : a.K.wscale, c < 3 ? a.K.vfix : a.K.wfix);
+    }
+    if (earlier) {
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < NOUT; ++c) red[0][warp][c][lane] = __double_as_longlong(tot[c]);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int o = tid + k * kFxTpb, i = o / NOUT, c = o - i * NOUT;
+        if (o >= nt * NOUT) continue;
+        double v = sum[k];
+        if (earlier) {
+            const auto r = [&](int w) { return __longlong_as_double(red[0][w][c][i]); };
+            v += (r(0) + r(1)) + (r(2) + r(3));
+        }
         if (a.partial != nullptr)
             a.partial[blockIdx.y * count + base + o] = v;
         else
@@ -374,12 +418,12 @@ static FxPackFn pack_fn(int kind)
 // Sources per split, a power of two.  Measured on M_ss and M_bb of 200 to
 // 12,800 particles (152 SMs): with work enough, the largest split that still
 // gives 24 CTAs per SM, so that the last CTAs to finish idle the chip for
-// little of the launch (4096 segments: 128 sources 339 us, 1024 407; 12,800:
-// 1024 sources 2.79 ms, 128 2.86, 2048 2.82); below that a tile, down to 1.5
-// CTAs per SM (2000 segments: 128 111 us, 64 117; 962: 41 against 49); then
-// parts of a tile, whose CTAs have less to do than to set up (642: 32 28 us,
-// 64 29, 128 33), and 16 or 8 while the CTAs still find an SM each (200: 16
-// 16.5 us, 8 and 32 18.5; 320: 32 18.5 us, 16 20.5, 8 24.6).
+// little of the launch (4096 segments: 128 sources 325 us, 1024 403; 12,800:
+// 1024 sources 2.82 ms, 128 2.87, 2048 2.84); below that a tile, down to 1.5
+// CTAs per SM (1669 segments: 128 72 us, 64 78, 32 82); then parts of a tile,
+// whose CTAs have less to do than to set up (642: 32 20.6 us, 64 24.7, 128
+// 30.8), and 16 or 8 while the CTAs still find an SM each (60: 8 12.4 us, 16
+// 14.4, 32 16.5; 320: 32 17.7 us, 16 and 8 16.5).
 static int fx_chunk(int groups, int n_src, int sm_count, int most_splits)
 {
     const auto splits = [&](long long chunk) { return ((long long)n_src + chunk - 1) / chunk; };

@@ -1817,7 +1817,7 @@ gmi_status launch_pair(gmi_context *ctx, int kind, const void *tgt_rec, int tgt_
 // kernel of the context's precision.  FP64 takes the wall kernel or, without a
 // wall, the fixed-point kernel, at every size: against the FP64 kernels M_ss of 320
 // segments went from 61 to 16.4 us, of 12,800 from 20.4 to 2.81 ms, M_bb of
-// 4096 blobs from 1223 to 188 us.  The FP64 kernels keep radii that the
+// 4096 blobs from 1223 to 178 us.  The FP64 kernels keep radii that the
 // fixed-point formats do not hold, and shapes pinned by gmi_set_shape.
 gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt, int tgt_start, int n_tgt,
                     const double *xs, const double *fs, int n_src, double as, double ab, double mu, double *out,

@@ -45,10 +45,10 @@ constexpr double kFxPosLimit = 1152921504606845952.0;  // 2^60 - 2^10: |position
 enum FxKind : int { kFxSS = 0, kFxBB = 2, kFxSB = 3, kFxBS = 4 };  // as PairKind
 
 struct FxConsts {
-    double pos_scale;          // 2^51 / U
-    double unit, inv_unit;     // U, 1/U
-    double vscale, wscale;     // 1/(8 pi mu U), 1/(8 pi mu U^2)
-    double vscale_fix;         // their common relative error: exact = rounded * (1 + fix)
+    int pos_shift, unit_exp;   // 2^pos_shift = 2^51 / U, 2^unit_exp = U
+    double pos_scale, unit;    // 2^51 / U, U
+    double vscale, vfix;       // 1/(8 pi mu U), and what its rounding leaves out
+    double wscale, wfix;       // 1/(8 pi mu U^2)
     double as, ab, inv_as;     // radii (equal kinds: both the one radius)
     double a0, ar0;            // near field: 4U/(3a) (unequal: 4U/(3 as ab)), (U/a)^3
     fxop k3;                   // far field: (as^2 + ab^2) / (3 U^2)
@@ -294,13 +294,64 @@ template <int N> GMI_FX_HD void fx_settle(FxAcc<N> &a)
     }
 }
 
-// One settled accumulator to FP64 in final units: scale = vscale or wscale
-// times the block's 2^E.
-template <int N> GMI_FX_HD double fx_fold(const FxAcc<N> &a, int c, double scale, double fix)
+GMI_FX_HD long long fx_rintf(float v)
 {
-    const double s = scale * (1.0 / 1152921504606846976.0) * (1.0 / (double)(1 << kFxAccBits));
-    const double high = (double)a.H[c], low = (double)a.L[c] + ((double)a.xh[c] + (double)a.xl[c]);
-    return fma(high, s * 4294967296.0, fma(low, s, high * (s * 4294967296.0 * fix)));
+#ifdef __CUDA_ARCH__
+    return __float2ll_rn(v);
+#else
+    return (long long)llrintf(v);
+#endif
+}
+
+// A sum as an integer a 2^32 + b in 2^-84 of the block's unit; sums add part
+// by part.
+struct FxTotal {
+    long long a, b;
+};
+
+// One settled accumulator.  Its FP32 parts lie below 2^65.
+template <int N> GMI_FX_HD FxTotal fx_total(const FxAcc<N> &acc, int c)
+{
+    const float top = rintf(acc.xh[c] * (1.0f / 4294967296.0f));
+    const long long low = (long long)(acc.L[c] & 0xffffffffull) + fx_rintf(acc.xh[c] - top * 4294967296.0f) +
+                          fx_rintf(acc.xl[c]);
+    return FxTotal{acc.H[c] + (long long)(acc.L[c] >> 32) + fx_rintf(top) + (low >> 32), low & 0xffffffffll};
+}
+
+// A sum in FP64, times 2^E (scale + fix): the integer is rounded once, to 53
+// bits, by integer instructions (a conversion holds the FP64 unit longer than
+// an addition does).
+GMI_FX_HD double fx_value(const FxTotal &t, int E, double scale, double fix)
+{
+    const long long a = t.a + (t.b >> 32);
+    const unsigned b = (unsigned)t.b;
+    const bool neg = a < 0;
+    // |a 2^32 + b| as the 128-bit number (hi, lo) 2^-32
+    unsigned long long hi = neg ? ~(unsigned long long)a + (b == 0) : (unsigned long long)a;
+    unsigned long long lo = (unsigned long long)(neg ? 0u - b : b) << 32;
+    int e = 32 + 11;  // of the 53-bit significand's last place, before the shift
+    if (hi == 0) {
+        hi = lo;
+        lo = 0;
+        e -= 64;
+    }
+    if (hi == 0) return 0.0;
+    const int z = fx_clzll(hi);
+    if (z > 0) {
+        hi = (hi << z) | (lo >> (64 - z));
+        lo <<= z;
+    }
+    e -= z;
+    const unsigned rest = ((unsigned)hi & 2047u) * 2u + (lo != 0);
+    const unsigned long long m = hi >> 11;  // 2^52 <= m < 2^53
+    union {
+        unsigned long long u;
+        double d;
+    } c;
+    c.u = ((unsigned long long)(unsigned)(1023 + 52 - 60 - kFxAccBits + e + E - 1) << 52) + m +
+          (rest > 2048u || (rest == 2048u && (m & 1)));
+    const double v = neg ? -c.d : c.d;
+    return fma(v, scale, v * fix);
 }
 
 // The constants of one kind; false where the formats do not hold them: the
@@ -316,12 +367,15 @@ inline bool fx_consts(int kind, double as, double ab, double mu, FxConsts *K)
     // 8 pi mu in two parts: the one rounding that every velocity shares
     const double pi = 3.14159265358979323846264338327950288, pi_low = 1.2246467991473532e-16;
     const double d8 = 8.0 * pi * mu, d8_low = fma(8.0 * pi, mu, -d8) + 8.0 * pi_low * mu, f8 = 1.0 / d8;
+    const double fix = fma(-f8, d8, 1.0) - f8 * d8_low;
     K->unit = U;
-    K->inv_unit = 1.0 / U;
+    K->unit_exp = e - 1;
+    K->pos_shift = kFxPosBits - (e - 1);
     K->pos_scale = ldexp(1.0, kFxPosBits) / U;
     K->vscale = f8 / U;
+    K->vfix = K->vscale * fix;
     K->wscale = f8 / (U * U);
-    K->vscale_fix = fma(-f8, d8, 1.0) - f8 * d8_low;
+    K->wfix = K->wscale * fix;
     K->as = as;
     K->ab = ab;
     K->inv_as = 1.0 / as;
@@ -338,43 +392,78 @@ inline bool fx_consts(int kind, double as, double ab, double mu, FxConsts *K)
     return true;
 }
 
-// A position in quanta relative to `origin` (a multiple of 2^59 quanta, in
-// quanta).  False when it is out of range or not finite.  Below 2^62 quanta
-// the subtraction is done in integers; above, the FP64 difference is exact.
-GMI_FX_HD bool fx_position(double x, double pos_scale, double origin, long long *X)
-{
-    const double t = x * pos_scale, rel = t - origin;
-    if (!(fabs(rel) < kFxPosLimit)) {
-        *X = 0;
-        return false;
-    }
-    *X = fabs(t) < 4611686018427387904.0 ? fx_rint(t) - (long long)origin : fx_rint(rel);
-    return true;
-}
-
-GMI_FX_HD double fx_origin(double x0, double pos_scale)
-{
-    return rint(x0 * pos_scale * (1.0 / 576460752303423488.0)) * 576460752303423488.0;
-}
-
-// The exponent that makes the loads fractions (every |load| < 2^e), or
-// kFxNoLoad when all are zero; false when not finite or out of range.
-constexpr int kFxNoLoad = -100000;
-constexpr int kFxMaxExp = 900;
-GMI_FX_HD bool fx_load_exponent(double largest, int *e)
+// v 2^s to the nearest integer, ties to even, by integer instructions; false
+// (and 0) when that reaches 2^62 or v is not finite.  Denormals are zeros.
+GMI_FX_HD bool fx_fixed(double v, int s, long long *r)
 {
     union {
         double d;
         unsigned long long u;
     } c;
-    c.d = largest;
-    const int be = (int)(c.u >> 52);  // largest >= 0
-    if (largest == 0.0) {
-        *e = kFxNoLoad;
-        return true;
-    }
-    *e = be - 1022;
-    return be != 2047 && *e <= kFxMaxExp && *e >= -kFxMaxExp;
+    c.d = v;
+    const int be = (int)(c.u >> 52) & 2047, sh = be - 1075 + s;
+    *r = 0;
+    if (be == 2047) return false;
+    if (be == 0 || sh < -54) return true;
+    if (sh > 9) return false;
+    long long m = (long long)((c.u & 0xfffffffffffffull) | 0x10000000000000ull);
+    if (sh >= 0)
+        m <<= sh;
+    else
+        m = (m + ((1ll << (-sh - 1)) - 1) + ((m >> -sh) & 1)) >> -sh;
+    *r = (long long)c.u < 0 ? -m : m;
+    return true;
 }
+
+// Where positions are counted from, in quanta: a multiple of 2^59 next to the
+// first source; in FP64 (d) when that is 2^62 quanta from zero or further.
+struct FxOrigin {
+    long long i;
+    double d;
+    bool far;
+};
+GMI_FX_HD FxOrigin fx_origin(double x0, const FxConsts &K)
+{
+    FxOrigin o;
+    long long t;
+    o.far = !fx_fixed(x0, K.pos_shift, &t);
+    o.i = ((t + (1ll << 58)) >> 59) << 59;
+    o.d = o.far ? rint(x0 * K.pos_scale * (1.0 / 576460752303423488.0)) * 576460752303423488.0 : 0.0;
+    return o;
+}
+
+// A position in quanta relative to the origin; false when it is out of range
+// or not finite.  Past 2^62 quanta the FP64 difference is exact.
+GMI_FX_HD bool fx_position(double x, const FxConsts &K, const FxOrigin &o, long long *X)
+{
+    long long t;
+    if (!o.far && fx_fixed(x, K.pos_shift, &t)) {
+        t -= o.i;
+    } else {
+        const double rel = x * K.pos_scale - (o.far ? o.d : (double)o.i);
+        t = fabs(rel) < kFxPosLimit ? fx_rint(rel) : (long long)kFxPosLimit;
+    }
+    const bool ok = t < (long long)kFxPosLimit && t > -(long long)kFxPosLimit;
+    *X = ok ? t : 0;
+    return ok;
+}
+
+// The exponent e that makes v 2^-unit_exp a fraction (below 2^e): kFxNoLoad for
+// a zero, out of the range +-kFxMaxExp for what the formats do not hold.
+constexpr int kFxNoLoad = -100000;
+constexpr int kFxMaxExp = 900;
+GMI_FX_HD int fx_exponent(double v, int unit_exp)
+{
+    union {
+        double d;
+        unsigned long long u;
+    } c;
+    c.d = v;
+    const int be = (int)(c.u >> 52) & 2047;
+    if (be == 0) return (c.u << 1) == 0 ? kFxNoLoad : -5000;
+    return be == 2047 ? 5000 : be - 1022 - unit_exp;
+}
+// The exponent of a source is its components' largest.
+GMI_FX_HD bool fx_exponent_held(int e) { return e == kFxNoLoad || (e <= kFxMaxExp && e >= -kFxMaxExp); }
 
 }  // namespace gmi

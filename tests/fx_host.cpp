@@ -18,32 +18,32 @@ static int sum(int nt, const double *xt, int ns, const double *xs, const double 
     if (!fx_consts(KIND, as, ab, mu, &K)) return 1;
     std::vector<FxSource> src(ns);
     std::vector<int> e(ns), E((ns + tile - 1) / tile, kFxNoLoad);
-    double origin[3];
-    for (int c = 0; c < 3; ++c) origin[c] = fx_origin(xs[c], K.pos_scale);
+    FxOrigin origin[3];
+    for (int c = 0; c < 3; ++c) origin[c] = fx_origin(xs[c], K);
     for (int j = 0; j < ns; ++j) {
-        double mx = 0;
         for (int c = 0; c < 3; ++c)
-            if (!fx_position(xs[3 * j + c], K.pos_scale, origin[c], &src[j].X[c])) return 2;
-        for (int c = 0; c < nf; ++c) {
-            const double v = fabs(f[nf * j + c]) * (c < 3 ? 1.0 : K.inv_unit);
-            mx = v > mx || v != v ? v : mx;  // a NaN stays
-        }
-        if (!fx_load_exponent(mx, &e[j])) return 2;
+            if (!fx_position(xs[3 * j + c], K, origin[c], &src[j].X[c])) return 2;
+        e[j] = kFxNoLoad;
+        for (int c = 0; c < nf; ++c) e[j] = std::max(e[j], fx_exponent(f[nf * j + c], c < 3 ? 0 : K.unit_exp));
+        if (!fx_exponent_held(e[j])) return 2;
         E[j / tile] = std::max(E[j / tile], e[j]);
     }
     for (int j = 0; j < ns; ++j) {
         src[j].gap = e[j] == kFxNoLoad ? 0 : std::min(E[j / tile] - e[j], kFxMaxGap);
-        const double s = fx_exp2(e[j] == kFxNoLoad ? 0 : -(E[j / tile] - src[j].gap));
+        const int used = e[j] == kFxNoLoad ? 0 : E[j / tile] - src[j].gap;
         for (int c = 0; c < 3; ++c) {
-            src[j].F[c] = fx_from_double(f[nf * j + c] * s);
-            src[j].T[c] = torque ? fx_rint(f[nf * j + nf - 3 + c] * K.inv_unit * s * 4611686018427387904.0) : 0;
+            long long v;
+            fx_fixed(f[nf * j + c], 62 - used, &v);
+            src[j].F[c] = fx_split(v);
+            src[j].T[c] = 0;
+            if (torque) fx_fixed(f[nf * j + nf - 3 + c], 62 - used - K.unit_exp, &src[j].T[c]);
         }
     }
     for (int i = 0; i < nt; ++i) {
         long long X[3];
         double tot[6] = {0, 0, 0, 0, 0, 0};
         for (int c = 0; c < 3; ++c)
-            if (!fx_position(xt[3 * i + c], K.pos_scale, origin[c], &X[c])) return 2;
+            if (!fx_position(xt[3 * i + c], K, origin[c], &X[c])) return 2;
         for (int j0 = 0; j0 < ns; j0 += kFxFold) {
             FxAcc<nout> acc;
             fx_clear(acc);
@@ -52,8 +52,9 @@ static int sum(int nt, const double *xt, int ns, const double *xs, const double 
                 if ((j - j0) % kFxSettle[KIND] == kFxSettle[KIND] - 1) fx_settle(acc);
             }
             fx_settle(acc);
-            const double s = fx_exp2(E[j0 / tile] == kFxNoLoad ? 0 : E[j0 / tile]);
-            for (int c = 0; c < nout; ++c) tot[c] += fx_fold(acc, c, (c < 3 ? K.vscale : K.wscale) * s, K.vscale_fix);
+            const int Ej = E[j0 / tile] == kFxNoLoad ? 0 : E[j0 / tile];
+            for (int c = 0; c < nout; ++c)
+                tot[c] += fx_value(fx_total(acc, c), Ej, c < 3 ? K.vscale : K.wscale, c < 3 ? K.vfix : K.wfix);
         }
         for (int c = 0; c < nout; ++c) out[nout * i + c] = tot[c];
     }
@@ -68,3 +69,6 @@ extern "C" int fx_host_sum(int kind, int nt, const double *xt, int ns, const dou
          : kind == 3 ? sum<kFxSB>(nt, xt, ns, xs, f, as, ab, mu, out)
                      : sum<kFxBS>(nt, xt, ns, xs, f, as, ab, mu, out);
 }
+
+extern "C" int fx_host_fixed(double v, int s, long long *r) { return fx_fixed(v, s, r) ? 1 : 0; }
+extern "C" double fx_host_value(long long a, long long b, int E) { return fx_value(FxTotal{a, b}, E, 1.0, 0.0); }

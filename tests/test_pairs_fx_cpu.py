@@ -9,6 +9,7 @@ within n 2^-53 of the terms' size; n 2^-52 of the largest velocity is allowed.
 import ctypes
 import os
 import subprocess
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -113,3 +114,28 @@ def test_translation_and_range(host, oracle_built):
         g[17, 4] = bad
         assert fx_sum(host, "ss", xs, xs, g, 1.0, 1.0)[0] == 2
     assert fx_sum(host, "sb", xs, xs, f[:, :3], 1.0, 2.1)[0] == 1
+
+
+def test_conversions_round_once(host):
+    """FP64 to fixed point and back by integer instructions: the nearest, ties
+    to even, as exact arithmetic rounds (no tolerance)."""
+    host.fx_host_fixed.argtypes = [ctypes.c_double, ctypes.c_int, ctypes.c_void_p]
+    host.fx_host_value.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
+    host.fx_host_value.restype = ctypes.c_double
+    rng = np.random.default_rng(11)
+    values = [0.0, -0.0, 0.5, 1.5, -2.5, 2.0 ** 52 + 0.5, 2.0 ** 61, -(2.0 ** 62 - 512), 2.0 ** 62, 5e-324, np.inf, np.nan]
+    values += list(rng.normal(size=200) * 2.0 ** rng.integers(-70, 64, 200))
+    for v in values:
+        for s in (-3, 0, 1, 11):
+            r = ctypes.c_longlong(7)
+            held = host.fx_host_fixed(v, s, ctypes.byref(r))
+            exact = round(Fraction(v) * Fraction(2) ** s) if np.isfinite(v) else None
+            fits = exact is not None and abs(Fraction(v)) * Fraction(2) ** s < 2 ** 62
+            assert held == fits and r.value == (exact if fits else 0)
+    sums = [(0, 0), (0, 1), (0, 2 ** 34), (-1, 0), (-1, 2 ** 32 - 1), (-1, 2 ** 32), (2 ** 20, 1), (2 ** 21 - 1, 2 ** 32 - 1),
+            (2 ** 53 + 1, 0), (2 ** 53 + 1, 1), (2 ** 21 + 2 ** 10, 2 ** 31), (-2 ** 62, 0), (2 ** 62, 2 ** 34)]
+    sums += [(int(a) >> int(k), int(b)) for a, k, b in zip(rng.integers(-2 ** 62, 2 ** 62, 300), rng.integers(0, 63, 300),
+                                                           rng.integers(0, 2 ** 34, 300))]
+    for a, b in sums:
+        for e in (0, 84, -37):
+            assert host.fx_host_value(a, b, e) == float(Fraction(a * 2 ** 32 + b) * Fraction(2) ** (e - 84))
