@@ -15,10 +15,38 @@ from . import _lib
 from ._lib import GMI_FP64, HostArrays, SolverConfig, check
 
 
-def _view(ptr, count, cols):
+class _Owner:
+    """The library's solver; destroyed by close() or with the last reference."""
+
+    def __init__(self, lib, handle):
+        self.lib, self.handle = lib, handle
+
+    def close(self):
+        if self.handle:
+            self.lib.gmi_solver_destroy(self.handle)
+            self.handle = None
+
+    def __del__(self):
+        try:
+            self.close()
+        except Exception:
+            pass
+
+
+class _HostMemory:
+    """Part of a solver's pinned memory as an array's base: an array that
+    outlives the MobilitySolver keeps the memory it shows."""
+
+    def __init__(self, owner, ptr, shape):
+        self.owner = owner
+        address = ctypes.cast(ptr, ctypes.c_void_p).value
+        self.__array_interface__ = dict(shape=shape, typestr="<f8", data=(address, False), version=3)
+
+
+def _view(owner, ptr, count, cols):
     if count == 0:
         return np.zeros((0, cols))
-    return np.ctypeslib.as_array(ptr, shape=(count * cols,)).reshape(count, cols)
+    return np.asarray(_HostMemory(owner, ptr, (count, cols)))
 
 
 def _cptr(a: np.ndarray):
@@ -38,29 +66,24 @@ class MobilitySolver:
         h = ctypes.c_void_p()
         check(self.lib.gmi_solver_create(ctypes.byref(cfg), ctypes.byref(h)))
         self.handle = h
+        self._owner = _Owner(self.lib, h)
         arrays = HostArrays()
         check(self.lib.gmi_solver_host_arrays(self.handle, ctypes.byref(arrays)))
         S, B = nswim * nfil * nseg, nswim * nblob
         self.S, self.B, self.W = S, B, nswim
-        self.v_segs_host = _view(arrays.v_segs_host, S, 6)
-        self.v_blobs_host = _view(arrays.v_blobs_host, B, 3)
-        self.x_segs_host = _view(arrays.x_segs_host, S, 3)
-        self.x_blobs_host = _view(arrays.x_blobs_host, B, 3)
-        self.f_segs_host = _view(arrays.f_segs_host, S, 6)
-        self.f_blobs_host = _view(arrays.f_blobs_host, B, 3)
-        self.f_blobs_repulsion_host = _view(arrays.f_blobs_repulsion_host, B, 3)
+        self.v_segs_host = _view(self._owner, arrays.v_segs_host, S, 6)
+        self.v_blobs_host = _view(self._owner, arrays.v_blobs_host, B, 3)
+        self.x_segs_host = _view(self._owner, arrays.x_segs_host, S, 3)
+        self.x_blobs_host = _view(self._owner, arrays.x_blobs_host, B, 3)
+        self.f_segs_host = _view(self._owner, arrays.f_segs_host, S, 6)
+        self.f_blobs_host = _view(self._owner, arrays.f_blobs_host, B, 3)
+        self.f_blobs_repulsion_host = _view(self._owner, arrays.f_blobs_repulsion_host, B, 3)
 
     # ---- lifetime ----------------------------------------------------------
     def close(self):
         if getattr(self, "handle", None):
-            self.lib.gmi_solver_destroy(self.handle)
+            self._owner.close()
             self.handle = None
-
-    def __del__(self):
-        try:
-            self.close()
-        except Exception:
-            pass
 
     def __enter__(self):
         return self
