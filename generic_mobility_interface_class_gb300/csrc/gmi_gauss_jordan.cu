@@ -32,8 +32,8 @@
 // filaments, where one CTA per matrix would leave most SMs idle).  Both are
 // templates on the element type: FP64 for the reference's arithmetic, FP32
 // for the mixed-precision time step, whose approximate inverse only starts
-// the Broyden iteration (on the FMA pipe a step is latency-bound, not
-// FP64-bound).
+// the Broyden iteration.  Up to 128 x 128 a third kernel takes the FP32
+// matrices, one CTA each whatever their number, and keeps them in registers.
 #include <cooperative_groups.h>
 
 #include "gmi_context.hpp"
@@ -151,7 +151,7 @@ static __device__ __forceinline__ void gj_cols(T *A, int n, int j0, const int (&
             // it were neither k nor p, and the lanes that hold rows p and k
             // redo theirs: row p from the old row k, row k as akj / pivot (a
             // zero addend; when p == k the second fix wins, as in the
-            // swap-free case).  1.77 -> 1.57 ms for 640 matrices of 120 x 120.
+            // swap-free case).  12 % less time.
 #pragma unroll
             for (int t = 0; t < RPL; ++t) v[c][t] = gj_fma(akj, ncr[t], v[c][t]);
             if (lane == pl) {
@@ -306,6 +306,149 @@ __global__ void __launch_bounds__(kGjTpb) gj_invert_kernel(T *mats, int n, int u
     }
 }
 
+template <int T> struct GjRow {
+    static constexpr int value = T;
+};
+
+// FP32, n <= 32 RPL: the matrix stays in the CTA's registers, row lane + 32 t
+// of column wid + NW c in v[c][t], and only the published pivot column goes
+// through shared memory.  The rows are not swapped: a row keeps its lane, and
+// pos holds the place that the swaps would have brought it to, so the pivot
+// row's factor comes from one lane by shuffle, the same for every column, and
+// an element costs its FMA and a fifth of a shuffle and a select.  The arithmetic
+// per element, the pivots and their ties (the lowest place) are those of
+// gj_invert_kernel, so the results have the same bits.  A step is then bound
+// by its chain: barrier, one column's elimination, pivot search, division.
+// 640 matrices of 120 x 120: 1558 -> 345 us (the matrix in shared memory spent
+// three instructions in moving an element for each FMA), 160: 651 -> 128, 40:
+// 386 (clusters of two CTAs) -> 109, 8: 240 (clusters of eight) -> 107; 640 of
+// 60 x 60: 320 -> 66.  Eight warps with twice the columns: 899 us for 640; one
+// CTA per SM's registers 448, three 610.
+template <int RPL, int NW>
+__global__ void __launch_bounds__(32 * NW, 2) gj_register_kernel(float *mats, int n, int *flags)
+{
+    constexpr int R = 32 * RPL, C = R / NW;
+    __shared__ float mult[2][R];      // by step parity: -A(i, k) / pivot, and 1 / pivot in the pivot's row
+    __shared__ int prow[2];           // the pivot's row, -1: none
+    __shared__ int pos[R], rowat[R];  // place of a row, and back
+    float *Mg = mats + (size_t)blockIdx.x * n * n;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    float v[C][RPL];
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int t = 0; t < RPL; ++t) {
+            const int i = lane + 32 * t, j = wid + NW * c;
+            v[c][t] = i < n && j < n ? Mg[(size_t)n * j + i] : 0.0f;
+        }
+    for (int i = tid; i < R; i += 32 * NW) pos[i] = rowat[i] = i;
+    __syncthreads();
+
+    // the pivot of column k, held in w, among the rows at place k and beyond
+    const auto search = [&](const float (&w)[RPL], int k) {
+        unsigned mag[RPL], place[RPL], most = 0u;
+#pragma unroll
+        for (int t = 0; t < RPL; ++t) {
+            const int i = lane + 32 * t;
+            place[t] = (unsigned)pos[i];
+            mag[t] = i < n && (int)place[t] >= k ? gj_mag(w[t]) : 0u;
+            most = max(most, mag[t]);
+        }
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (most == 0u) {
+            if (lane == 0) prow[k & 1] = -1;
+            return;
+        }
+        unsigned key = 0xffffffffu;
+#pragma unroll
+        for (int t = 0; t < RPL; ++t)
+            if (mag[t] == most) key = min(key, place[t] << 8 | (unsigned)(lane + 32 * t));
+        key = __reduce_min_sync(0xffffffffu, key);
+        const int r = key & 255u, at = key >> 8;
+        float own = w[0];
+#pragma unroll
+        for (int t = 1; t < RPL; ++t)
+            if (r >> 5 == t) own = w[t];
+        const float pivinv = 1.0f / __shfl_sync(0xffffffffu, own, r & 31);
+#pragma unroll
+        for (int t = 0; t < RPL; ++t) {
+            const int i = lane + 32 * t;
+            mult[k & 1][i] = i == r ? pivinv : -(w[t] * pivinv);
+        }
+        if (lane == 0) {
+            const int q = rowat[k];  // at place k so far
+            prow[k & 1] = r;
+            rowat[at] = q;
+            pos[q] = at;
+            rowat[k] = r;
+            pos[r] = k;
+        }
+    };
+    if (wid == 0) search(v[0], 0);
+    __syncthreads();
+
+    for (int k = 0; k < n; ++k) {
+        const int p = prow[k & 1];
+        if (p < 0) {  // the same in every thread
+            if (tid == 0) atomicOr(flags + 2, 1);
+            return;
+        }
+        float m[RPL];
+#pragma unroll
+        for (int t = 0; t < RPL; ++t) m[t] = mult[k & 1][lane + 32 * t];
+        const int pt = p >> 5, pl = p & 31;
+        if (k + 1 < n && (k + 1) % NW == wid) {  // the next pivot's column first
+            float w[RPL];
+            const int cn = (k + 1) / NW;
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+                if (c == cn)
+#pragma unroll
+                    for (int t = 0; t < RPL; ++t) w[t] = v[c][t];
+            float own = w[0];
+#pragma unroll
+            for (int t = 1; t < RPL; ++t)
+                if (pt == t) own = w[t];
+            const float f = __shfl_sync(0xffffffffu, own, pl);
+#pragma unroll
+            for (int t = 0; t < RPL; ++t) w[t] = fmaf(f, m[t], pt == t && lane == pl ? 0.0f : w[t]);
+            search(w, k + 1);
+        }
+        const auto eliminate = [&](auto row) {
+            constexpr int T = decltype(row)::value;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float f = __shfl_sync(0xffffffffu, v[c][T], pl);
+                if (lane == pl) v[c][T] = 0.0f;
+#pragma unroll
+                for (int t = 0; t < RPL; ++t) v[c][t] = fmaf(f, m[t], v[c][t]);
+            }
+        };
+        if (RPL == 1 || pt == 0) eliminate(GjRow<0>{});
+        else if (RPL == 2 || pt == 1) eliminate(GjRow<RPL >= 2 ? 1 : 0>{});
+        else if (pt == 2) eliminate(GjRow<RPL >= 4 ? 2 : 0>{});
+        else eliminate(GjRow<RPL >= 4 ? 3 : 0>{});
+        if (k % NW == wid) {  // column k becomes the inverse's
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+                if (c == k / NW)
+#pragma unroll
+                    for (int t = 0; t < RPL; ++t) v[c][t] = m[t];
+        }
+        __syncthreads();
+    }
+    // the rows to their places, and the column swaps that undo them
+#pragma unroll
+    for (int t = 0; t < RPL; ++t) {
+        const int i = lane + 32 * t;
+        if (i >= n) continue;
+        const int at = pos[i];
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (wid + NW * c < n) Mg[(size_t)n * rowat[wid + NW * c] + at] = v[c][t];
+    }
+}
+
 // One cluster of C CTAs per matrix; CTA r owns columns [r nc, r nc + nc).
 // Per step: one cluster barrier, after which every CTA copies the step's
 // multiplier column, pivot row and 1/pivot from the owner of column k (who
@@ -423,13 +566,24 @@ static gmi_status gj_invert_t(cudaStream_t stream, T *mats, int nmat, int n, int
     if (nmat <= 0) return GMI_OK;
     int dev_max = 0;
     GMI_CUDA_TRY(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    switch (registers ? gj_rows_per_lane(n) : 0) {
-    case 1: return gj_launch<T, 1>(stream, mats, nmat, n, csize, dev_max, flags);
-    case 2: return gj_launch<T, 2>(stream, mats, nmat, n, csize, dev_max, flags);
-    case 4: return gj_launch<T, 4>(stream, mats, nmat, n, csize, dev_max, flags);
-    case 8: return gj_launch<T, 8>(stream, mats, nmat, n, csize, dev_max, flags);
-    default: return gj_launch<T, 0>(stream, mats, nmat, n, csize, dev_max, flags);
+    const int rows = registers ? gj_rows_per_lane(n) : 0;
+    if constexpr (sizeof(T) == 4) {
+        if (rows >= 1 && rows <= 4) {
+            const auto kernel = rows == 1 ? gj_register_kernel<1, kGjWarps>
+                              : rows == 2 ? gj_register_kernel<2, kGjWarps> : gj_register_kernel<4, kGjWarps>;
+            kernel<<<nmat, kGjTpb, 0, stream>>>(mats, n, flags);
+            GMI_CUDA_TRY(cudaGetLastError());
+            return GMI_OK;
+        }
+    } else {
+        switch (rows) {
+        case 1: return gj_launch<T, 1>(stream, mats, nmat, n, csize, dev_max, flags);
+        case 2: return gj_launch<T, 2>(stream, mats, nmat, n, csize, dev_max, flags);
+        case 4: return gj_launch<T, 4>(stream, mats, nmat, n, csize, dev_max, flags);
+        }
     }
+    if (rows == 8) return gj_launch<T, 8>(stream, mats, nmat, n, csize, dev_max, flags);
+    return gj_launch<T, 0>(stream, mats, nmat, n, csize, dev_max, flags);
 }
 
 gmi_status gj_invert(cudaStream_t stream, double *mats, int nmat, int n, int csize, bool registers, int device,

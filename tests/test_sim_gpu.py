@@ -109,6 +109,34 @@ def test_fp32_jacobian_inverse_in_mixed_precision(gmi_lib, monkeypatch):
         assert rel_err(v.ravel(), ref[2].ravel()) < 3e-4, key
 
 
+@pytest.mark.parametrize("nseg,nfil", [(5, 3), (6, 90), (11, 4), (20, 1), (21, 170)])
+def test_fp32_inverse_in_registers_keeps_its_bits(gmi_lib, monkeypatch, nseg, nfil):
+    """The FP32 Jacobian inverse held in registers (6 nseg <= 128) performs the
+    arithmetic of the shared-memory path (GMI_GJ_REGISTERS=0): the same state,
+    bit for bit, around its 32, 64 and 128 rows and for few and many matrices."""
+    from generic_mobility_interface_class_gb300 import seeding, workloads
+    from generic_mobility_interface_class_gb300._lib import GmiError
+    from generic_mobility_interface_class_gb300.sim import Simulation
+    out = {}
+    for registers in ("0", "1"):
+        monkeypatch.setenv("GMI_GJ_REGISTERS", registers)
+        fils = seeding.fibonacci_sphere(nfil)
+        sim = Simulation(**workloads.free_swimmer(seeding.fibonacci_sphere(400), fils, radius=14.0, nseg=nseg, seed=3),
+                         precision=1)
+        sim.prepare()
+        iters = []
+        try:
+            for nt in range(2):
+                iters.append(sim.step(nt)[0])
+        except GmiError as e:  # a step that Broyden's method gives up on does so either way
+            iters.append(str(e))
+        out[registers] = (iters, sim.state("seg_q").copy(), sim.state("seg_v").copy())
+        sim.close()
+    assert out["0"][0] == out["1"][0]
+    np.testing.assert_array_equal(out["0"][1], out["1"][1])
+    np.testing.assert_array_equal(out["0"][2], out["1"][2])
+
+
 def test_trajectory_matches_reference(gmi_lib):
     """12 steps of a 4-filament swimmer, every step compared."""
     run_against_golden("small_swimmer", TRAJ_TOL, VEL_TOL)
