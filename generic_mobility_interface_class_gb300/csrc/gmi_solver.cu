@@ -390,7 +390,7 @@ constexpr int kSGroup = 16;   // CTAs per first-level group of the projection su
 constexpr int kFMaxK = 160;   // >= max_iter + 1
 // layout of the step's scalar workspace (doubles)
 constexpr int kHOff = 0;             // h[kFMaxK]: the last projections
-constexpr int kNormOff = kFMaxK;     // ||w|| of the last step (or beta0 before the first)
+constexpr int kNormOff = kFMaxK;     // ||w|| of the last step (or beta0 before the first), and its reciprocal
 constexpr int kStepScalars = kFMaxK + 8;
 
 // ||x|| into *out in one launch: CTA c sums the squares of rows
@@ -462,6 +462,21 @@ __device__ __forceinline__ void swimmer_sums(const double *part, int W, int gx, 
     const int nw = blockDim.x >> 5, lane = threadIdx.x & 31;
     const int per_warp = (W + nw - 1) / nw * (6 * ((gx + 31) / 32) + 9);
     const int per_thread = (6 * W + blockDim.x - 1) / blockDim.x * gx;
+    if (W == 1 && nw >= 3) {  // two components per warp, each in the order of the general case
+        const int q = threadIdx.x >> 5;
+        if (q < 3) {
+            double a = 0.0, b = 0.0;
+#pragma unroll 4
+            for (int x = lane; x < gx; x += 32) {
+                a += __ldcg(part + (size_t)x * 6 + q);
+                b += __ldcg(part + (size_t)x * 6 + q + 3);
+            }
+            const double t = warp_sum2(a, b);
+            if ((lane & 15) == 0) sh[q + (lane == 16 ? 3 : 0)] = t;
+        }
+        __syncthreads();
+        return;
+    }
     if (per_warp < per_thread) {
         for (int n = threadIdx.x >> 5; n < W; n += nw) {
             double a[6] = {0, 0, 0, 0, 0, 0};
@@ -510,9 +525,15 @@ __device__ __forceinline__ void swimmer_sums(const double *part, int W, int gx, 
 // CGS pass's update that the previous S4 left pending, w -= Q[:, 0..k-1) h2
 // (h2 still in h): lane = blob, warp q takes the columns i = q mod 4, and
 // the CTAs with the lowest linear indices also update the body rows, 32
-// each.  Then q_{k-1} = w / ||w|| into Q and the body moments of q; the
-// last CTA adds the moments per swimmer and forms the body rows of q and
-// z_body.
+// each.  Then q_{k-1} = w / ||w|| into Q and the body moments of q, one
+// component of w and two moments per warp; the last CTA adds the moments per
+// swimmer and forms the body rows of q and z_body.
+//
+// What bounds S1 to S4: chains of FP64 instructions, 76 cycles each on their
+// scheduler, between cache latencies.  So the four warps (one per scheduler)
+// share what one would do alone, what depends on the solve only (the rotated
+// references, the positions' records) is computed before the wait for the
+// previous kernel, and S1 finds 1/||w|| beside ||w||.
 constexpr int kS1Blobs = 32;
 constexpr int kS1Tpb = 128;
 __global__ void __launch_bounds__(kS1Tpb) s1_update_normalise_moments_kernel(
@@ -521,22 +542,33 @@ __global__ void __launch_bounds__(kS1Tpb) s1_update_normalise_moments_kernel(
     const double *__restrict__ mob_rot, const double *__restrict__ ktkf_rot, double minv, double *__restrict__ z,
     double *__restrict__ part, const double *__restrict__ scal, int *ticket, const GmresCtl *ctl)
 {
-    pdl_wait_then_release();
     static_assert(kS1Tpb == 4 * 32 && kS1Blobs == 32, "S1: four warps over 32 blobs");
-    if (ctl->done) return;
-    __shared__ double hs[kFMaxK];
+    __shared__ double hs[kFMaxK];  // h, then the new q of the CTA's blobs by component
     __shared__ double up[4][3 * kS1Blobs];
     __shared__ double upb[4][32];
     const int n = blockIdx.y, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nb = W * nblob;
     const int m = blockIdx.x * kS1Blobs + lane;
-    const int kq = ctl->k, cnt = kq - 1;  // the pending update spans Q[:, 0..cnt)
-    double *q = Q + ld * (size_t)(kq - 1);
-    const double nrm = scal[kNormOff], inrm = 1.0 / nrm;
-    for (int i = threadIdx.x; i < cnt; i += kS1Tpb) hs[i] = scal[kHOff + i];
-    __syncthreads();
+    // of the solve: R ref, the components that this warp's moment takes
+    const int c0 = wid % 3, c1 = (c0 + 1) % 3, c2 = (c0 + 2) % 3;
+    double d1 = 0.0, d2 = 0.0;
+    if (wid < 3 && m < nblob) {
+        d1 = rot_row(R + 9 * n + 3 * c1, refs + 3 * m);
+        d2 = rot_row(R + 9 * n + 3 * c2, refs + 3 * m);
+    }
+    pdl_wait_then_release();
+    // all first loads before the branch on one of them
+    const int done = ctl->done, kq = ctl->k, cnt = kq - 1;  // the pending update spans Q[:, 0..cnt)
+    const double inrm = scal[kNormOff + 1];
+    for (int i = threadIdx.x; i < kFMaxK; i += kS1Tpb) hs[i] = scal[kHOff + i];
     const size_t row = 3 * ((size_t)n * nblob + m);
+    double wc = 0.0;
+    if (wid < 3 && m < nblob) wc = w[row + c0];
+    if (done) return;
+    double *q = Q + ld * (size_t)(kq - 1);
+    __syncthreads();
     double p0 = 0.0, p1 = 0.0, p2 = 0.0;
     if (m < nblob)
+#pragma unroll 4
         for (int i = wid; i < cnt; i += 4) {
             const double *qi = Q + ld * i + row;
             p0 += hs[i] * qi[0];
@@ -555,47 +587,63 @@ __global__ void __launch_bounds__(kS1Tpb) s1_update_normalise_moments_kernel(
         upb[wid][lane] = pb;
     }
     __syncthreads();
-    if (body_cta && wid == 0 && br < 6 * W)
+    if (body_cta && wid == 3 && br < 6 * W)
         w[3 * (size_t)nb + br] -= (upb[0][lane] + upb[1][lane]) + (upb[2][lane] + upb[3][lane]);
-    double a[6] = {0, 0, 0, 0, 0, 0};
-    if (wid == 0 && m < nblob) {
-        double f[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int e = 3 * lane + c;
-            f[c] = (w[row + c] - ((up[0][e] + up[1][e]) + (up[2][e] + up[3][e]))) * inrm;
-            q[row + c] = f[c];
+    double f = 0.0;
+    if (wid < 3) {
+        if (m < nblob) {
+            const int e = 3 * lane + c0;
+            f = (wc - ((up[0][e] + up[1][e]) + (up[2][e] + up[3][e]))) * inrm;
+            q[row + c0] = f;
         }
-        double d[3];
-        rot_apply(R + 9 * n, refs + 3 * m, d);
-        a[0] = f[0];
-        a[1] = f[1];
-        a[2] = f[2];
-        a[3] = d[1] * f[2] - d[2] * f[1];
-        a[4] = d[2] * f[0] - d[0] * f[2];
-        a[5] = d[0] * f[1] - d[1] * f[0];
+        hs[32 * c0 + lane] = f;
     }
-    block_sum6<kS1Tpb>(a, part + ((size_t)n * gridDim.x + blockIdx.x) * 6);
+    __syncthreads();
+    if (wid < 3) {  // the force's and the torque's component c0, over the CTA's blobs
+        const double t = warp_sum2(f, m < nblob ? d1 * hs[32 * c2 + lane] - d2 * hs[32 * c1 + lane] : 0.0);
+        if ((lane & 15) == 0) part[((size_t)n * gridDim.x + blockIdx.x) * 6 + c0 + (lane == 16 ? 3 : 0)] = t;
+    }
     if (!last_cta(ticket, gridDim.x * gridDim.y)) return;
-    extern __shared__ double sh[];  // 6 W moments of q, then 6 W of z_body
+    extern __shared__ double sh[];  // 6 W moments of q, then 6 W of mob_rot w_body, in its place z_body
     double *zsh = sh + 6 * W;
-    swimmer_sums(part, W, gridDim.x, sh);
-    // body rows of q, and z_body = KTKinv_rot (-sums) - mob_rot q_body: one
-    // thread per (swimmer, row), the products in two interleaved chains each
-    for (int e = threadIdx.x; e < 6 * W; e += kS1Tpb) {
+    // the first rows' matrices, on their way while the moments are added
+    double kt[6], kf[6];
+    if (threadIdx.x < 6 * W)
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            kt[j] = ktk_rot[36 * (threadIdx.x / 6) + 6 * j + threadIdx.x % 6];
+            kf[j] = ktkf_rot[36 * (threadIdx.x / 6) + 6 * j + threadIdx.x % 6];
+        }
+    // body rows of q, and the part of z_body that does not wait for the
+    // moments, from the last warp on
+    for (int e = (threadIdx.x + 32) % kS1Tpb; e < 6 * W; e += kS1Tpb) {
         const int sw = e / 6, i = e % 6;
-        const double *sums = sh + 6 * sw, *wb = w + 3 * (size_t)nb + 6 * sw;
+        const double *wb = w + 3 * (size_t)nb + 6 * sw, *Mb = mob_rot + 36 * sw + i;
         q[3 * nb + e] = __ldcg(wb + i) * inrm;
-        const double *Kt = ktk_rot + 36 * sw + i, *Mb = mob_rot + 36 * sw + i;
-        double x0 = 0.0, x1 = 0.0, y0 = 0.0, y1 = 0.0;
+        double y0 = 0.0, y1 = 0.0;
 #pragma unroll
         for (int j = 0; j < 6; j += 2) {
-            x0 += Kt[6 * j] * (-sums[j]);
-            x1 += Kt[6 * (j + 1)] * (-sums[j + 1]);
             y0 += Mb[6 * j] * __ldcg(wb + j);
             y1 += Mb[6 * (j + 1)] * __ldcg(wb + j + 1);
         }
-        const double zb = (x0 + x1) - (y0 + y1) * inrm;
+        zsh[e] = y0 + y1;
+    }
+    swimmer_sums(part, W, gridDim.x, sh);
+    // z_body = KTKinv_rot (-sums) - mob_rot q_body: one thread per (swimmer,
+    // row), the products in two interleaved chains each
+    for (int e = threadIdx.x; e < 6 * W; e += kS1Tpb) {
+        const int sw = e / 6, i = e % 6;
+        const double *sums = sh + 6 * sw;
+        if (e >= kS1Tpb)
+#pragma unroll
+            for (int j = 0; j < 6; ++j) kt[j] = ktk_rot[36 * sw + 6 * j + i];
+        double x0 = 0.0, x1 = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; j += 2) {
+            x0 += kt[j] * (-sums[j]);
+            x1 += kt[j + 1] * (-sums[j + 1]);
+        }
+        const double zb = (x0 + x1) - zsh[e] * inrm;
         z[3 * nb + e] = zb;
         zsh[e] = zb;
     }
@@ -606,12 +654,15 @@ __global__ void __launch_bounds__(kS1Tpb) s1_update_normalise_moments_kernel(
     // the blobs of z, mobility_solver.cpp:921-940)
     for (int e = threadIdx.x; e < 6 * W; e += kS1Tpb) {
         const int sw = e / 6, i = e % 6;
-        const double *Kf = ktkf_rot + 36 * sw + i, *zb = zsh + 6 * sw;
+        const double *zb = zsh + 6 * sw;
+        if (e >= kS1Tpb)
+#pragma unroll
+            for (int j = 0; j < 6; ++j) kf[j] = ktkf_rot[36 * sw + 6 * j + i];
         double x0 = 0.0, x1 = 0.0;
 #pragma unroll
         for (int j = 0; j < 6; j += 2) {
-            x0 += Kf[6 * j] * zb[j];
-            x1 += Kf[6 * (j + 1)] * zb[j + 1];
+            x0 += kf[j] * zb[j];
+            x1 += kf[j + 1] * zb[j + 1];
         }
         double v = sh[e] + (x0 + x1);
         for (int k = sw; k < W; ++k) v *= minv;
@@ -629,15 +680,27 @@ __global__ void __launch_bounds__(kSBlobs) s2_precond_blobs_kernel(
     const double *__restrict__ refs, double minv, const double *__restrict__ xb, double *__restrict__ z, void *rec,
     int f64, const GmresCtl *ctl)
 {
-    pdl_wait_then_release();
-    if (ctl->done) return;
     const int n = blockIdx.y, m = blockIdx.x * kSBlobs + threadIdx.x, nb = W * nblob;
-    if (m >= nblob) return;
-    const double *in = Q + ld * (size_t)(ctl->k - 1);
-    const double *U = z + 3 * nb + 6 * n;
     const size_t i = (size_t)n * nblob + m;
-    double d[3];
-    rot_apply(R + 9 * n, refs + 3 * m, d);
+    // of the solve: R ref and the position's part of the record
+    double d[3] = {0.0, 0.0, 0.0}, x[3] = {0.0, 0.0, 0.0};
+    float hi[3], lo[3];
+    if (m < nblob) {
+        rot_apply(R + 9 * n, refs + 3 * m, d);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (rec != nullptr) x[c] = xb[3 * i + c];
+            hi[c] = (float)x[c];
+            lo[c] = (float)(x[c] - widen(hi[c]));
+        }
+    }
+    pdl_wait_then_release();
+    const int done = ctl->done, kq = ctl->k;
+    double U[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) U[c] = z[3 * nb + 6 * n + c];
+    if (done || m >= nblob) return;
+    const double *in = Q + ld * (size_t)(kq - 1);
     double o[3] = {in[3 * i] + U[0], in[3 * i + 1] + U[1], in[3 * i + 2] + U[2]};
     o[0] += U[4] * d[2] - U[5] * d[1];
     o[1] += U[5] * d[0] - U[3] * d[2];
@@ -650,7 +713,15 @@ __global__ void __launch_bounds__(kSBlobs) s2_precond_blobs_kernel(
     z[3 * i] = o[0];
     z[3 * i + 1] = o[1];
     z[3 * i + 2] = o[2];
-    if (rec != nullptr) pack_record(rec, (int)i, xb + 3 * i, o, f64);
+    if (rec == nullptr) return;
+    if (f64) {
+        pack_record(rec, (int)i, x, o, f64);
+    } else {  // pack_record's record
+        float4 *r = static_cast<float4 *>(rec) + 3 * i;
+        r[0] = make_float4(hi[0], hi[1], hi[2], (float)o[0]);
+        r[1] = make_float4(lo[0], lo[1], lo[2], (float)o[1]);
+        r[2] = make_float4((float)o[2], 0.f, 0.f, 0.f);
+    }
 }
 
 // Column sums out[i * ostride] = sum over b < count of p[i * stride + b],
@@ -740,13 +811,28 @@ __global__ void __launch_bounds__(kSTpb) s3_finish_project_kernel(
     double *__restrict__ G, int *tickets, double *__restrict__ scal, double *__restrict__ H, int ldh,
     double *__restrict__ beta, double *__restrict__ cs, double *__restrict__ sn, GmresCtl *ctl, double eta2)
 {
-    pdl_wait_then_release();
     static_assert(kSTpb == 4 * kSRows && kSRows == 32, "S3's split sum: four warps over 32 rows");
-    if (ctl->done) return;
     __shared__ double ws[kSRows];
     __shared__ double msum[4][kSRows];
-    const int k = ctl->k, row0 = blockIdx.x * kSRows, nb3 = 3 * W * nblob;
+    const int row0 = blockIdx.x * kSRows, nb3 = 3 * W * nblob;
     const int rows = min(kSRows, n - row0);
+    // of the solve: the rows' blobs, and the components of R ref that K z takes
+    const int kr = row0 + threadIdx.x, kc = kr % 3, sw = kr / 3 / nblob;
+    double d1 = 0.0, d2 = 0.0;
+    if (threadIdx.x < kSRows && kr < nb3) {
+        const double *ref = refs + 3 * (kr / 3 % nblob);
+        d1 = rot_row(R + 9 * sw + 3 * ((kc + 1) % 3), ref);
+        d2 = rot_row(R + 9 * sw + 3 * ((kc + 2) % 3), ref);
+    }
+    pdl_wait_then_release();
+    const int done = ctl->done, k = ctl->k;
+    double u0 = 0.0, u1 = 0.0, u2 = 0.0;
+    if (threadIdx.x < kSRows && kr < nb3) {
+        const double *U = z + nb3 + 6 * sw;
+        u0 = U[kc];
+        u1 = U[3 + (kc + 2) % 3];
+        u2 = U[3 + (kc + 1) % 3];
+    }
     if (splits > 1) {
         const int lr = threadIdx.x & 31, q = threadIdx.x >> 5, r = row0 + lr;
         double a0 = 0.0, a1 = 0.0;
@@ -759,22 +845,16 @@ __global__ void __launch_bounds__(kSTpb) s3_finish_project_kernel(
             if (p < splits) a0 += mpart[(size_t)p * nb3 + r];
         }
         msum[q][lr] = a0 + a1;
-        __syncthreads();
     }
+    if (done) return;
+    if (splits > 1) __syncthreads();
     if (threadIdx.x < kSRows) {
         const int r = row0 + threadIdx.x;
         double v = 0.0;
         if (r < nb3) {
-            const int i = r / 3, c = r % 3, sw = i / nblob, m = i % nblob;
-            double d[3];
-            rot_apply(R + 9 * sw, refs + 3 * m, d);
-            const double *U = z + nb3 + 6 * sw;
-            double kz;
-            if (c == 0) kz = U[0] - d[1] * U[5] + d[2] * U[4];
-            else if (c == 1) kz = U[1] - d[2] * U[3] + d[0] * U[5];
-            else kz = U[2] - d[0] * U[4] + d[1] * U[3];
             const int t = threadIdx.x;
             const double mb = splits > 1 ? (msum[0][t] + msum[1][t]) + (msum[2][t] + msum[3][t]) : mbb[r];
+            const double kz = u0 - d1 * u1 + d2 * u2;  // (U + Omega x (R ref))_kc
             v = -kz + mb;
             w[r] = v;
         } else if (r < n) {
@@ -880,6 +960,7 @@ __device__ __forceinline__ void givens_step(double *__restrict__ H, int ldh, int
         }
     }
     __syncthreads();
+    if (threadIdx.x == 32) scal[kNormOff + 1] = 1.0 / nrm;  // for S1, beside warp 0's chain
     if (threadIdx.x >= 32) return;
     const int lane = threadIdx.x;
     // The previous rotations over the new H column, as a warp scan: entry i
@@ -1496,6 +1577,7 @@ static gmi_status gmres_run(gmi_solver *s, double norm_b, double norm_ref, doubl
         }
     }
     s->h_stage[0] = beta0;
+    s->h_stage[1] = 1.0 / beta0;
     GMI_CUDA_TRY(cudaMemcpyAsync(s->beta, s->h_stage, sizeof(double), cudaMemcpyHostToDevice, st));
     const int max_iter = n < s->m ? n : s->m;
     const int ldh = s->m + 1;
@@ -1532,7 +1614,7 @@ static gmi_status gmres_run(gmi_solver *s, double norm_b, double norm_ref, doubl
     if (cluster || s->use_graphs) {
       if (!cluster) {
         // the first step normalises w = r0 by beta0 into Q[:, 0]
-        GMI_CUDA_TRY(cudaMemcpyAsync(s->st_scal + kNormOff, s->h_stage, sizeof(double), cudaMemcpyHostToDevice, st));
+        GMI_CUDA_TRY(cudaMemcpyAsync(s->st_scal + kNormOff, s->h_stage, 2 * sizeof(double), cudaMemcpyHostToDevice, st));
         GmresCtl c{};
         c.k = 1;
         c.done = 0;

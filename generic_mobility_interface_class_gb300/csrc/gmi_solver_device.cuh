@@ -67,7 +67,22 @@ __device__ __forceinline__ bool last_cta(int *ticket, int total)
     return is_last;
 }
 
-// o = R v, R row-major 3x3
+// The same for two values: lanes 0..15 return the total of a, the others b's.
+__device__ __forceinline__ double warp_sum2(double a, double b)
+{
+    const unsigned full = 0xffffffffu;
+    const bool h16 = (threadIdx.x & 16) != 0;
+    double t = (h16 ? b : a) + __shfl_xor_sync(full, h16 ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(full, t, o);
+    return t;
+}
+
+// a row of R v, and o = R v, R row-major 3x3
+__device__ __forceinline__ double rot_row(const double *R, const double *v)
+{
+    return R[0] * v[0] + R[1] * v[1] + R[2] * v[2];
+}
 __device__ __forceinline__ void rot_apply(const double *R, const double *v, double *o)
 {
     o[0] = R[0] * v[0] + R[1] * v[1] + R[2] * v[2];
