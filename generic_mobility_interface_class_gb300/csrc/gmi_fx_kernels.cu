@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kFxBlock) fx_pack_kernel(const double *__restr
                                                           int n, FxConsts K, int4 *__restrict__ rec, const int *skip)
 {
     __shared__ int wmax[kFxBlock / 32];
-    pdl_wait_then_release();
+    pdl_wait();
     if (skip != nullptr && *skip != 0) return;
     const int i = blockIdx.x * kFxBlock + threadIdx.x;
     FxPacking<KIND> p;
@@ -497,8 +497,8 @@ gmi_status launch_pair_fx(const FxPairSum &s, int *launched)
         // a kernel of its own: the last CTA of a target group adding the
         // group's partials took 2 us longer (320 segments: 18.5, 16.4 us)
         const int count = s.n_tgt * nout;
-        GMI_CUDA_TRY(launch_chained(true, reduce_splits, dim3((count + 255) / 256), dim3(256), s.stream, a.partial, splits,
-                                    count, a.out, a.accumulate, nullptr));
+        GMI_CUDA_TRY(launch_chained(true, reduce_splits_tree, dim3((count + 63) / 64), dim3(64), s.stream, a.partial,
+                                    splits, count, s.out, s.accumulate));
         ++*launched;
     }
     return GMI_OK;

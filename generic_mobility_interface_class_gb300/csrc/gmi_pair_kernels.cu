@@ -38,15 +38,23 @@ constexpr int kStages = 4;   // depth of the shared-memory ring
 // ---------------------------------------------------------------------------
 // 1. pack kernels
 // ---------------------------------------------------------------------------
+// release: the next kernel on the stream may take its place early.  The pack
+// kernels of a sum between two sets do so (12,800 segments with 4096 blobs in
+// FP32, both ways: 176 us, 182 without) and those of small sums (1500 blobs
+// 23.2 us, 23.9); a larger set's does not (4096 blobs 30.7 us, 32.8 with it;
+// 2501 segments 28.0, 28.7).
 __global__ void pack_records_f32(const double *__restrict__ x, const double *__restrict__ f, int nf, int n,
-                                 float4 *__restrict__ rec)
+                                 float4 *__restrict__ rec, int release)
 {
-    pdl_wait_then_release();
+    if (release != 0)
+        pdl_wait_then_release();
+    else
+        pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double px = x[3 * i], py = x[3 * i + 1], pz = x[3 * i + 2];
     const float hx = (float)px, hy = (float)py, hz = (float)pz;
-    const float lx = (float)(px - (double)hx), ly = (float)(py - (double)hy), lz = (float)(pz - (double)hz);
+    const float lx = (float)(px - widen(hx)), ly = (float)(py - widen(hy)), lz = (float)(pz - widen(hz));
     float f0 = 0.f, f1 = 0.f, f2 = 0.f, t0 = 0.f, t1 = 0.f, t2 = 0.f;
     if (f != nullptr) {
         f0 = (float)f[nf * i];
@@ -71,7 +79,7 @@ __global__ void pack_records_f32(const double *__restrict__ x, const double *__r
 __global__ void pack_records_df(const double *__restrict__ x, const double *__restrict__ f, int n,
                                 float4 *__restrict__ rec)
 {
-    pdl_wait_then_release();
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const df2 px = df_from_double(x[3 * i] - x[0]), py = df_from_double(x[3 * i + 1] - x[1]),
@@ -89,9 +97,12 @@ __global__ void pack_records_df(const double *__restrict__ x, const double *__re
 }
 
 __global__ void pack_records_f64(const double *__restrict__ x, const double *__restrict__ f, int nf, int n,
-                                 double2 *__restrict__ rec)
+                                 double2 *__restrict__ rec, int release)
 {
-    pdl_wait_then_release();
+    if (release != 0)
+        pdl_wait_then_release();
+    else
+        pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double f0 = 0, f1 = 0, f2 = 0, t0 = 0, t1 = 0, t2 = 0;
@@ -1436,13 +1447,13 @@ gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int 
     if (st != GMI_OK) return st;
     if (n == 0) return GMI_OK;
     const int tpb = 256;
-    const int grid = (n + tpb - 1) / tpb;
+    const int grid = (n + tpb - 1) / tpb, release = f == nullptr || chained || n <= kPairWarpMaxSources ? 1 : 0;
     if (f64)
         GMI_CUDA_TRY(launch_chained(chained, pack_records_f64, dim3(grid), dim3(tpb), ctx->stream, x, f, nf, n,
-                                    static_cast<double2 *>(buf.ptr)));
+                                    static_cast<double2 *>(buf.ptr), release));
     else
         GMI_CUDA_TRY(launch_chained(chained, pack_records_f32, dim3(grid), dim3(tpb), ctx->stream, x, f, nf, n,
-                                    static_cast<float4 *>(buf.ptr)));
+                                    static_cast<float4 *>(buf.ptr), release));
     ctx->launches++;
     return GMI_OK;
 }
@@ -2025,9 +2036,9 @@ gmi_status pack_records_into(cudaStream_t stream, bool f64, const double *x, con
     if (n == 0) return GMI_OK;
     const int tpb = 256, grid = (n + tpb - 1) / tpb;
     if (f64)
-        pack_records_f64<<<grid, tpb, 0, stream>>>(x, f, nf, n, static_cast<double2 *>(dst));
+        pack_records_f64<<<grid, tpb, 0, stream>>>(x, f, nf, n, static_cast<double2 *>(dst), 0);
     else
-        pack_records_f32<<<grid, tpb, 0, stream>>>(x, f, nf, n, static_cast<float4 *>(dst));
+        pack_records_f32<<<grid, tpb, 0, stream>>>(x, f, nf, n, static_cast<float4 *>(dst), 0);
     GMI_CUDA_TRY(cudaGetLastError());
     return GMI_OK;
 }

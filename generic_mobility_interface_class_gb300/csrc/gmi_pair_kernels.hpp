@@ -57,7 +57,7 @@ void fill_consts(PairConsts &c, double a_eq, double a_seg, double a_blob, double
 
 // Pack AoS FP64 positions (and forces with nf = 3 or 6 components, or none
 // when f == nullptr) into the context's record format for its precision.
-// `chained`: launch_chained after an earlier kernel of the same call.
+// `chained`: launch_chained after the targets' pack kernel of the same call.
 gmi_status pack_records(gmi_context *ctx, const double *x, const double *f, int nf, int n, DeviceBuffer &buf,
                         bool chained = false);
 

@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kSBlobs) s2_precond_blobs_kernel(
             lo[c] = (float)(x[c] - widen(hi[c]));
         }
     }
-    pdl_wait_then_release();
+    pdl_wait();
     const int done = ctl->done, kq = ctl->k;
     double U[6];
 #pragma unroll
@@ -1266,7 +1266,7 @@ static void ktk_from_refs(const double *refs, int nblob, double *KTK)
 
 // A kernel launch of the Arnoldi step; with pdl, marked for programmatic
 // dependent launch, so that it may start while the previous kernel finishes
-// (each step kernel waits first, in pdl_wait_then_release).
+// (each step kernel waits for the one before it, in pdl_wait).
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_step(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                cudaStream_t st, Args... args)
