@@ -797,9 +797,100 @@ __device__ __forceinline__ bool finish_projections(const double *P, int k, int n
     return true;
 }
 
-__device__ __forceinline__ void givens_step(double *__restrict__ H, int ldh, int iter, double nrm,
-                                            double *__restrict__ beta, double *__restrict__ cs,
-                                            double *__restrict__ sn, double *__restrict__ scal, GmresCtl *ctl);
+// The Givens step of solve_linear_system (mobility_solver.cpp:1189-1231) on
+// H column iter-1, run by the last CTA of S3 or S4: the previous rotations over
+// the column (givens_scan, warp 0), then, with the column's subdiagonal entry
+// nrm, the new rotation, beta, the residual and the iteration control
+// (givens_finish).  The scan does not need nrm, so warp 1 forms it meanwhile.
+// The column and the rotations lie in shared memory, so the sequential parts
+// read no global memory.
+struct GivensColumn {
+    double col[kFMaxK + 1], cs[kFMaxK], sn[kFMaxK];
+};
+
+// The previous rotations over the new H column, as a warp scan: entry i
+// after rotation i is x_i = -s_{i-1} x_{i-1} + c_{i-1} col_i, a
+// first-order linear recurrence (x -> a x + b pairs, Kogge-Stone over 32
+// entries at a time); the rotated entries are c_{i-1} x_{i-1} + s_{i-1}
+// col_i.  (One thread's serial sweep costs ~64 cycles per FP64 step here.)
+// Returns the column's last entry.
+__device__ __forceinline__ double givens_scan(GivensColumn &g, int iter)
+{
+    const int lane = threadIdx.x & 31;
+    double xin = 0.0;
+    for (int base = 0; base < iter; base += 32) {
+        const int i = base + lane;
+        double aa = 1.0, bb = 0.0, cur = 0.0;
+        if (i < iter) {
+            cur = g.col[i];
+            if (i == 0) {
+                aa = 0.0;
+                bb = cur;
+            } else {
+                aa = -g.sn[i - 1];
+                bb = g.cs[i - 1] * cur;
+            }
+        }
+        for (int o = 1; o < 32; o <<= 1) {
+            const double ap = __shfl_up_sync(0xffffffffu, aa, o), bp = __shfl_up_sync(0xffffffffu, bb, o);
+            if (lane >= o) {
+                bb = fma(aa, bp, bb);
+                aa = aa * ap;
+            }
+        }
+        const double xi = fma(aa, xin, bb);
+        double xm1 = __shfl_up_sync(0xffffffffu, xi, 1);
+        if (lane == 0) xm1 = xin;
+        if (i >= 1 && i < iter) g.col[i - 1] = g.cs[i - 1] * xm1 + g.sn[i - 1] * cur;
+        xin = __shfl_sync(0xffffffffu, xi, 31);  // lanes past the column repeat its last entry
+    }
+    return xin;
+}
+
+// hd: givens_scan's result, in warp 0.
+__device__ __forceinline__ void givens_finish(GivensColumn &g, double hd, double *__restrict__ H, int ldh, int iter,
+                                              double nrm, double *__restrict__ beta, double *__restrict__ cs,
+                                              double *__restrict__ sn, double *__restrict__ scal, GmresCtl *ctl)
+{
+    if (threadIdx.x == 32) scal[kNormOff + 1] = 1.0 / nrm;  // for S1, beside warp 0's chain
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    if (lane == 0) {
+        scal[kNormOff] = nrm;
+        const double hk = nrm;
+        double c, s;
+        if (hk == 0.0) {
+            c = 1.0;
+            s = 0.0;
+        } else if (fabs(hk) > fabs(hd)) {  // the reference's scaled form; rsqrt saves a division
+            const double u = hd / hk;
+            s = (2.0 * (double)(hk > 0) - 1.0) * rsqrt(1.0 + u * u);
+            c = u * s;
+        } else {
+            const double u = hk / hd;
+            c = (2.0 * (double)(hd > 0) - 1.0) * rsqrt(1.0 + u * u);
+            s = u * c;
+        }
+        cs[iter - 1] = c;
+        sn[iter - 1] = s;
+        g.col[iter - 1] = c * hd + s * hk;
+        g.col[iter] = 0.0;
+        beta[iter] = -s * beta[iter - 1];
+        beta[iter - 1] = c * beta[iter - 1];
+        const double resid = fabs(beta[iter]) * ctl->inv_norm_ref;
+        ctl->resid = resid;
+        const int replays = ++ctl->replays;
+        // converged, at the cap, or NaN; the replay count bounds the loop even if k stalled
+        const bool done = !(resid > ctl->tol) || iter >= ctl->max_iter || replays > ctl->max_iter;
+        if (done)
+            ctl->done = 1;
+        else
+            ctl->k = iter + 1;
+    }
+    __syncwarp();
+    double *gcol = H + (size_t)ldh * (iter - 1);
+    for (int i = lane; i <= iter; i += 32) gcol[i] = g.col[i];
+}
 
 // S3: blob rows of w, first CGS pass.  With splits > 1 the blob-blob pair
 // sum left per-split partials (mpart[p * 3B + r]), which this kernel adds:
@@ -872,8 +963,18 @@ __global__ void __launch_bounds__(kSTpb) s3_finish_project_kernel(
     }
     double *h = scal + kHOff;
     if (!finish_projections(P, dgks ? k + 1 : k, gridDim.x, G, tickets, h)) return;
+    __shared__ GivensColumn g;
     double *Hcol = H + (size_t)ldh * (k - 1);
-    for (int i = threadIdx.x; i < k; i += kSTpb) Hcol[i] = h[i];
+    for (int i = threadIdx.x; i < k; i += kSTpb) {
+        const double v = h[i];
+        Hcol[i] = v;  // for S4, where it runs
+        g.col[i] = v;
+        if (i < k - 1) {
+            g.cs[i] = cs[i];
+            g.sn[i] = sn[i];
+        }
+    }
+    __syncthreads();
     // Conditional re-orthogonalisation (Daniel, Gragg, Kaufman and Stewart):
     // after one classical pass ||w - Q h||^2 = ||w||^2 - ||h||^2; when that
     // keeps at least eta^2 of ||w||^2 (eta = 1/sqrt 2: "twice is enough"),
@@ -883,25 +984,28 @@ __global__ void __launch_bounds__(kSTpb) s3_finish_project_kernel(
     // pending update w -= Q h with these first-pass coefficients.
     __shared__ double nrm_s;
     __shared__ int skip_s;
+    double hd = 0.0;
     if (threadIdx.x < 32) {
+        if (dgks) hd = givens_scan(g, k);
+    } else if (threadIdx.x < 64) {
         int skip = 0;
         double nrm = 0.0;
         if (dgks) {
             double t = 0.0;
-            for (int i = threadIdx.x; i < k; i += 32) t += h[i] * h[i];
+            for (int i = threadIdx.x - 32; i < k; i += 32) t += h[i] * h[i];
             t = warp_sum(t);
             const double w2 = h[k], after = w2 - t;
             skip = (w2 > 0.0 && after >= eta2 * w2 && after < INFINITY) ? 1 : 0;
             nrm = skip ? sqrt(after) : 0.0;
         }
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 32) {
             nrm_s = nrm;
             skip_s = skip;
             ctl->pass2 = skip ? 0 : 1;
         }
     }
-    __syncthreads();  // the H column is written; the decision is shared
-    if (skip_s) givens_step(H, ldh, k, nrm_s, beta, cs, sn, scal, ctl);
+    __syncthreads();  // the decision is shared
+    if (skip_s) givens_finish(g, hd, H, ldh, k, nrm_s, beta, cs, sn, scal, ctl);
 }
 
 // w -= Q h on this CTA's rows (rows go to ws): warp q takes the columns
@@ -940,97 +1044,6 @@ __device__ __forceinline__ void cta_update(const double *__restrict__ Q, size_t 
     __syncthreads();
 }
 
-// The Givens step of solve_linear_system (mobility_solver.cpp:1189-1231) on
-// H column iter-1, whose subdiagonal entry is nrm, run by the last CTA of
-// S4 (all of its threads enter; warp 0 does the work): the previous
-// rotations over the column, the new rotation, beta, the residual and the
-// iteration control.  The H column and the rotations go to shared memory
-// first, so the sequential parts read no global memory.
-__device__ __forceinline__ void givens_step(double *__restrict__ H, int ldh, int iter, double nrm,
-                                            double *__restrict__ beta, double *__restrict__ cs,
-                                            double *__restrict__ sn, double *__restrict__ scal, GmresCtl *ctl)
-{
-    __shared__ double col[kFMaxK + 1], csh[kFMaxK], snh[kFMaxK];
-    double *gcol = H + (size_t)ldh * (iter - 1);
-    for (int i = threadIdx.x; i < iter; i += blockDim.x) {
-        col[i] = gcol[i];
-        if (i < iter - 1) {
-            csh[i] = cs[i];
-            snh[i] = sn[i];
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 32) scal[kNormOff + 1] = 1.0 / nrm;  // for S1, beside warp 0's chain
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    // The previous rotations over the new H column, as a warp scan: entry i
-    // after rotation i is x_i = -s_{i-1} x_{i-1} + c_{i-1} col_i, a
-    // first-order linear recurrence (x -> a x + b pairs, Kogge-Stone over 32
-    // entries at a time); the rotated entries are c_{i-1} x_{i-1} + s_{i-1}
-    // col_i.  (One thread's serial sweep costs ~64 cycles per FP64 step here.)
-    double xin = 0.0;
-    for (int base = 0; base < iter; base += 32) {
-        const int i = base + lane;
-        double aa = 1.0, bb = 0.0, cur = 0.0;
-        if (i < iter) {
-            cur = col[i];
-            if (i == 0) {
-                aa = 0.0;
-                bb = cur;
-            } else {
-                aa = -snh[i - 1];
-                bb = csh[i - 1] * cur;
-            }
-        }
-        for (int o = 1; o < 32; o <<= 1) {
-            const double ap = __shfl_up_sync(0xffffffffu, aa, o), bp = __shfl_up_sync(0xffffffffu, bb, o);
-            if (lane >= o) {
-                bb = fma(aa, bp, bb);
-                aa = aa * ap;
-            }
-        }
-        const double xi = fma(aa, xin, bb);
-        double xm1 = __shfl_up_sync(0xffffffffu, xi, 1);
-        if (lane == 0) xm1 = xin;
-        if (i >= 1 && i < iter) col[i - 1] = csh[i - 1] * xm1 + snh[i - 1] * cur;
-        xin = __shfl_sync(0xffffffffu, xi, 31);  // lanes past the column repeat its last entry
-    }
-    if (lane == 0) {
-        scal[kNormOff] = nrm;
-        const double hk = nrm, hd = xin;
-        double c, s;
-        if (hk == 0.0) {
-            c = 1.0;
-            s = 0.0;
-        } else if (fabs(hk) > fabs(hd)) {  // the reference's scaled form; rsqrt saves a division
-            const double u = hd / hk;
-            s = (2.0 * (double)(hk > 0) - 1.0) * rsqrt(1.0 + u * u);
-            c = u * s;
-        } else {
-            const double u = hk / hd;
-            c = (2.0 * (double)(hd > 0) - 1.0) * rsqrt(1.0 + u * u);
-            s = u * c;
-        }
-        cs[iter - 1] = c;
-        sn[iter - 1] = s;
-        col[iter - 1] = c * hd + s * hk;
-        col[iter] = 0.0;
-        beta[iter] = -s * beta[iter - 1];
-        beta[iter - 1] = c * beta[iter - 1];
-        const double resid = fabs(beta[iter]) * ctl->inv_norm_ref;
-        ctl->resid = resid;
-        const int replays = ++ctl->replays;
-        // converged, at the cap, or NaN; the replay count bounds the loop even if k stalled
-        const bool done = !(resid > ctl->tol) || iter >= ctl->max_iter || replays > ctl->max_iter;
-        if (done)
-            ctl->done = 1;
-        else
-            ctl->k = iter + 1;
-    }
-    __syncwarp();
-    for (int i = lane; i <= iter; i += 32) gcol[i] = col[i];
-}
-
 // S4: second CGS pass.  w -= Q h1 (S3's projections), then h2 = Q^T w and,
 // as one more projection column, ||w||^2.  The last CTA adds h2 to the H
 // column and takes the new basis vector's norm as
@@ -1058,16 +1071,27 @@ __global__ void __launch_bounds__(kSTpb) s4_project_norm_givens_kernel(
     }
     // h is overwritten only after every CTA has read it (all arrived)
     if (!finish_projections(P, k + 1, gridDim.x, G, tickets, h)) return;
-    double *Hcol = H + (size_t)ldh * (k - 1);
-    for (int i = threadIdx.x; i < k; i += kSTpb) Hcol[i] += h[i];
-    if (threadIdx.x < 32) {
-        double t = 0.0;
-        for (int i = threadIdx.x; i < k; i += 32) t += h[i] * h[i];
-        t = warp_sum(t);
-        if (threadIdx.x == 0) nrm_s = sqrt(fmax(h[k] - t, 0.0));
+    __shared__ GivensColumn g;
+    const double *Hcol = H + (size_t)ldh * (k - 1);
+    for (int i = threadIdx.x; i < k; i += kSTpb) {
+        g.col[i] = Hcol[i] + h[i];
+        if (i < k - 1) {
+            g.cs[i] = cs[i];
+            g.sn[i] = sn[i];
+        }
     }
     __syncthreads();
-    givens_step(H, ldh, k, nrm_s, beta, cs, sn, scal, ctl);
+    double hd = 0.0;
+    if (threadIdx.x < 32) {
+        hd = givens_scan(g, k);
+    } else if (threadIdx.x < 64) {
+        double t = 0.0;
+        for (int i = threadIdx.x - 32; i < k; i += 32) t += h[i] * h[i];
+        t = warp_sum(t);
+        if (threadIdx.x == 32) nrm_s = sqrt(fmax(h[k] - t, 0.0));
+    }
+    __syncthreads();
+    givens_finish(g, hd, H, ldh, k, nrm_s, beta, cs, sn, scal, ctl);
 }
 
 // Last node of the device-side loop's body: one thread decides whether the
