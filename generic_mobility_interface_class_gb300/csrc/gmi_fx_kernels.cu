@@ -172,13 +172,18 @@ struct FxSum {
     double v[6];
 };
 
-// The sources [j0, j1) on one target in FP64, for the tiles and targets that
-// the fixed-point formats do not hold.
+// The sources [j0, j1) on one target in FP64, for the blocks and targets that
+// the fixed-point formats do not hold.  M_bb four at a time, for the loads in
+// flight (the others gain nothing and lose 0.6 % of the sums that do fit):
+// 12,800 blobs spread over 2400 radii 13.2 -> 12.2 ms (the tiled FP64 kernel,
+// which stages them in shared memory: 12.0).
 template <int KIND>
 static __device__ __noinline__ FxSum fx_sum_fp64(const FxLaunch &a, int ti, int j0, int j1)
 {
     FxSum s{};
     const double xi = a.xt[3 * (size_t)ti], yi = a.xt[3 * (size_t)ti + 1], zi = a.xt[3 * (size_t)ti + 2];
+    constexpr int kAtOnce = KIND == kFxBB ? 4 : 1;
+#pragma unroll kAtOnce
     for (int j = j0; j < j1; ++j) {
         double F[6] = {0, 0, 0, 0, 0, 0};
         for (int c = 0; c < FxTraits<KIND>::nf; ++c) F[c] = a.fs[FxTraits<KIND>::nf * (size_t)j + c];
