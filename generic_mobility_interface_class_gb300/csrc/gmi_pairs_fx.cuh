@@ -52,7 +52,7 @@ struct FxConsts {
     double as, ab, inv_as;     // radii (equal kinds: both the one radius)
     double a0, ar0;            // near field: 4U/(3a) (unequal: 4U/(3 as ab)), (U/a)^3
     fxop k3;                   // far field: (as^2 + ab^2) / (3 U^2)
-    long long t4;              // near up to r^2 = t4 U^2 (2^-58): (as + ab)^2
+    unsigned long long t4;     // near up to r^2 = t4 U^2 (2^-58): (as + ab)^2 < 36 U^2, so more than 63 bits
     fxop a_zero, ar_zero;      // at r = 0: A = 4U / (3 max(as, ab)), Ar = (U/a)^3
     fxop bb_b;                 // blob-blob near field: (U/a)^2, an eighth of it at scale 33
 };
@@ -183,7 +183,7 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
     }
     s.x *= 2.0f;
     const fxop ir = fx_rsqrt(s.h, s.x);  // 30
-    const bool near = k < 0 || (k <= 2 && s.h <= (K.t4 >> (2 * k)));
+    const bool near = k < 0 || (k <= 2 && (unsigned long long)s.h <= (K.t4 >> (2 * k)));
 
     fxop e[3];
     for (int c = 0; c < 3; ++c) e[c] = fx_product<29>(d[c], ir);
@@ -382,7 +382,7 @@ inline bool fx_consts(int kind, double as, double ab, double mu, FxConsts *K)
     K->a0 = equal ? 4.0 * U / (3.0 * as) : 4.0 * U / (3.0 * as * ab);
     K->ar0 = (U / as) * (U / as) * (U / as);
     K->k3 = fx_split(fx_rint((as * as + ab * ab) / (3.0 * U * U) * 1152921504606846976.0));  // 28
-    K->t4 = fx_rint((as + ab) * (as + ab) / (U * U) * 288230376151711744.0);
+    K->t4 = (unsigned long long)((as + ab) * (as + ab) / (U * U) * 288230376151711744.0);  // a whole number
     // the self term is the largest of most sums: the quotient's remainder too
     const double a3 = 3.0 * amax, a_zero = 4.0 * U / a3;
     K->a_zero = fx_from_double(a_zero);

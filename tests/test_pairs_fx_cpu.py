@@ -86,6 +86,23 @@ def test_fixed_point_sums_against_oracle(host, oracle_built, kind, a, b, layout)
         assert rel_err(got[:, block:block + 3], want[:, block:block + 3]) < n * 2.0 ** -52
 
 
+@pytest.mark.parametrize("kind", ["sb", "bs"])
+@pytest.mark.parametrize("small", [1.0, 1.42, 1.89, 1.95, 1.999, 0.95])
+@pytest.mark.parametrize("ratio", [1.5, 1.8, 2.0])
+@pytest.mark.parametrize("swap", [False, True])
+def test_near_field_limit_of_unequal_radii(host, oracle_built, kind, small, ratio, swap):
+    """Overlapping particles over the whole range of radii held: the limit of
+    the near field, ((a + b) / U)^2, reaches 36."""
+    a, b = (small, ratio * small)[::-1] if swap else (small, ratio * small)
+    n = 300
+    xt, xs, f = cloud(kind, "dense", n, small, seed=12)
+    status, got = fx_sum(host, kind, xt, xs, f, a, b)
+    assert status == 0
+    want = oracle_sum(oracle_built, kind, xt, xs, f, a, b)
+    for block in range(0, want.shape[1], 3):
+        assert rel_err(got[:, block:block + 3], want[:, block:block + 3]) < n * 2.0 ** -52
+
+
 @pytest.mark.parametrize("kind", ["ss", "bb"])
 def test_loads_of_very_different_sizes(host, oracle_built, kind):
     """Loads from 1e-9 to 1e9 in one tile, zero loads, and a whole tile of zeros."""

@@ -92,6 +92,19 @@ def test_slices_and_radii_ratio(gpu_ctx, oracle_built):
         check_all(gpu_ctx, rpy, xs, fs, xb, fb[:, :3], b=b)
 
 
+@pytest.mark.parametrize("a,b", [(0.95, 1.9), (1.9, 0.95), (1.95, 3.9), (3.7, 1.89)])
+def test_overlapping_unequal_radii(gpu_ctx, oracle_built, a, b):
+    """Radii whose near field, in the formats' units, ends furthest out."""
+    rng = np.random.default_rng(13)
+    xs, xb = (rng.uniform(-3.0 * min(a, b), 3.0 * min(a, b), size=(n, 3)) for n in (300, 200))
+    fs, fb, v = rng.normal(size=(300, 6)), rng.normal(size=(200, 3)), rng.normal(size=(300, 6))
+    gpu_ctx.set_precision(0)
+    got = T(v)
+    gpu_ctx.msb(T(xs), T(xb), T(fb), got, a_seg=a, a_blob=b)
+    assert rel_err(N(got), oracle_built.msb(xs, xb, fb, a, b, v_in=v)) < tol(500)
+    assert rel_err(N(gpu_ctx.mbs(T(xb), T(xs), T(fs), a_seg=a, a_blob=b)), oracle_built.mbs(xb, xs, fs, a, b)) < tol(500)
+
+
 def test_pinned_fp64_shape_keeps_its_kernel(gmi_lib, oracle_built):
     """A shape pinned in FP64 runs the FP64 kernel of that shape."""
     from generic_mobility_interface_class_gb300.mobility import Context
