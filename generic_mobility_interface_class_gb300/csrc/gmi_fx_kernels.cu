@@ -29,6 +29,8 @@
 // conversion): positions and loads become integers, and sums FP64 numbers, by
 // integer instructions.  With FP64 there, 642 segments took 28.6 us (now 20.5),
 // 962 41.0 (34.8), 1669 blobs 55.3 (45.1), a solve of 962 particles 4.25 ms (3.80).
+// A sum of wide sources only (gmi_pairs_fx.cuh), such as torques without forces,
+// takes 18 % longer in M_ss and 9 % in M_bs and M_sb; with loads alike none or 1 %.
 // Error against extended precision (2-norm, mean of four draws), FP64 kernel ->
 // this: 60 to 700 segments 0.81 to 0.96 of it, 1500 segments 2.9e-16 -> 1.9e-16;
 // 50 to 1200 blobs 0.65 to 0.95; segments on blobs and back 0.82 to 1.05.
@@ -50,14 +52,16 @@ constexpr int kFxTpb = 128;    // four warps
 constexpr int kFxWarps = kFxTpb / 32;
 constexpr int kFxStages = 2;
 constexpr int kFxInlinePerSm = 4;  // CTAs per SM up to which a CTA packs its own sources
-constexpr int kFxBadTile = -(1 << 22);  // in place of a block's exponent: sum it in FP64
+constexpr int kFxBadTile = -(1 << 15);  // in place of a block's exponent: sum it in FP64
 static_assert(kFxBlock == kFxWarps * kFxFold && kFxBlock % kFxTile == 0, "a warp's quarter of a block is one fold");
+static_assert(kFxTile == 32 * kFxWarps, "fx_place: four warps hold a tile's sources");
 
 template <int KIND> struct FxTraits {
     static constexpr bool torque = KIND == kFxSS || KIND == kFxBS;
     static constexpr int nout = (KIND == kFxSS || KIND == kFxSB) ? 6 : 3;
     static constexpr int nf = torque ? 6 : 3;
-    // 16-byte quarters per record: X0 X1 | X2 F0.h F0.hf | F0.lf F1 | F2 meta | T0 T1 | T2 pad
+    // 16-byte quarters per record: X0 X1 | X2 F0.h F0.hf | F0.lf F1 | F2 meta | T0 T1 | T2 T's gap, pad,
+    // meta: the block's exponent << 16 | the tile's records that are not wide << 8 | F's gap
     static constexpr int quads = torque ? 6 : 4;
 };
 
@@ -76,11 +80,11 @@ struct FxLaunch {
 };
 
 // One source on its way into a record: its position, its loads and their
-// exponent (torques over U).
+// exponent (torques over U), that of its force and of its torque.
 template <int KIND> struct FxPacking {
     long long X[3];
     double F[FxTraits<KIND>::nf];
-    int e;
+    int e, f, t;
 };
 constexpr int kFxMark = 0x7fffffff;  // as an exponent: the formats do not hold this source
 
@@ -93,12 +97,16 @@ __device__ __forceinline__ FxPacking<KIND> fx_read_source(const double *__restri
     bool ok = true;
 #pragma unroll
     for (int c = 0; c < 3; ++c) ok = fx_position(x[3 * (size_t)i + c], K, fx_origin(x[c], K), &p.X[c]) && ok;
-    p.e = kFxNoLoad;
+    p.f = p.t = kFxNoLoad;
 #pragma unroll
     for (int c = 0; c < Tr::nf; ++c) {
         p.F[c] = f[Tr::nf * (size_t)i + c];
-        p.e = max(p.e, fx_exponent(p.F[c], c < 3 ? 0 : K.unit_exp));
+        if (c < 3)
+            p.f = max(p.f, fx_exponent(p.F[c], 0));
+        else
+            p.t = max(p.t, fx_exponent(p.F[c], K.unit_exp));
     }
+    p.e = max(p.f, p.t);
     if (!ok || !fx_exponent_held(p.e)) p.e = kFxMark;
     return p;
 }
@@ -116,56 +124,91 @@ template <int NW> __device__ __forceinline__ int fx_block_max(int e, int *wmax)
     return e;
 }
 
+// Where a CTA's sources go in their tiles, the wide ones last, so that each kind
+// has a loop of its own: a choice in the one loop cost M_ss 4 % of its time whether
+// or not it met a wide source.  even: records of the tile that are not wide.
+struct FxPlace {
+    int at, even;
+};
+template <int KIND, int NW> __device__ __forceinline__ FxPlace fx_place(bool present, bool wide, int *counts)
+{
+    const int tid = threadIdx.x, warp = tid >> 5, first = warp & ~(kFxWarps - 1);
+    if (KIND == kFxBB) return FxPlace{tid, kFxTile};
+    const unsigned mine = __ballot_sync(0xffffffffu, present && !wide);
+    if ((tid & 31) == 0) counts[warp] = __popc(mine);
+    __syncthreads();
+    int before = __popc(mine & ((1u << (tid & 31)) - 1u)), even = 0;
+#pragma unroll
+    for (int w = 0; w < kFxWarps; ++w) {
+        const int n = counts[first + w];
+        before += first + w < warp ? n : 0;
+        even += n;
+    }
+    const int start = 32 * first;
+    return FxPlace{wide ? even + tid - before : start + before, even};
+}
+
 // The record of a source in a block whose largest exponent is E.
 template <int KIND>
-__device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E, const FxConsts &K, int4 *r)
+__device__ __forceinline__ void fx_write_record(const FxPacking<KIND> &p, int E, const FxHeld &h, int even,
+                                                const FxConsts &K, int4 *r)
 {
     using Tr = FxTraits<KIND>;
     const bool bad = E == kFxMark;
-    int gap = 0, used = 0;
-    if (!bad && p.e != kFxNoLoad) {
-        gap = min(E - p.e, kFxMaxGap);
-        used = E - gap;
-    }
-    const int tile = bad ? kFxBadTile : E == kFxNoLoad ? 0 : E;
+    const int tile = bad ? kFxBadTile : E;
+    const int meta = (int)((unsigned)tile << 16) | even << 8 | h.gap;
     const auto lo = [](long long v) { return (int)(unsigned)v; };
     const auto hi = [](long long v) { return (int)(v >> 32); };
     fxop F[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         long long v;
-        fx_fixed(p.F[c], 62 - used, &v);
+        fx_fixed(p.F[c], 62 - (tile - h.gap), &v);
         F[c] = bad ? fxop{0, 0.0f, 0.0f} : fx_split(v);
     }
     r[0] = make_int4(lo(p.X[0]), hi(p.X[0]), lo(p.X[1]), hi(p.X[1]));
     r[1] = make_int4(lo(p.X[2]), hi(p.X[2]), F[0].h, __float_as_int(F[0].hf));
     r[2] = make_int4(__float_as_int(F[0].lf), F[1].h, __float_as_int(F[1].hf), __float_as_int(F[1].lf));
-    r[3] = make_int4(F[2].h, __float_as_int(F[2].hf), __float_as_int(F[2].lf), (int)((unsigned)tile << 8) | gap);
+    r[3] = make_int4(F[2].h, __float_as_int(F[2].hf), __float_as_int(F[2].lf), meta);
     if constexpr (Tr::torque) {
         long long T[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            fx_fixed(p.F[3 + c], 62 - used - K.unit_exp, &T[c]);
+            fx_fixed(p.F[3 + c], 62 - (tile - h.tgap) - K.unit_exp, &T[c]);
             if (bad) T[c] = 0;
         }
         r[4] = make_int4(lo(T[0]), hi(T[0]), lo(T[1]), hi(T[1]));
-        r[5] = make_int4(lo(T[2]), hi(T[2]), 0, 0);
+        r[5] = make_int4(lo(T[2]), hi(T[2]), h.tgap, 0);
     }
+}
+
+// A CTA's records, NW tiles' quarters, the thread's source p into its tile of
+// `rec` (records of the CTA's first source on).
+template <int KIND, int NW>
+__device__ __forceinline__ void fx_write_records(const FxPacking<KIND> &p, bool present, const FxConsts &K, int *ints,
+                                                 int4 *rec)
+{
+    int E = fx_block_max<NW>(p.e, ints);
+    if (E == kFxNoLoad) E = 0;
+    FxHeld h{0, 0, false};
+    if (E != kFxMark) h = fx_held<KIND>(p.f, p.t, E);
+    const FxPlace to = fx_place<KIND, NW>(present, h.wide, ints + NW);
+    if (present) fx_write_record<KIND>(p, E, h, to.even, K, rec + (size_t)to.at * FxTraits<KIND>::quads);
 }
 
 template <int KIND>
 __global__ void __launch_bounds__(kFxBlock) fx_pack_kernel(const double *__restrict__ x, const double *__restrict__ f,
                                                           int n, FxConsts K, int4 *__restrict__ rec, const int *skip)
 {
-    __shared__ int wmax[kFxBlock / 32];
+    __shared__ int ints[2 * kFxBlock / 32];
     pdl_wait();
     if (skip != nullptr && *skip != 0) return;
     const int i = blockIdx.x * kFxBlock + threadIdx.x;
     FxPacking<KIND> p;
-    p.e = kFxNoLoad;
+    p.e = p.f = p.t = kFxNoLoad;
     if (i < n) p = fx_read_source<KIND>(x, f, i, K);
-    const int E = fx_block_max<kFxBlock / 32>(p.e, wmax);
-    if (i < n) fx_write_record<KIND>(p, E, K, rec + (size_t)i * FxTraits<KIND>::quads);
+    fx_write_records<KIND, kFxBlock / 32>(p, i < n, K, ints,
+                                          rec + (size_t)blockIdx.x * kFxBlock * FxTraits<KIND>::quads);
 }
 
 struct FxSum {
@@ -213,11 +256,13 @@ template <int KIND> __device__ __forceinline__ FxSource fx_load_source(const int
     s.F[1] = fxop{c.y, __int_as_float(c.z), __int_as_float(c.w)};
     s.F[2] = fxop{d.x, __int_as_float(d.y), __int_as_float(d.z)};
     s.gap = d.w & 255;
+    s.tgap = 0;
     if constexpr (FxTraits<KIND>::torque) {
         const int4 e = q[4], f = q[5];
         s.T[0] = fx_word(e.x, e.y);
         s.T[1] = fx_word(e.z, e.w);
         s.T[2] = fx_word(f.x, f.y);
+        s.tgap = f.z;
     }
     return s;
 }
@@ -246,7 +291,7 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
     __shared__ __align__(128) int4 ring[kFxStages][kFxTile * Tr::quads];
     __shared__ long long red[2][kFxWarps][NOUT][33];
     __shared__ uint64_t bars[kFxStages];
-    __shared__ int wmax[kFxWarps];
+    __shared__ int ints[2 * kFxWarps];
 
     pdl_wait();
     if (a.skip != nullptr && *a.skip != 0) return;
@@ -272,11 +317,10 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
         for (; issued < kFxStages && issued < ntiles; ++issued) request(issued);
     if (kInline) {
         FxPacking<KIND> p;
-        p.e = kFxNoLoad;
+        p.e = p.f = p.t = kFxNoLoad;
         const int i = j_begin + tid;
         if (i < j_end) p = fx_read_source<KIND>(a.xs, a.fs, i, a.K);
-        const int E = fx_block_max<kFxWarps>(p.e, wmax);
-        if (i < j_end) fx_write_record<KIND>(p, E, a.K, ring[0] + tid * Tr::quads);
+        fx_write_records<KIND, kFxWarps>(p, i < j_end, a.K, ints, ring[0]);
         __syncthreads();
     }
 
@@ -312,7 +356,7 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
         const int j0 = j_begin + t * kFxTile, jn = min(kFxTile, j_end - j0);
         const int per = (jn + kFxWarps - 1) / kFxWarps, b = min(warp * per, jn), e = min(b + per, jn);
         const int4 *tile = ring[s];
-        const int Et = tile[3].w >> 8;
+        const int Et = tile[3].w >> 16;
         if (Et == kFxBadTile || !warp_ok) {  // the whole block
             const FxSum r = fx_sum_fp64<KIND>(a, ti, j0 + b, j0 + e);
 #pragma unroll
@@ -321,11 +365,21 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
             continue;
         }
         E = Et;
-        for (int j = b; j < e;) {
-            const int stop = min(j + kFxSettle[KIND], e);
+        // the wide sources are the tile's last
+        const int mid = KIND == kFxBB ? e : min(e, max(b, tile[3].w >> 8 & 255));
+        for (int j = b; j < mid;) {
+            const int stop = min(j + kFxSettle[KIND], mid);
 #pragma unroll 1
-            for (; j < stop; ++j) fx_pair<KIND>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc);
+            for (; j < stop; ++j)
+                fx_pair<KIND, false>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc);
             fx_settle(acc);
+        }
+        if (KIND != kFxBB) {
+#pragma unroll 1
+            for (int j = mid; j < e; ++j) {
+                fx_pair<KIND, true>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc);
+                fx_settle(acc);
+            }
         }
         if (t + 1 < ntiles && (j0 + kFxTile) % kFxBlock == 0) {  // the block's last tile
 #pragma unroll
@@ -489,7 +543,9 @@ gmi_status launch_pair_fx(const FxPairSum &s, int *launched)
     a.wait_ns = s.wait_ns;
     // a CTA packs its own sources where the packing kernel and its boundary
     // (5 us) cost more than packing each tile once per target group
-    const bool packs_itself = a.chunk <= kFxTile && (long long)groups * splits <= kFxInlinePerSm * s.sm_count;
+    // (slices of less than a tile always: their records do not cross the slice)
+    const bool packs_itself =
+        a.chunk < kFxTile || (a.chunk == kFxTile && (long long)groups * splits <= kFxInlinePerSm * s.sm_count);
     *launched = packs_itself ? 1 : 2;
     if (!packs_itself)
         GMI_CUDA_TRY(launch_chained(s.pdl != 0, pack_fn(s.kind), dim3((s.n_src + kFxBlock - 1) / kFxBlock), dim3(kFxBlock),

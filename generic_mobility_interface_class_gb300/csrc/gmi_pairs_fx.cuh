@@ -24,6 +24,23 @@
 // three-word add.  Its FP32 part enters an FP32 sum, which fx_settle adds to a
 // compensated one every kFxSettle terms.  |term| < 8, so 128 terms keep the
 // 64-bit accumulators in range; the caller folds them into FP64 by then.
+//
+// Wide sources.  A term is rounded at about 2^-55 of its operands' ranges
+// before its shift, so a product must be as large as its range to have FP64's
+// relative error.  Two things break that: a torque so much larger than the force (or
+// the reverse) that the shared exponent leaves the smaller load too few bits where
+// it decides a target's sum (T'' = 2^-k T loses k more), and a source far below its
+// block's largest load.  Such a source (fx_held) is held with an exponent for its
+// force and one for its torque, and its terms enter apart, T's with the shift 2k or
+// 3k in the term in place of T'', and integer parts shifted down beyond 24 (one
+// of the two enters times 2^-3 at most, so the low words' sum of 128 sources stays
+// below 2^64).  With the block's largest load at distance 2^10 U its own w is still above 2^-30
+// of the unit, 54 bits above the accumulators' last place.  All targets of a warp
+// meet the same source, so nothing diverges.  Worst target of two
+// groups 300 radii apart, torques only, the one group's 1e-6 of the other's: error
+// of w 3.6e-12 with one exponent, 6.8e-16 with two (FP64 formulas: 1.6e-15).  Where
+// a target's terms cancel (a lone force nearly along the separation, and its w) the
+// error is a few 2^-55 of the terms, up to five times that of the FP64 formulas.
 #pragma once
 
 #include <math.h>
@@ -34,7 +51,15 @@ namespace gmi {
 
 constexpr int kFxPosBits = 51;     // position quantum 2^-51 U
 constexpr int kFxAccBits = 24;     // a term without shift enters times 2^24
-constexpr int kFxMaxGap = 6;       // exponent gap of a source within its block
+// Exponent gap of a source within its block: with one exponent for force and
+// torque (shifts up to k = 9 for v and 18 for w stay within 24), and at all, by
+// which a source is below what rounds away.
+constexpr int kFxEvenGap[5] = {6, 0, 15, 6, 15};  // by FxKind
+constexpr int kFxMaxGap = 40;
+// A torque may exceed the force of its source by 2^kFxTorqueOver, or stay
+// below it by 2^kFxTorqueUnder, and share its exponent: 1.3 % of sources with
+// normally distributed loads are wide (8 % with 1 and 3, whose error is no smaller).
+constexpr int kFxTorqueOver = 2, kFxTorqueUnder = 3;
 constexpr int kFxFold = 128;       // terms between folds
 // Terms between fx_settle: the running FP32 parts are a quarter of the error
 // of a few hundred particles' sum; every 4 instead of 8 takes 1.3 % longer.
@@ -61,7 +86,14 @@ struct FxSource {
     long long X[3];
     fxop F[3];
     long long T[3];  // torques over U, 2^-62
-    int gap;         // the block's exponent less the source's, <= kFxMaxGap
+    int gap, tgap;   // the block's exponent less the source's, of F and (wide) of T
+};
+
+// How a source is held whose forces are below 2^f and torques (over U) below
+// 2^t (kFxNoLoad: none), in a block of exponent E: wide, or with one exponent.
+struct FxHeld {
+    int gap, tgap;
+    bool wide;
 };
 
 // One target's accumulators, in 2^(-60 - 24) of the block's unit: H 2^32 + L,
@@ -144,8 +176,30 @@ GMI_FX_HD fxsum fx_scale(fxsum s, int k)
     return s;
 }
 
+// The factors by which a term of shift s enters the accumulators, and (kWide) its
+// shift beyond them.
+struct FxEnter {
+    int m, down;
+    float f;
+};
+template <bool kWide> GMI_FX_HD FxEnter fx_enter(int s)
+{
+    FxEnter n;
+    n.down = kWide && s > kFxAccBits ? s - kFxAccBits : 0;
+    n.m = 1 << (kFxAccBits - s + n.down);
+    n.f = fx_as_float((127 + kFxAccBits - 32 - s) << 23);
+    return n;
+}
+template <bool kWide, int N> GMI_FX_HD void fx_add_term(FxAcc<N> &acc, int c, const fxsum &q, const FxEnter &n)
+{
+    const long long h = kWide ? q.h >> n.down : q.h;
+    acc.H[c] = fx_madw((int)(h >> 32), n.m, acc.H[c]);
+    acc.L[c] = fx_madw_u((unsigned)h, (unsigned)n.m, acc.L[c]);
+    acc.x[c] = fmaf(q.x, n.f, acc.x[c]);
+}
+
 // One source's contribution to one target's accumulators.
-template <int KIND, int N>
+template <int KIND, bool kWide, int N>
 GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K, FxAcc<N> &acc)
 {
     constexpr bool kTorque = KIND == kFxSS || KIND == kFxBS;  // sources carry torques
@@ -237,27 +291,31 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
             cn[c] = fx_neg(cp[c]);
         }
     if (kTorque)
-        for (int c = 0; c < 3; ++c) T[c] = fx_split(S.T[c] >> kk);
+        for (int c = 0; c < 3; ++c) T[c] = fx_split(kWide ? S.T[c] : S.T[c] >> kk);
     if (KIND == kFxSS) {
         q = fxsum{0, 0.0f};
         for (int c = 0; c < 3; ++c) fx_mac(q, e[c], T[c]);
         Br = fx_product<30>(g.Br, fx_close<30>(q.h, q.x));
     }
-    const int sv = S.gap + kk, sw = S.gap + 2 * kk;
-    const int mv = 1 << (kFxAccBits - sv), mw = 1 << (kFxAccBits - sw);
-    const float fv = fx_as_float((127 + kFxAccBits - 32 - sv) << 23);
-    const float fw = fx_as_float((127 + kFxAccBits - 32 - sw) << 23);
+    const FxEnter nv = fx_enter<kWide>(S.gap + kk), nw = fx_enter<kWide>(S.gap + 2 * kk);
+    FxEnter tv = nv, tw = nw;  // of the torque's terms
+    if (kWide) {
+        tv = fx_enter<true>(S.tgap + 2 * kk);
+        tw = fx_enter<true>(S.tgap + 3 * kk);
+    }
     for (int c = 0; c < 3; ++c) {
         const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
         q = fx_mul(g.A, S.F[c]);
         fx_mac(q, Bt, e[c]);
         if (kTorque) {
+            if (kWide) {
+                fx_add_term<true>(acc, c, q, nv);
+                q = fxsum{0, 0.0f};
+            }
             fx_mac(q, T[c1], cp[c2]);
             fx_mac(q, T[c2], cn[c1]);
         }
-        acc.H[c] = fx_madw((int)(q.h >> 32), mv, acc.H[c]);
-        acc.L[c] = fx_madw_u((unsigned)q.h, (unsigned)mv, acc.L[c]);
-        acc.x[c] = fmaf(q.x, fv, acc.x[c]);
+        fx_add_term<kWide>(acc, c, q, kTorque ? tv : nv);
     }
     if (kAngular)
         for (int c = 0; c < 3; ++c) {
@@ -265,12 +323,14 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
             q = fx_mul(S.F[c1], cp[c2]);
             fx_mac(q, S.F[c2], cn[c1]);
             if (KIND == kFxSS) {
+                if (kWide) {
+                    fx_add_term<true>(acc, o, q, nw);
+                    q = fxsum{0, 0.0f};
+                }
                 fx_mac(q, g.Ar, T[c]);
                 fx_mac(q, Br, e[c]);
             }
-            acc.H[o] = fx_madw((int)(q.h >> 32), mw, acc.H[o]);
-            acc.L[o] = fx_madw_u((unsigned)q.h, (unsigned)mw, acc.L[o]);
-            acc.x[o] = fmaf(q.x, fw, acc.x[o]);
+            fx_add_term<kWide>(acc, o, q, KIND == kFxSS ? tw : nw);
         }
 }
 
@@ -462,6 +522,18 @@ GMI_FX_HD int fx_exponent(double v, int unit_exp)
     const int be = (int)(c.u >> 52) & 2047;
     if (be == 0) return (c.u << 1) == 0 ? kFxNoLoad : -5000;
     return be == 2047 ? 5000 : be - 1022 - unit_exp;
+}
+GMI_FX_HD int fx_gap(int e, int E, int most) { return e == kFxNoLoad ? 0 : E - e < most ? E - e : most; }
+template <int KIND> GMI_FX_HD FxHeld fx_held(int f, int t, int E)
+{
+    constexpr int kEven = kFxEvenGap[KIND];
+    const int e = f > t ? f : t;
+    FxHeld h;
+    h.wide = (t != kFxNoLoad && (t > f + kFxTorqueOver || t < f - kFxTorqueUnder)) ||
+             (KIND != kFxBB && e != kFxNoLoad && E - e > kEven);
+    h.gap = fx_gap(h.wide ? f : e, E, h.wide ? kFxMaxGap : kEven);
+    h.tgap = h.wide ? fx_gap(t, E, kFxMaxGap) : h.gap;
+    return h;
 }
 // The exponent of a source is its components' largest.
 GMI_FX_HD bool fx_exponent_held(int e) { return e == kFxNoLoad || (e <= kFxMaxExp && e >= -kFxMaxExp); }

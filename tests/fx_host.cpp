@@ -17,26 +17,32 @@ static int sum(int nt, const double *xt, int ns, const double *xs, const double 
     FxConsts K;
     if (!fx_consts(KIND, as, ab, mu, &K)) return 1;
     std::vector<FxSource> src(ns);
-    std::vector<int> e(ns), E((ns + tile - 1) / tile, kFxNoLoad);
+    std::vector<char> wide(ns);
+    std::vector<int> e(ns), te(ns), E((ns + tile - 1) / tile, kFxNoLoad);
     FxOrigin origin[3];
     for (int c = 0; c < 3; ++c) origin[c] = fx_origin(xs[c], K);
     for (int j = 0; j < ns; ++j) {
         for (int c = 0; c < 3; ++c)
             if (!fx_position(xs[3 * j + c], K, origin[c], &src[j].X[c])) return 2;
-        e[j] = kFxNoLoad;
-        for (int c = 0; c < nf; ++c) e[j] = std::max(e[j], fx_exponent(f[nf * j + c], c < 3 ? 0 : K.unit_exp));
-        if (!fx_exponent_held(e[j])) return 2;
-        E[j / tile] = std::max(E[j / tile], e[j]);
+        e[j] = te[j] = kFxNoLoad;
+        for (int c = 0; c < 3; ++c) e[j] = std::max(e[j], fx_exponent(f[nf * j + c], 0));
+        for (int c = 3; c < nf; ++c) te[j] = std::max(te[j], fx_exponent(f[nf * j + c], K.unit_exp));
+        if (!fx_exponent_held(std::max(e[j], te[j]))) return 2;
+        E[j / tile] = std::max(E[j / tile], std::max(e[j], te[j]));
     }
     for (int j = 0; j < ns; ++j) {
-        src[j].gap = e[j] == kFxNoLoad ? 0 : std::min(E[j / tile] - e[j], kFxMaxGap);
-        const int used = e[j] == kFxNoLoad ? 0 : E[j / tile] - src[j].gap;
+        const int Ej = E[j / tile] == kFxNoLoad ? 0 : E[j / tile];
+        const FxHeld h = fx_held<KIND>(e[j], te[j], Ej);
+        const int used = Ej - h.gap, tused = Ej - h.tgap;
+        src[j].gap = h.gap;
+        src[j].tgap = h.tgap;
+        wide[j] = h.wide;
         for (int c = 0; c < 3; ++c) {
             long long v;
             fx_fixed(f[nf * j + c], 62 - used, &v);
             src[j].F[c] = fx_split(v);
             src[j].T[c] = 0;
-            if (torque) fx_fixed(f[nf * j + nf - 3 + c], 62 - used - K.unit_exp, &src[j].T[c]);
+            if (torque) fx_fixed(f[nf * j + nf - 3 + c], 62 - tused - K.unit_exp, &src[j].T[c]);
         }
     }
     for (int i = 0; i < nt; ++i) {
@@ -48,7 +54,10 @@ static int sum(int nt, const double *xt, int ns, const double *xs, const double 
             FxAcc<nout> acc;
             fx_clear(acc);
             for (int j = j0; j < std::min(ns, j0 + kFxFold); ++j) {
-                fx_pair<KIND>(X, src[j], K, acc);
+                if (wide[j])
+                    fx_pair<KIND, true>(X, src[j], K, acc);
+                else
+                    fx_pair<KIND, false>(X, src[j], K, acc);
                 if ((j - j0) % kFxSettle[KIND] == kFxSettle[KIND] - 1) fx_settle(acc);
             }
             fx_settle(acc);

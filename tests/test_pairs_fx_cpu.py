@@ -116,6 +116,64 @@ def test_loads_of_very_different_sizes(host, oracle_built, kind):
     assert rel_err(got, oracle_sum(oracle_built, kind, xt, xs, f, 1.0, 1.0)) < n * 2.0 ** -52
 
 
+def extended_sum(kind, xt, xs, f):
+    """The sums at radii and viscosity 1 in extended precision, and for each
+    target the sum of its terms' sizes (|coefficient| |load|, v and w)."""
+    R = np.longdouble
+    xt, xs, f = xt.astype(R), xs.astype(R), f.astype(R)
+    d = xt[:, None] - xs[None]
+    r = np.sqrt((d * d).sum(-1))
+    s = np.where(r > 0, r, R(1))
+    e = d / s[..., None]
+    F, T = f[None, :, :3], f[None, :, 3:] if f.shape[1] == 6 else np.zeros((1, len(f), 3), R)
+    k8 = 1 / (8 * R("3.14159265358979323846264338327950288"))
+    far = r > 2
+    A = np.where(far, k8 / s * (1 + 2 / (3 * s * s)), k8 * (R(4) / 3 - 3 * r / 8))
+    B = np.where(far, k8 / s * (1 - 2 / (s * s)), k8 * r / 8)
+    Ar = np.where(far, -k8 / (2 * s ** 3), k8 * (1 - 27 * r / 32 + 5 * r ** 3 / 64))
+    Br = np.where(far, 3 * k8 / (2 * s ** 3), k8 * (9 * r / 32 - 3 * r ** 3 / 64))
+    C = np.where(far, k8 / (s * s), k8 * r / 2 * (1 - 3 * r / 8))
+    A, B, Ar, Br, C = (c[..., None] for c in (A, B, Ar, Br, C))
+    cross = lambda p, q: np.cross(np.broadcast_to(p, d.shape), q)
+    dot = lambda p: (e * p).sum(-1)[..., None]
+    v = (A * F + B * dot(F) * e + C * cross(T, e)).sum(1)
+    w = (C * cross(F, e) + Ar * T + Br * dot(T) * e).sum(1)
+    size = lambda p: np.sqrt((p * p).sum(-1))[..., None]
+    v_size = ((A + B) * size(F) + C * size(T)).sum((1, 2))
+    w_size = (C * size(F) + (abs(Ar) + Br) * size(T)).sum((1, 2))
+    if kind in ("ss", "sb"):
+        return np.concatenate([v, w], 1), np.stack([v_size, w_size], 1)
+    return v, v_size[:, None]
+
+
+@pytest.mark.parametrize("distance", [30.0, 120.0, 300.0, 450.0])
+@pytest.mark.parametrize("other", [1.0, 1e-3, 1e-6, 1e-9, 0.0])
+@pytest.mark.parametrize("kind,force,torque", [("ss", 1, 1), ("ss", 0, 1), ("ss", 1, 0), ("ss", 1e-2, 1), ("ss", 1, 1e-7),
+                                               ("bb", 1, 0), ("sb", 1, 0), ("bs", 0, 1), ("bs", 1e-2, 1), ("bs", 1, 1)])
+def test_every_target_of_uneven_loads(host, kind, force, torque, other, distance):
+    """Each target's error, however small its velocity: a group of particles,
+    and a distant one whose loads are `other` times as large.
+
+    Tolerance: a term (force and torque apart) is rounded at about 2^-54 of its size,
+    a sum of sums once more at 2^-53 of its own, so a few times that of the
+    sum of the terms' sizes; 2^-51 of it is allowed."""
+    rng = np.random.default_rng(int(distance) + 17)
+    xs = rng.uniform(-15.0, 15.0, size=(180, 3))
+    xs[0] = 0.0
+    xs[90:, 0] += distance
+    xt = xs if kind in ("ss", "bb") else xs + rng.normal(size=xs.shape)
+    f = rng.normal(size=(180, 6)) * np.repeat([force, torque], 3)
+    f[90:] *= other
+    if kind in ("bb", "sb"):
+        f = f[:, :3].copy()
+    status, got = fx_sum(host, kind, xt, xs, f, 1.0, 1.0)
+    assert status == 0
+    want, size = extended_sum(kind, xt, xs, f)
+    for b in range(size.shape[1]):
+        error = np.sqrt(((got[:, 3 * b:3 * b + 3] - want[:, 3 * b:3 * b + 3]) ** 2).sum(1))
+        assert (error <= 2.0 ** -51 * size[:, b]).all(), float((error[size[:, b] > 0] / size[size[:, b] > 0, b]).max())
+
+
 def test_translation_and_range(host, oracle_built):
     """Far from the origin the positions stay exact; a cloud too wide, loads
     too large or not finite, and radii too different are reported."""

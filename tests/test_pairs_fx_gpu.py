@@ -105,6 +105,31 @@ def test_overlapping_unequal_radii(gpu_ctx, oracle_built, a, b):
     assert rel_err(N(gpu_ctx.mbs(T(xb), T(xs), T(fs), a_seg=a, a_blob=b)), oracle_built.mbs(xb, xs, fs, a, b)) < tol(500)
 
 
+@pytest.mark.parametrize("n", [90, 700, 2300])
+@pytest.mark.parametrize("force,torque,other", [(0, 1, 1e-6), (1e-2, 1, 1), (1, 1e-7, 1e-3), (1, 1, 1e-8)])
+def test_every_target_of_uneven_loads(gpu_ctx, n, force, torque, other):
+    """As test_pairs_fx_cpu.py's test of that name: every target, with loads
+    whose forces, torques and particles differ much in size."""
+    from test_pairs_fx_cpu import extended_sum
+    rng = np.random.default_rng(n)
+    size = 1.6 * n ** (1 / 3)
+    xs, xt = (rng.uniform(-size, size, size=(m, 3)) for m in (n, 130))
+    xs[n // 3:, 1] += 260.0
+    fs = rng.normal(size=(n, 6)) * np.repeat([force, torque], 3)
+    fs[n // 3:] *= other
+    fb = fs[:, :3].copy()
+    gpu_ctx.set_precision(0)
+    few = slice(n // 3 - 20, n // 3 + 20)
+    v = torch.zeros((130, 6), dtype=torch.float64, device="cuda")
+    for kind, x, f, got in (("ss", xs[few], fs, gpu_ctx.mss(T(xs), T(fs), start=few.start, num=40)),
+                            ("sb", xt, fb, gpu_ctx.msb(T(xt), T(xs), T(fb), v)),
+                            ("bs", xt, fs, gpu_ctx.mbs(T(xt), T(xs), T(fs)))):
+        want, terms = extended_sum(kind, x, xs, f)
+        for b in range(terms.shape[1]):
+            error = np.sqrt(((N(got)[:, 3 * b:3 * b + 3] - want[:, 3 * b:3 * b + 3]) ** 2).sum(1))
+            assert (error <= 2.0 ** -51 * terms[:, b]).all(), kind
+
+
 def test_pinned_fp64_shape_keeps_its_kernel(gmi_lib, oracle_built):
     """A shape pinned in FP64 runs the FP64 kernel of that shape."""
     from generic_mobility_interface_class_gb300.mobility import Context
