@@ -1064,7 +1064,14 @@ __global__ void barrier_reduce(BarrierLaunch a, int splits)
 // the 27 cells around its own.  Cell (cx, cy, cz) of a particle's FP32 screen
 // position hashes to one of T = 2^k >= 2N buckets of kCellSlots entries, each
 // an entry's screen position and index, filled by an atomic count: no scan, no
-// scatter, and a search reads entries without a look at the particle.
+// scatter, and a search reads entries without a look at the particle.  The
+// particles that find their bucket full form a list from it: cells are as wide as
+// the largest radii need, so blobs smaller than the segments fill them (at
+// radius 0.3 beside 1 most targets met a full bucket; sending those to the
+// all-pairs kernel took 9.9 ms for 40,000 blobs and 12,800 segments, the lists
+// take 0.1 ms).  Entries per bucket at blob radius 1, 0.4 and 0.3: 16 43.1, 64.2
+// and 91.8 us, 8 43.1, 69.9 and 97.9, 4 43.1, 77.9 and 108; 8 hold a call of 16,896
+// particles to 9 MB of scratch (16: 17 MB).
 //
 // What bounds it is latency: a search is a chain of dependent L2 reads.  One
 // thread per target walked its 27 buckets in turn, and the kernel took 61 us
@@ -1077,14 +1084,16 @@ __global__ void barrier_reduce(BarrierLaunch a, int splits)
 // share a bucket, is dropped), and one thread per target and component adds
 // them in ascending j: the reference's per-target order, so each force is the
 // reference's bit for bit.  A target with more than kCellCand candidates, or
-// with a bucket that overflowed, goes to an overflow list, which a
-// warp-per-target all-pairs kernel finishes in the same order.
+// with a bucket of more than max(kCellLongest, N / 32) particles (where all N by
+// a warp are the fewer steps), goes to an overflow list, which a warp-per-target
+// all-pairs kernel finishes in the same order.
 // 16,896 particles: 69 us of kernels and three memsets -> 25 us of four kernels,
 // the search 61 -> 16; a call from Python 93 -> 38 us, 30 of them on the host.
 // ---------------------------------------------------------------------------
 constexpr int kCellTpb = 128;
 constexpr int kCellTargets = 16;       // targets per CTA
-constexpr int kCellSlots = 16;         // entries per bucket
+constexpr int kCellSlots = 8;          // entries per bucket
+constexpr int kCellLongest = 64;       // a bucket's particles up to which it is searched, at least
 constexpr int kCellCand = 40;          // candidates per target kept in shared memory
 constexpr int kCellPackTpb = 256;
 constexpr int kCellMinParticles = 8192;          // fewer particles: the all-pairs kernel
@@ -1096,8 +1105,10 @@ struct CellList {
     float *block_max;   // [ceil(N / kCellPackTpb)] largest |coordinate| of each pack CTA
     int blocks;
     unsigned *extent;   // largest |coordinate| of all, as FP32 bits
-    int *count;         // [T] particles per bucket
+    int2 *bucket;       // [T] its particles, and 1 + the first of those beyond kCellSlots (0: none)
     float4 *slot;       // [T][kCellSlots] screen position and index (as bits)
+    int *next;          // [N] 1 + the next of a bucket's particles beyond kCellSlots (0: none)
+    int longest;        // particles up to which a bucket is searched
     int *overflow;      // [1 + targets]: count, then the overflowed targets (launch-local indices)
 };
 
@@ -1133,7 +1144,7 @@ __global__ void __launch_bounds__(kCellPackTpb) cell_pack_kernel(CellList c, con
         out[i] = make_float4(rx, ry, rz, 0.f);
         m = fmaxf(fabsf(rx), fmaxf(fabsf(ry), fabsf(rz)));
     }
-    for (int b = i; b < c.T; b += gridDim.x * kCellPackTpb) c.count[b] = 0;
+    for (int b = i; b < c.T; b += gridDim.x * kCellPackTpb) c.bucket[b] = make_int2(0, 0);
     if (i == 0) {
         c.overflow[0] = 0;
         *c.extent = 0u;
@@ -1168,8 +1179,11 @@ __global__ void __launch_bounds__(kCellPackTpb) cell_insert_kernel(CellList c, c
     const float inv_h = cell_inv_width(c, __uint_as_float(mb));
     const float4 p = screen[i];
     const int b = cell_bucket(cell_coord(p.x, inv_h), cell_coord(p.y, inv_h), cell_coord(p.z, inv_h), c.T);
-    const int k = atomicAdd(c.count + b, 1);
-    if (k < kCellSlots) c.slot[(size_t)b * kCellSlots + k] = make_float4(p.x, p.y, p.z, __int_as_float(i));
+    const int k = atomicAdd(&c.bucket[b].x, 1);
+    if (k < kCellSlots)
+        c.slot[(size_t)b * kCellSlots + k] = make_float4(p.x, p.y, p.z, __int_as_float(i));
+    else
+        c.next[i] = atomicExch(&c.bucket[b].y, i + 1);
 }
 
 // The FP64 force of one accepted pair, as barrier_flush, in the two factors
@@ -1280,10 +1294,11 @@ __global__ void __launch_bounds__(kCellTpb) barrier_cell_kernel(BarrierLaunch a,
         const int3 q = cell[t];
         const int b = cell_bucket(q.x + nb % 3 - 1, q.y + nb / 3 % 3 - 1, q.z + nb / 9 - 1, c.T);
         const float4 *slots = c.slot + (size_t)b * kCellSlots;
-        const int held = __ldcg(c.count + b);
+        const int2 q2 = __ldcg(c.bucket + b);
+        const int held = q2.x;
         const float4 ahead = __ldcg(slots);  // with the count: an empty bucket's entry is not used
         if (held == 0) continue;
-        if (held > kCellSlots) {
+        if (held > c.longest) {
             atomicAdd(&n_cand[t], kCellCand + 1);
             continue;
         }
@@ -1294,12 +1309,19 @@ __global__ void __launch_bounds__(kCellTpb) barrier_cell_kernel(BarrierLaunch a,
         float c2_s, c2_b;
         barrier_cutoffs(a, tg.seg, c2_s, c2_b);
         const float4 pf = pos[t];
-        for (int k = 0; k < held; ++k) {
-            const float4 e = k == 0 ? ahead : __ldcg(slots + k);
-            const int j = __float_as_int(e.w);
-            if (!barrier_candidate(a, tg, pf, c2_s, c2_b, j, e)) continue;
+        const auto screen = [&](int j, float4 e) {
+            if (!barrier_candidate(a, tg, pf, c2_s, c2_b, j, e)) return;
             const int at = atomicAdd(&n_cand[t], 1);
             if (at < kCellCand) cand[t][at] = j;
+        };
+        for (int k = 0; k < min(held, kCellSlots); ++k) {
+            const float4 e = k == 0 ? ahead : __ldcg(slots + k);
+            screen(__float_as_int(e.w), e);
+        }
+        for (int k = kCellSlots, at = q2.y; k < held; ++k) {
+            const int j = at - 1;
+            at = __ldcg(c.next + j);
+            screen(j, a.screen[j]);
         }
     }
     __syncthreads();
@@ -1933,7 +1955,8 @@ gmi_status launch_barrier(gmi_context *ctx, const BarrierLaunch &in)
         a.partial = nullptr;
         const int blocks = (N + kCellPackTpb - 1) / kCellPackTpb;
         const auto round = [](size_t n) { return (n + 3) & ~(size_t)3; };
-        const size_t words = 4 * (size_t)T * kCellSlots + (size_t)T + round(blocks) + 4 + 1 + (size_t)ntg;
+        const size_t words =
+            4 * (size_t)T * kCellSlots + 2 * (size_t)T + round(N) + round(blocks) + 4 + 1 + (size_t)ntg;
         st = ctx->cells.reserve(words * sizeof(int));
         if (st != GMI_OK) return st;
         CellList c{};
@@ -1942,9 +1965,11 @@ gmi_status launch_barrier(gmi_context *ctx, const BarrierLaunch &in)
         c.extent = a.extent;
         c.blocks = blocks;
         c.slot = static_cast<float4 *>(ctx->cells.ptr);
-        c.count = reinterpret_cast<int *>(c.slot + (size_t)T * kCellSlots);
-        c.block_max = reinterpret_cast<float *>(c.count + T);
-        c.overflow = c.count + T + round(blocks);
+        c.bucket = reinterpret_cast<int2 *>(c.slot + (size_t)T * kCellSlots);
+        c.next = reinterpret_cast<int *>(c.bucket + T);
+        c.block_max = reinterpret_cast<float *>(c.next + round(N));
+        c.overflow = c.next + round(N) + round(blocks);
+        c.longest = std::max(kCellLongest, N / 32);
         cell_pack_kernel<<<blocks, kCellPackTpb, 0, ctx->stream>>>(c, a.xs, a.S, a.xb, a.B, a.screen);
         GMI_CUDA_TRY(launch_chained(true, cell_insert_kernel, dim3(blocks), dim3(kCellPackTpb), ctx->stream, c, a.screen,
                                     N));

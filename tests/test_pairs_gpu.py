@@ -128,6 +128,45 @@ def test_barrier_cell_overflow_against_oracle(gpu_ctx, oracle_built, monkeypatch
     assert np.abs(want_b[-64:]).max() > 0
 
 
+@pytest.mark.parametrize("rblob,ball", [(0.35, 0), (0.25, 0), (0.1, 0), (0.3, 3000)])
+def test_barrier_of_small_blobs_against_oracle(gpu_ctx, oracle_built, monkeypatch, rblob, ball):
+    """Cells as wide as the segments' reach hold many small blobs, more than
+    a bucket's entries; and a ball of blobs in one cell, more than are searched."""
+    rpy = oracle_built
+    monkeypatch.setenv("GMI_BARRIER_CELLS", "1")
+    xs, xb = _swimmer_cloud(3000, 60, 20, 34.2 * rblob, seed=21)
+    rng = np.random.default_rng(22)
+    if ball:
+        xb = np.concatenate([xb, rng.uniform(-0.5, 0.5, size=(ball, 3)) + np.array([0.0, 0.0, 80.0])])
+    fs = rng.normal(size=(len(xs), 6))
+    want_s, want_b = rpy.barrier(xs, xb, fs, 20, 1.0, rblob, 1.5)
+    assert np.count_nonzero(want_b.any(1)) > 20
+    got = T(fs)
+    fb = gpu_ctx.barrier(T(xs), T(xb), got, 20, 1.0, rblob, 1.5)
+    assert rel_err(N(got), want_s) < 1e-14
+    assert rel_err(N(fb), want_b) < 1e-14
+
+
+def test_barrier_of_small_blobs_keeps_the_cell_list(gpu_ctx):
+    """40,000 blobs of radius 0.3 beside 1200 segments of radius 1: the call's
+    time against that with blobs of radius 1, as dense on their sphere.  Most
+    targets by the all-pairs kernel took 200 times as long, all by their
+    cells 2 to 4 times; 20 is allowed."""
+    def microseconds(rblob):
+        xs, xb = _swimmer_cloud(40000, 60, 20, 125.0 * rblob, seed=23)
+        xs, xb, f = T(xs), T(xb), T(np.zeros((len(xs), 6)))
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        times = []
+        for _ in range(5):
+            start.record()
+            gpu_ctx.barrier(xs, xb, f, 20, 1.0, rblob, 1.0)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(1e3 * start.elapsed_time(end))
+        return min(times)
+    assert microseconds(0.3) < 20 * microseconds(1.0)
+
+
 @pytest.mark.parametrize("case", WALL)
 def test_wall_barrier_cell_list(case, gpu_ctx, monkeypatch):
     monkeypatch.setenv("GMI_BARRIER_CELLS", "1")
