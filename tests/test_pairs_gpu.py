@@ -167,6 +167,28 @@ def test_barrier_of_small_blobs_keeps_the_cell_list(gpu_ctx):
     assert microseconds(0.3) < 20 * microseconds(1.0)
 
 
+def test_barrier_overflow_fills_the_gpu(gpu_ctx, monkeypatch):
+    """Every target with more candidates than the cell kernel keeps: the
+    overflow kernel evaluates the same pairs as the all-pairs kernel, so it takes
+    about as long (1.2 times; 7 times when its CTAs share a few SMs)."""
+    rng = np.random.default_rng(24)
+    xs, xb = T(rng.uniform(-1.0, 1.0, size=(20000, 3))), T(np.zeros((0, 3)))
+    f = T(np.zeros((20000, 6)))
+    best = {}
+    for cells in "10":
+        monkeypatch.setenv("GMI_BARRIER_CELLS", cells)
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        times = []
+        for _ in range(3):
+            start.record()
+            gpu_ctx.barrier(xs, xb, f, 20)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        best[cells] = min(times)
+    assert best["1"] < 3 * best["0"], best
+
+
 @pytest.mark.parametrize("case", WALL)
 def test_wall_barrier_cell_list(case, gpu_ctx, monkeypatch):
     monkeypatch.setenv("GMI_BARRIER_CELLS", "1")
