@@ -258,8 +258,11 @@ gmi_status gmi_autotune(gmi_context *ctx, int kind, int num_targets, int num_sou
     GMI_ARG_CHECK(num_targets > 0 && num_sources > 0, "gmi_autotune: sizes must be positive");
     gmi_status st = select_device(ctx);
     if (st != GMI_OK) return st;
-    if (ctx->precision == GMI_FP64) {
-        // one kernel a kind, which sizes its own splits: nothing to time
+    // FP64: the fixed-point and the wall kernel size their own splits, so there
+    // is nothing to time for them, but segments and blobs may have radii that
+    // the fixed-point formats do not hold, and the FP64 kernels then
+    const bool fp64 = ctx->precision == GMI_FP64;
+    if (fp64 && kind != kSB && kind != kBS) {
         PairShape fx;
         fx.tt = 1;
         fx.packed = 0;
@@ -311,6 +314,7 @@ gmi_status gmi_autotune(gmi_context *ctx, int kind, int num_targets, int num_sou
     PairConsts k;
     fill_consts(k, 1.0, 1.0, 1.0, 1.0);
     st = autotune_pair(ctx, kind, rt.ptr, num_targets, rs.ptr, num_sources, k, static_cast<double *>(out.ptr));
+    if (st == GMI_OK && fp64) ctx->tuned[TuneKey{kind, ctx->precision, num_targets, num_sources}].fx = true;
     cudaStreamSynchronize(ctx->stream);
     xt.release();
     xsrc.release();

@@ -50,7 +50,8 @@ struct PairShape {
     int tt = 2;        // targets per thread
     int splits = 0;    // source splits; 0 = choose from the SM count
     int packed = -1;   // two sources per thread step (FP32, no wall): 1 yes, 0 no, -1 where available
-    bool fx = false;   // FP64: the fixed-point or the wall kernel, which choose their own splits
+    bool fx = false;   // FP64, not pinned: the fixed-point or the wall kernel, which choose their own splits; the
+                       // shape is for radii that they do not hold (kSB and kBS)
 };
 
 enum PairKind : int { kSS = 0, kSSWall = 1, kBB = 2, kSB = 3, kBS = 4 };

@@ -1776,7 +1776,8 @@ gmi_status launch_pair(gmi_context *ctx, int kind, const void *tgt_rec, int tgt_
         shape = *force_shape;
     } else {
         auto it = ctx->tuned.find(TuneKey{kind, ctx->precision, n_tgt, n_src});
-        if (it != ctx->tuned.end()) {
+        // (the autotuner's mark for the fixed-point sums within one set is no shape)
+        if (it != ctx->tuned.end() && !(it->second.fx && kind != kSB && kind != kBS)) {
             shape = it->second;
         } else if (n_src <= kWarpMaxSources) {
             shape = PairShape{kWarpShapeTpb, 2, 0};  // few sources: warp per two targets

@@ -162,8 +162,9 @@ GMI_API gmi_status gmi_barrier_forces(gmi_context *ctx, double *f_segs_d, double
 
 /* Autotuner: time the candidate launch shapes of one pair kernel for the
  * given sizes on the context's GPU and keep the fastest for later calls.
- * In FP64 there is one kernel a kind, which sizes its own splits: the call
- * only drops a pinned shape.
+ * In FP64 the usual kernels size their own splits: the call drops a pinned
+ * shape, and for kinds 3 and 4 tunes the kernel that takes radii more than a
+ * factor of two apart.
  * kind: 0 = ss, 1 = ss wall, 2 = bb, 3 = sb, 4 = bs. */
 GMI_API gmi_status gmi_autotune(gmi_context *ctx, int kind, int num_targets, int num_sources);
 /* The launch shape the context will use for this kernel and size:

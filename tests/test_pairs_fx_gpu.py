@@ -143,3 +143,24 @@ def test_pinned_fp64_shape_keeps_its_kernel(gmi_lib, oracle_built):
         ctx.autotune(0, 700, 700)
         assert ctx.tuned_shape(0, 700, 700)[3]
         np.testing.assert_array_equal(N(ctx.mss(T(xs), T(fs))), auto)
+
+
+def test_autotuned_fp64_outside_the_formats(gmi_lib, oracle_built):
+    """Radii that the formats do not hold after a call to the autotuner: the
+    FP64 kernel that it found (a few hundred sources: the warp kernel, seven
+    times faster than the tiled ones), or the same as without the call."""
+    from generic_mobility_interface_class_gb300.mobility import Context
+    xs, fs = cloud(300, 14)
+    xb, fb = cloud(280, 15)
+    with Context(0) as ctx, Context(0) as plain:
+        ctx.autotune(0, 300, 300)
+        tiny = 1e-70
+        np.testing.assert_array_equal(N(ctx.mss(T(xs), T(fs), a=tiny)), N(plain.mss(T(xs), T(fs), a=tiny)))
+        ctx.autotune(3, 300, 280)
+        ctx.autotune(4, 280, 300)
+        assert ctx.tuned_shape(3, 300, 280)[0] == 32 and ctx.tuned_shape(4, 280, 300)[0] == 32
+        for b in (0.3, 1.0):
+            got = [N(c.mbs(T(xb), T(xs), T(fs), a_blob=b)) for c in (ctx, plain)]
+            assert rel_err(got[0], oracle_built.mbs(xb, xs, fs, 1.0, b)) < tol(300)
+            if b == 1.0:
+                np.testing.assert_array_equal(*got)
