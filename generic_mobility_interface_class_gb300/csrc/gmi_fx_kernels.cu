@@ -46,7 +46,6 @@ namespace gmi {
 static_assert((int)kFxSS == (int)kSS && (int)kFxBB == (int)kBB && (int)kFxSB == (int)kSB && (int)kFxBS == (int)kBS,
               "FxKind follows PairKind");
 
-constexpr int kFxTile = 128;   // sources per tile: one stage
 constexpr int kFxBlock = 512;  // sources per block: one exponent, one fold
 constexpr int kFxTpb = 128;    // four warps
 constexpr int kFxWarps = kFxTpb / 32;
@@ -472,26 +471,6 @@ static FxPackFn pack_fn(int kind)
 {
     return kind == kSS ? fx_pack_kernel<kFxSS> : kind == kBB ? fx_pack_kernel<kFxBB>
          : kind == kSB ? fx_pack_kernel<kFxSB> : fx_pack_kernel<kFxBS>;
-}
-
-// Sources per split, a power of two.  Measured on M_ss and M_bb of 200 to
-// 12,800 particles (152 SMs): with work enough, the largest split that still
-// gives 24 CTAs per SM, so that the last CTAs to finish idle the chip for
-// little of the launch (4096 segments: 128 sources 325 us, 1024 403; 12,800:
-// 1024 sources 2.82 ms, 128 2.87, 2048 2.84); below that a tile, down to 1.5
-// CTAs per SM (1669 segments: 128 72 us, 64 78, 32 82); then parts of a tile,
-// whose CTAs have less to do than to set up (642: 32 20.6 us, 64 24.7, 128
-// 30.8), and 16 or 8 while the CTAs still find an SM each (60: 8 12.4 us, 16
-// 14.4, 32 16.5; 320: 32 17.7 us, 16 and 8 16.5).
-static int fx_chunk(int groups, int n_src, int sm_count, int most_splits)
-{
-    const auto splits = [&](long long chunk) { return ((long long)n_src + chunk - 1) / chunk; };
-    const auto ctas = [&](long long chunk) { return (double)groups * (double)splits(chunk) / sm_count; };
-    long long chunk = kFxTile;
-    while (ctas(2 * chunk) >= 24.0) chunk *= 2;
-    if (ctas(kFxTile) < 1.5) chunk = ctas(64) >= 2.0 ? 64 : ctas(8) <= 0.5 ? 8 : ctas(16) <= 1.0 ? 16 : 32;
-    while (splits(chunk) > std::min(most_splits, 65535)) chunk *= 2;
-    return (int)std::min<long long>(chunk, 1 << 30);
 }
 
 int fx_splits(int n_tgt, int n_src, int sm_count)

@@ -49,6 +49,7 @@
 
 namespace gmi {
 
+constexpr int kFxTile = 128;       // sources per tile of the pair kernel: one stage
 constexpr int kFxPosBits = 51;     // position quantum 2^-51 U
 constexpr int kFxAccBits = 24;     // a term without shift enters times 2^24
 // Exponent gap of a source within its block: with one exponent for force and
@@ -537,5 +538,25 @@ template <int KIND> GMI_FX_HD FxHeld fx_held(int f, int t, int E)
 }
 // The exponent of a source is its components' largest.
 GMI_FX_HD bool fx_exponent_held(int e) { return e == kFxNoLoad || (e <= kFxMaxExp && e >= -kFxMaxExp); }
+
+// Sources per split, a power of two.  Measured on M_ss and M_bb of 200 to
+// 12,800 particles (152 SMs): with work enough, the largest split that still
+// gives 24 CTAs per SM, so that the last CTAs to finish idle the chip for
+// little of the launch (4096 segments: 128 sources 325 us, 1024 403; 12,800:
+// 1024 sources 2.82 ms, 128 2.87, 2048 2.84); below that a tile, down to 1.5
+// CTAs per SM (1669 segments: 128 72 us, 64 78, 32 82); then parts of a tile,
+// whose CTAs have less to do than to set up (642: 32 20.6 us, 64 24.7, 128
+// 30.8), and 16 or 8 while the CTAs still find an SM each (60: 8 12.4 us, 16
+// 14.4, 32 16.5; 320: 32 17.7 us, 16 and 8 16.5).
+inline int fx_chunk(int groups, int n_src, int sm_count, int most_splits)
+{
+    const auto splits = [&](long long chunk) { return ((long long)n_src + chunk - 1) / chunk; };
+    const auto ctas = [&](long long chunk) { return (double)groups * (double)splits(chunk) / sm_count; };
+    long long chunk = kFxTile;
+    while (chunk < n_src && ctas(2 * chunk) >= 24.0) chunk *= 2;
+    if (ctas(kFxTile) < 1.5) chunk = ctas(64) >= 2.0 ? 64 : ctas(8) <= 0.5 ? 8 : ctas(16) <= 1.0 ? 16 : 32;
+    while (splits(chunk) > (most_splits < 65535 ? most_splits : 65535)) chunk *= 2;
+    return (int)(chunk < 1 << 30 ? chunk : 1 << 30);
+}
 
 }  // namespace gmi

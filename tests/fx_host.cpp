@@ -81,3 +81,4 @@ extern "C" int fx_host_sum(int kind, int nt, const double *xt, int ns, const dou
 
 extern "C" int fx_host_fixed(double v, int s, long long *r) { return fx_fixed(v, s, r) ? 1 : 0; }
 extern "C" double fx_host_value(long long a, long long b, int E) { return fx_value(FxTotal{a, b}, E, 1.0, 0.0); }
+extern "C" int fx_host_chunk(int groups, int n_src, int sm_count, int most) { return fx_chunk(groups, n_src, sm_count, most); }

@@ -214,3 +214,14 @@ def test_conversions_round_once(host):
     for a, b in sums:
         for e in (0, 84, -37):
             assert host.fx_host_value(a, b, e) == float(Fraction(a * 2 ** 32 + b) * Fraction(2) ** (e - 84))
+
+
+def test_split_rule_over_all_sizes(host):
+    """Sources per split: a power of two from 8, no larger than it takes to
+    hold all of them, and no more splits than allowed."""
+    for groups in (1, 3, 40, 400, 3647, 3648, 4000, 100000, 60000000):
+        for n in (1, 7, 128, 5000, 131072, 2000000):
+            for most in (1, 5, 1 << 20):
+                chunk = host.fx_host_chunk(groups, n, 152, most)
+                assert 8 <= chunk < max(2 * n, 256) and chunk & (chunk - 1) == 0, (groups, n, most)
+                assert -(-n // chunk) <= most

@@ -108,26 +108,40 @@ def test_overlapping_unequal_radii(gpu_ctx, oracle_built, a, b):
 @pytest.mark.parametrize("n", [90, 700, 2300])
 @pytest.mark.parametrize("force,torque,other", [(0, 1, 1e-6), (1e-2, 1, 1), (1, 1e-7, 1e-3), (1, 1, 1e-8)])
 def test_every_target_of_uneven_loads(gpu_ctx, n, force, torque, other):
-    """As test_pairs_fx_cpu.py's test of that name: every target, with loads
-    whose forces, torques and particles differ much in size."""
+    """As test_pairs_fx_cpu.py's test of that name, with loads whose forces,
+    torques and particles differ much in size: 40 of the targets, of sums
+    whose CTAs pack their own sources and (2300) of sums with a pack kernel."""
     from test_pairs_fx_cpu import extended_sum
     rng = np.random.default_rng(n)
     size = 1.6 * n ** (1 / 3)
-    xs, xt = (rng.uniform(-size, size, size=(m, 3)) for m in (n, 130))
+    xs, xt = (rng.uniform(-size, size, size=(n, 3)) for _ in range(2))
     xs[n // 3:, 1] += 260.0
+    xt[n // 3:, 1] += 260.0
     fs = rng.normal(size=(n, 6)) * np.repeat([force, torque], 3)
     fs[n // 3:] *= other
     fb = fs[:, :3].copy()
     gpu_ctx.set_precision(0)
     few = slice(n // 3 - 20, n // 3 + 20)
-    v = torch.zeros((130, 6), dtype=torch.float64, device="cuda")
-    for kind, x, f, got in (("ss", xs[few], fs, gpu_ctx.mss(T(xs), T(fs), start=few.start, num=40)),
+    v = torch.zeros((n, 6), dtype=torch.float64, device="cuda")
+    for kind, x, f, got in (("ss", xs, fs, gpu_ctx.mss(T(xs), T(fs))),
                             ("sb", xt, fb, gpu_ctx.msb(T(xt), T(xs), T(fb), v)),
                             ("bs", xt, fs, gpu_ctx.mbs(T(xt), T(xs), T(fs)))):
-        want, terms = extended_sum(kind, x, xs, f)
+        want, terms = extended_sum(kind, x[few], xs, f)
+        got = N(got)[few]
         for b in range(terms.shape[1]):
-            error = np.sqrt(((N(got)[:, 3 * b:3 * b + 3] - want[:, 3 * b:3 * b + 3]) ** 2).sum(1))
+            error = np.sqrt(((got[:, 3 * b:3 * b + 3] - want[:, 3 * b:3 * b + 3]) ** 2).sum(1))
             assert (error <= 2.0 ** -51 * terms[:, b]).all(), kind
+
+
+def test_targets_that_fill_the_gpu_many_times(gpu_ctx, oracle_built):
+    """More targets than 24 CTAs per SM take: one slice of the sources."""
+    rng = np.random.default_rng(16)
+    xt, xs = rng.uniform(-60.0, 60.0, size=(150_000, 3)), rng.uniform(-60.0, 60.0, size=(300, 3))
+    fs = rng.normal(size=(300, 6))
+    gpu_ctx.set_precision(0)
+    got = N(gpu_ctx.mbs(T(xt), T(xs), T(fs)))
+    rows = rng.integers(0, len(xt), 400)
+    assert rel_err(got[rows], oracle_built.mbs(xt[rows], xs, fs, 1.0, 1.0)) < tol(300)
 
 
 def test_pinned_fp64_shape_keeps_its_kernel(gmi_lib, oracle_built):
