@@ -515,7 +515,7 @@ gmi_status launch_pair_fx(const FxPairSum &s, int *launched)
     a.n_tgt = s.n_tgt;
     a.n_src = s.n_src;
     a.out = s.out;
-    a.partial = splits > 1 ? s.partial : nullptr;
+    a.partial = splits > 1 || s.staged ? s.partial : nullptr;
     a.accumulate = s.accumulate;
     a.err = s.err;
     a.skip = s.skip;
@@ -533,7 +533,7 @@ gmi_status launch_pair_fx(const FxPairSum &s, int *launched)
                                 dim3(groups, splits), dim3(kFxTpb), s.stream, a));
     if (s.splits_out) {
         *s.splits_out = splits;
-    } else if (splits > 1) {
+    } else if (a.partial != nullptr) {
         // a kernel of its own: the last CTA of a target group adding the
         // group's partials took 2 us longer (320 segments: 18.5, 16.4 us)
         const int count = s.n_tgt * nout;

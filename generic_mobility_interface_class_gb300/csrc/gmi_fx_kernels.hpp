@@ -28,6 +28,8 @@ struct FxPairSum {
     int pdl;                       // the first kernel too may start while the previous one on the stream ends
     unsigned long long wait_ns;
     int max_splits;                // 0: no cap beyond the automatic choice
+    bool staged;                   // out overlaps an input: it is written by a last kernel, from `partial` (one
+                                   // split's place at least)
 };
 
 // Whether the formats hold this kind's radii (gmi_pairs_fx.cuh).

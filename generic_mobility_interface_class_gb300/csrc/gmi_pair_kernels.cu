@@ -1850,6 +1850,12 @@ gmi_status launch_pair(gmi_context *ctx, int kind, const void *tgt_rec, int tgt_
     return GMI_OK;
 }
 
+static bool overlap(const double *a, size_t na, const double *b, size_t nb)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb * sizeof(double) && y < x + na * sizeof(double);
+}
+
 // One pair sum of positions and loads in the reference's layouts, by the
 // kernel of the context's precision.  FP64 takes the wall kernel or, without a
 // wall, the fixed-point kernel, at every size: against the FP64 kernels M_ss of 320
@@ -1868,7 +1874,13 @@ gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt,
         // (30 us each)
         const int splits = wall ? wall_splits(n_tgt, n_src, ctx->sm_count) : fx_splits(n_tgt, n_src, ctx->sm_count);
         const size_t records = wall ? 0 : ((size_t)n_src * fx_record_bytes(kind) + 255) / 256 * 256;
-        const size_t partial = splits > 1 ? (size_t)splits * n_tgt * nout_of(kind) * sizeof(double) : 0;
+        // CTAs still read positions and loads when the first of them write
+        // sums: where these overlap, a last kernel writes
+        const int nout = nout_of(kind);
+        const bool in_place = overlap(out, (size_t)n_tgt * nout, xt, (size_t)n_all_tgt * 3) ||
+                              overlap(out, (size_t)n_tgt * nout, xs, (size_t)n_src * 3) ||
+                              overlap(out, (size_t)n_tgt * nout, fs, (size_t)n_src * (kind == kBB || kind == kSB ? 3 : 6));
+        const size_t partial = splits > 1 || in_place ? (size_t)splits * n_tgt * nout * sizeof(double) : 0;
         GMI_TRY(ctx->fx.reserve(records + partial));
         unsigned char *mem = static_cast<unsigned char *>(ctx->fx.ptr);
         int launched = 0;
@@ -1880,13 +1892,14 @@ gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt,
             s.n_tgt = n_tgt;
             s.n_src = n_src;
             s.out = out;
-            s.partial = reinterpret_cast<double *>(mem);
+            s.partial = partial > 0 ? reinterpret_cast<double *>(mem) : nullptr;
             const gmi_status st = launch_wall_fp64(ctx->stream, ctx->sm_count, s, &launched);
             ctx->launches += launched;
             return st;
         }
         FxPairSum s{};
         s.max_splits = splits;
+        s.staged = in_place;
         s.partial_bytes = partial;
         s.rec = mem;
         s.partial = reinterpret_cast<double *>(mem + records);

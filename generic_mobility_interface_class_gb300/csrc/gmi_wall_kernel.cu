@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kWallTpb) rpy_wall_kernel(const WallSum a, int
     for (int o = tid; o < nt * 6; o += kWallTpb) {
         const int i = o / 6, c = o - 6 * i;
         const double t = (red[0][c][i] + red[1][c][i]) + (red[2][c][i] + red[3][c][i]);
-        if (gridDim.y > 1)
+        if (a.partial != nullptr)
             a.partial[blockIdx.y * count + base + o] = t;
         else
             a.out[base + o] = t;
@@ -185,7 +185,7 @@ gmi_status launch_wall_fp64(cudaStream_t stream, int sm_count, const WallSum &a,
     rpy_wall_kernel<<<dim3((a.n_tgt + 31) / 32, splits), kWallTpb, 0, stream>>>(a, chunk);
     GMI_CUDA_TRY(cudaGetLastError());
     *launched = 1;
-    if (splits > 1) {
+    if (a.partial != nullptr) {
         const int count = a.n_tgt * 6;
         GMI_CUDA_TRY(launch_chained(true, reduce_splits_tree, dim3((count + 63) / 64), dim3(64), stream, a.partial, splits,
                                     count, a.out, 0));

@@ -11,7 +11,8 @@ struct WallSum {
     const double *x, *f;  // AoS positions and loads (6 values)
     int tgt_start, n_tgt, n_src;
     double *out;
-    double *partial;  // wall_splits() * 6 n_tgt values when there are several splits
+    double *partial;  // wall_splits() * 6 n_tgt values when there are several splits, or when out overlaps an
+                      // input (a last kernel then writes out); else null
 };
 
 int wall_splits(int n_tgt, int n_src, int sm_count);

@@ -144,6 +144,27 @@ def test_targets_that_fill_the_gpu_many_times(gpu_ctx, oracle_built):
     assert rel_err(got[rows], oracle_built.mbs(xt[rows], xs, fs, 1.0, 1.0)) < tol(300)
 
 
+@pytest.mark.parametrize("ns,nt", [(8, 3000), (300, 2000)])
+def test_sums_into_their_inputs(gpu_ctx, ns, nt):
+    """Velocities that overwrite positions or loads: as with arrays apart, also
+    where one split of the sources would let a CTA write at once (8)."""
+    rng = np.random.default_rng(18)
+    xs, fs, xt = T(rng.uniform(-9, 9, (ns, 3))), T(rng.normal(size=(ns, 6))), T(rng.uniform(-30, 30, (nt, 3)))
+    gpu_ctx.set_precision(0)
+    want = N(gpu_ctx.mbs(xt, xs, fs)) + 0.0
+    x = xt.clone()
+    np.testing.assert_array_equal(N(gpu_ctx.mbs(x, xs, fs, out=x)), want)
+    v = torch.zeros((nt, 3), dtype=torch.float64, device="cuda")
+    loads = v.view(-1)[-6 * ns:].view(ns, 6)
+    loads.copy_(fs)
+    np.testing.assert_array_equal(N(gpu_ctx.mbs(xt, xs, loads, out=v)), want)
+    f = fs.clone()
+    np.testing.assert_array_equal(N(gpu_ctx.mss(xs, f, out=f)), N(gpu_ctx.mss(xs, fs)))
+    f = fs.clone()
+    x = xs + torch.tensor([0.0, 0.0, 12.0], dtype=torch.float64, device="cuda")
+    np.testing.assert_array_equal(N(gpu_ctx.mss_wall(x, f, out=f)), N(gpu_ctx.mss_wall(x, fs)))
+
+
 def test_pinned_fp64_shape_keeps_its_kernel(gmi_lib, oracle_built):
     """A shape pinned in FP64 runs the FP64 kernel of that shape."""
     from generic_mobility_interface_class_gb300.mobility import Context
