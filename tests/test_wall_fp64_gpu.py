@@ -31,3 +31,19 @@ def test_wall_sizes_against_oracle(gpu_ctx, oracle_built, n):
     if n > 300:  # a slice of the targets, not on a group's edge
         got = gpu_ctx.mss_wall(T(x), T(f), start=37, num=211).cpu().numpy()
         assert rel_err(got, want[37:248]) < 2.0 ** -44
+
+
+def test_wall_separations_whose_square_overflows(gpu_ctx, oracle_built):
+    """Finite velocities, as from 1 / inf = 0; a position that is not finite still
+    makes every target NaN."""
+    rng = np.random.default_rng(2)
+    x = rng.uniform(0.0, 9.0, size=(40, 3)) + np.array([0.0, 0.0, 1.05])
+    f = rng.normal(size=(40, 6))
+    x[17, 0] = 1e170
+    gpu_ctx.set_precision(0)
+    want = oracle_built.mss_wall(x, f)
+    assert np.isfinite(want).all()
+    assert rel_err(gpu_ctx.mss_wall(T(x), T(f)).cpu().numpy(), want) < 2.0 ** -44
+    for bad in (np.nan, np.inf):
+        x[17, 0] = bad
+        assert not np.isfinite(gpu_ctx.mss_wall(T(x), T(f)).cpu().numpy()[:, :3]).any()
