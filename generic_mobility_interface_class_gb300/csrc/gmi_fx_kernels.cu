@@ -366,17 +366,30 @@ __global__ void __launch_bounds__(kFxTpb, kFxCtas<KIND>) rpy_fx_kernel(const __g
         E = Et;
         // the wide sources are the tile's last
         const int mid = KIND == kFxBB ? e : min(e, max(b, tile[3].w >> 8 & 255));
+        unsigned close = 0;  // of the warp's sources, those close to the lane's target
         for (int j = b; j < mid;) {
             const int stop = min(j + kFxSettle[KIND], mid);
 #pragma unroll 1
             for (; j < stop; ++j)
-                fx_pair<KIND, false>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc);
+                fx_pair<KIND, false>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc, close, 1u << (j - b));
             fx_settle(acc);
         }
         if (KIND != kFxBB) {
 #pragma unroll 1
             for (int j = mid; j < e; ++j) {
-                fx_pair<KIND, true>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc);
+                fx_pair<KIND, true>(X, fx_load_source<KIND>(tile + j * Tr::quads), a.K, acc, close, 1u << (j - b));
+                fx_settle(acc);
+            }
+        }
+        if constexpr (KIND == kFxSS) {
+#pragma unroll 1
+            for (; close != 0; close &= close - 1) {
+                const int j = b + __ffs(close) - 1;
+                const FxSource src = fx_load_source<KIND>(tile + j * Tr::quads);
+                if (j < mid)
+                    fx_close_cross<false>(X, src, a.K, acc);
+                else
+                    fx_close_cross<true>(X, src, a.K, acc);
                 fx_settle(acc);
             }
         }

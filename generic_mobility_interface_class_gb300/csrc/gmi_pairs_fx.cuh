@@ -33,8 +33,8 @@
 // block's largest load.  Such a source (fx_held) is held with an exponent for its
 // force and one for its torque, and its terms enter apart, T's with the shift 2k or
 // 3k in the term in place of T'', and integer parts shifted down beyond 24 (one
-// of the two enters times 2^-3 at most, so the low words' sum of 128 sources stays
-// below 2^64).  With the block's largest load at distance 2^10 U its own w is still above 2^-30
+// of the two enters times 2^-3 at most, a close pair's cross products times 2^-1, so
+// the low words' sum of 128 sources stays below 2^64).  With the block's largest load at distance 2^10 U its own w is still above 2^-30
 // of the unit, 54 bits above the accumulators' last place.  All targets of a warp
 // meet the same source, so nothing diverges.  Worst target of two
 // groups 300 radii apart, torques only, the one group's 1e-6 of the other's: error
@@ -133,12 +133,13 @@ struct FxScalars {
     fxop A, B, C, Ar, Br;
 };
 
-// Near-field scalars of the segment kinds in FP64 (few pairs get here), at r = ru U.
+// Near-field scalars of the segment kinds in FP64 (few pairs get here), at r = ru U;
+// C times `up`.
 template <int KIND>
 #ifdef __CUDACC__
 __host__ __device__ __noinline__
 #endif
-FxScalars fx_near_scalars(double ru, const FxConsts &K)
+FxScalars fx_near_scalars(double ru, double up, const FxConsts &K)
 {
     const fxop none{0, 0.0f, 0.0f};
     FxScalars s;
@@ -148,7 +149,7 @@ FxScalars fx_near_scalars(double ru, const FxConsts &K)
         s.B = fx_from_double(K.a0 * 3.0 * q);
         s.Ar = fx_from_double(K.ar0 * (1.0 - 27.0 * q + (5.0 / 64.0) * rho3));
         s.Br = fx_from_double(K.ar0 * (9.0 * q - (3.0 / 64.0) * rho3));
-        s.C = fx_from_double(0.5 * K.ar0 * ru * (1.0 - 12.0 * q));
+        s.C = fx_from_double(0.5 * K.ar0 * ru * (1.0 - 12.0 * q) * up);
         return s;
     }
     s.Ar = s.Br = none;
@@ -159,11 +160,11 @@ FxScalars fx_near_scalars(double ru, const FxConsts &K)
         const double p = K.ab * K.ab + 2.0 * K.ab * (r + K.as) - 3.0 * (K.as - r) * (K.as - r);
         s.A = fx_from_double(K.a0 * (0.5 * (K.as + K.ab) - t * t * i3));
         s.B = fx_from_double(K.a0 * 3.0 * b * b * i3);
-        s.C = fx_from_double(K.unit * K.unit * u * u * p / (16.0 * K.ab * K.as * K.as * K.as * r2d));
+        s.C = fx_from_double(K.unit * K.unit * u * u * p / (16.0 * K.ab * K.as * K.as * K.as * r2d) * up);
     } else {
         s.A = K.a_zero;
         s.B = none;
-        s.C = K.as > K.ab ? fx_from_double(K.unit * K.unit * r / (K.as * K.as * K.as)) : none;
+        s.C = K.as > K.ab ? fx_from_double(K.unit * K.unit * r / (K.as * K.as * K.as) * up) : none;
     }
     return s;
 }
@@ -193,15 +194,97 @@ template <bool kWide> GMI_FX_HD FxEnter fx_enter(int s)
 }
 template <bool kWide, int N> GMI_FX_HD void fx_add_term(FxAcc<N> &acc, int c, const fxsum &q, const FxEnter &n)
 {
-    const long long h = kWide ? q.h >> n.down : q.h;
+    const long long h = kWide ? q.h >> (n.down < 63 ? n.down : 63) : q.h;
     acc.H[c] = fx_madw((int)(h >> 32), n.m, acc.H[c]);
     acc.L[c] = fx_madw_u((unsigned)h, (unsigned)n.m, acc.L[c]);
     acc.x[c] = fmaf(q.x, n.f, acc.x[c]);
 }
 
-// One source's contribution to one target's accumulators.
+// The separation of a target and a source, as fx_pair has it in place: d' (scale 29),
+// r'^2 (58), 1/r' (30), and k.
+struct FxSeparation {
+    fxop d[3], ir;
+    fxsum s;
+    int k;
+    bool zero;
+};
+GMI_FX_HD FxSeparation fx_separation(const long long *X, const FxSource &S)
+{
+    FxSeparation p;
+    long long D[3] = {X[0] - S.X[0], X[1] - S.X[1], X[2] - S.X[2]};  // |D| < 2^61
+    int m;
+    {
+        const int h0 = (int)(D[0] >> 32), h1 = (int)(D[1] >> 32), h2 = (int)(D[2] >> 32);
+        const int a0 = h0 ^ (h0 >> 31), a1 = h1 ^ (h1 >> 31), a2 = h2 ^ (h2 >> 31);
+        m = a0 > a1 ? a0 : a1;
+        m = m > a2 ? m : a2;
+    }
+    int sl;
+    p.zero = false;
+    if (m == 0) {  // closer than 2^-19 U: the leading bit is in the low words
+        unsigned long long mx = 0;
+        for (int c = 0; c < 3; ++c) {
+            const unsigned long long a = (unsigned long long)(D[c] < 0 ? -D[c] : D[c]);
+            mx = a > mx ? a : mx;
+        }
+        p.zero = mx == 0;
+        if (p.zero) D[0] = 1;
+        sl = p.zero ? 61 : fx_clzll(mx) - 2;
+    } else {
+        sl = fx_clz((unsigned)m) - 2;  // the leading bit moves to 2^61 (one place off for a negative power of two)
+    }
+    p.k = 61 - kFxPosBits - sl;
+    for (int c = 0; c < 3; ++c) p.d[c] = fx_split((long long)((unsigned long long)D[c] << sl));  // scale 29
+    p.s = fxsum{0, 0.0f};
+    for (int c = 0; c < 3; ++c) {
+        p.s.h = fx_madw(p.d[c].h, p.d[c].h, p.s.h);
+        p.s.x = fmaf(p.d[c].hf, p.d[c].lf, p.s.x);
+    }
+    p.s.x *= 2.0f;
+    p.ir = fx_rsqrt(p.s.h, p.s.x);
+    return p;
+}
+
+// r / U in FP64
+GMI_FX_HD double fx_distance(const fxsum &s, const fxop &ir, int k)
+{
+    const double ird = ((double)ir.h + (double)ir.lf * (1.0 / 4294967296.0)) * (1.0 / 1073741824.0);
+    const double r2 = ((double)s.h + (double)s.x * (1.0 / 4294967296.0)) * (1.0 / 288230376151711744.0);
+    return r2 * ird * fx_exp2(k);
+}
+
+// The cross products' terms of a pair closer than about U / 2 (k < -1), with C times
+// 2^up, up = -k - 1 (so below 2: C <= r / U), and the shift up in the term: C vanishes
+// with r, and these terms can be all of a target's sum (two segments 1e-4 radii apart, torques alone: error of v
+// 3e-12 with C at the others' scale, 3e-16 so).
 template <int KIND, bool kWide, int N>
-GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K, FxAcc<N> &acc)
+GMI_FX_HD void fx_cross_terms(const fxop *e, const fxop &C, int up, const FxSource &S, FxAcc<N> &acc)
+{
+    const FxEnter nv = fx_enter<true>((kWide ? S.tgap : S.gap) + up), nw = fx_enter<true>(S.gap + up);
+    fxop cp[3];
+    for (int c = 0; c < 3; ++c) cp[c] = fx_product<30>(e[c], C);
+    for (int c = 0; c < 3; ++c) {
+        const int c1 = (c + 1) % 3, c2 = (c + 2) % 3, o = N == 6 ? 3 + c : c;
+        if (KIND == kFxSS || KIND == kFxBS) {
+            fxsum q = fx_mul(fx_split(S.T[c1]), cp[c2]);
+            fx_mac(q, fx_split(S.T[c2]), fx_neg(cp[c1]));
+            fx_add_term<true>(acc, c, q, nv);
+        }
+        if (KIND == kFxSS || KIND == kFxSB) {
+            fxsum q = fx_mul(S.F[c1], cp[c2]);
+            fx_mac(q, S.F[c2], fx_neg(cp[c1]));
+            fx_add_term<true>(acc, o, q, nw);
+        }
+    }
+}
+
+// One source's contribution to one target's accumulators.  M_ss leaves out the cross
+// products of a close pair and sets `bit` in `close` (fx_close_cross adds them in a
+// loop of its own: in this function they cost it 2 % of its time; the other kinds
+// lose 1 % by such a loop and 0.1 % by a branch here).
+template <int KIND, bool kWide, int N>
+GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K, FxAcc<N> &acc, unsigned &close,
+                       unsigned bit)
 {
     constexpr bool kTorque = KIND == kFxSS || KIND == kFxBS;  // sources carry torques
     constexpr bool kAngular = KIND == kFxSS || KIND == kFxSB; // targets turn
@@ -275,9 +358,15 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
             g.B = fx_close<31>(u.h, u.x);
             g.A = fx_add(K.a_zero, -3, g.B);
         } else {
-            const double ird = ((double)ir.h + (double)ir.lf * (1.0 / 4294967296.0)) * (1.0 / 1073741824.0);
-            const double r2 = ((double)s.h + (double)s.x * (1.0 / 4294967296.0)) * (1.0 / 288230376151711744.0);
-            g = fx_near_scalars<KIND>(r2 * ird * fx_exp2(k), K);
+            const int up = KIND == kFxSS || k >= -1 ? 0 : -k - 1;
+            g = fx_near_scalars<KIND>(fx_distance(s, ir, k), fx_exp2(up), K);
+            if (k < -1) {
+                if (KIND == kFxSS)
+                    close |= bit;
+                else
+                    fx_cross_terms<KIND, kWide>(e, g.C, up, S, acc);
+                g.C = fxop{0, 0.0f, 0.0f};
+            }
         }
     }
 
@@ -333,6 +422,17 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
             }
             fx_add_term<kWide>(acc, o, q, KIND == kFxSS ? tw : nw);
         }
+}
+
+// The cross products of a close pair of segments that fx_pair marked.
+template <bool kWide, int N>
+GMI_FX_HD void fx_close_cross(const long long *X, const FxSource &S, const FxConsts &K, FxAcc<N> &acc)
+{
+    const FxSeparation p = fx_separation(X, S);
+    fxop e[3];
+    for (int c = 0; c < 3; ++c) e[c] = fx_product<29>(p.d[c], p.ir);
+    const fxop C = fx_near_scalars<kFxSS>(fx_distance(p.s, p.ir, p.k), fx_exp2(-p.k - 1), K).C;
+    fx_cross_terms<kFxSS, kWide>(e, C, -p.k - 1, S, acc);
 }
 
 template <int N> GMI_FX_HD void fx_clear(FxAcc<N> &a)

@@ -54,10 +54,17 @@ static int sum(int nt, const double *xt, int ns, const double *xs, const double 
             FxAcc<nout> acc;
             fx_clear(acc);
             for (int j = j0; j < std::min(ns, j0 + kFxFold); ++j) {
+                unsigned close = 0;
                 if (wide[j])
-                    fx_pair<KIND, true>(X, src[j], K, acc);
+                    fx_pair<KIND, true>(X, src[j], K, acc, close, 1);
                 else
-                    fx_pair<KIND, false>(X, src[j], K, acc);
+                    fx_pair<KIND, false>(X, src[j], K, acc, close, 1);
+                if constexpr (KIND == kFxSS) {
+                    if (close != 0 && wide[j])
+                        fx_close_cross<true>(X, src[j], K, acc);
+                    else if (close != 0)
+                        fx_close_cross<false>(X, src[j], K, acc);
+                }
                 if ((j - j0) % kFxSettle[KIND] == kFxSettle[KIND] - 1) fx_settle(acc);
             }
             fx_settle(acc);

@@ -174,6 +174,28 @@ def test_every_target_of_uneven_loads(host, kind, force, torque, other, distance
         assert (error <= 2.0 ** -51 * size[:, b]).all(), float((error[size[:, b] > 0] / size[size[:, b] > 0, b]).max())
 
 
+@pytest.mark.parametrize("distance", [1.0, 0.1, 1e-2, 1e-4, 1e-7])
+@pytest.mark.parametrize("kind,force,torque", [("ss", 0, 1), ("ss", 1, 0), ("ss", 1, 1e-9), ("ss", 1, 1), ("bb", 1, 0)])
+def test_every_target_of_close_pairs(host, kind, force, torque, distance):
+    """Three particles that overlap almost wholly, so that the cross products, which
+    vanish with the distance, are all that torques give to v and forces to w.
+
+    Tolerance: as test_every_target_of_uneven_loads, and the positions are
+    multiples of the formats' quantum there."""
+    rng = np.random.default_rng(19)
+    for _ in range(20):
+        x = 3.3 + distance * rng.normal(size=(3, 3))
+        x = np.rint(np.ldexp(x, 51)) * 2.0 ** -51
+        f = rng.normal(size=(3, 6)) * np.repeat([force, torque], 3)
+        f = f if kind == "ss" else f[:, :3].copy()
+        status, got = fx_sum(host, kind, x, x, f, 1.0, 1.0)
+        assert status == 0
+        want, size = extended_sum(kind, x, x, f)
+        for b in range(size.shape[1]):
+            error = np.sqrt(((got[:, 3 * b:3 * b + 3] - want[:, 3 * b:3 * b + 3]) ** 2).sum(1))
+            assert (error <= 2.0 ** -51 * size[:, b]).all(), float((error / size[:, b]).max())
+
+
 def test_translation_and_range(host, oracle_built):
     """Far from the origin the positions stay exact; a cloud too wide, loads
     too large or not finite, and radii too different are reported."""
