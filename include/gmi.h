@@ -8,7 +8,9 @@
  * exits the process.  Device pointers are marked _d; host pointers _h.
  *
  * Precision: GMI_FP64 evaluates the pair sums to FP64 accuracy (the wall in
- * FP64 like the reference, the free-space sums in 64-bit fixed point);
+ * FP64 like the reference, the free-space sums in 64-bit fixed point, each
+ * target's error within 2^-51 of its terms' sizes; positions are held to
+ * 2^-52 of the smaller radius);
  * GMI_FP32C evaluates them in FP32 with double-float source positions and
  * compensated (two-sum) accumulation, and returns FP64 results; GMI_DF64
  * (blob-blob only) carries every step of the pair formula as a double-float
