@@ -78,7 +78,9 @@ struct UnequalCoeffs {
 static __device__ __noinline__ UnequalCoeffs unequal_near2(float r2, float ir, float dF, UnequalK<float> k)
 {
     UnequalCoeffs c;
-    unequal_coeffs<float>(r2, ir, dF, k, c.A, c.Bd, c.Cd);
+    // coincident (r^2 is kTinyR2 then) or as good as that in FP32: the formula's
+    // 1/r^3 would overflow between equal radii
+    unequal_coeffs<float>(r2 < 1e-24f ? 0.0f : r2, ir, dF, k, c.A, c.Bd, c.Cd);
     const float u = 1.0f / k.f8pm;
     c.A *= u; c.Bd *= u; c.Cd *= u;
     return c;

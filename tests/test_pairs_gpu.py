@@ -167,6 +167,20 @@ def test_barrier_of_small_blobs_keeps_the_cell_list(gpu_ctx):
     assert microseconds(0.3) < 20 * microseconds(1.0)
 
 
+def test_coincident_segments_and_blobs_in_fp32(gpu_ctx, oracle_built):
+    """Blobs in the places of segments, of the same radius: finite velocities from
+    the packed kernel (2600 particles), as accurate as the others."""
+    rng = np.random.default_rng(25)
+    xs = rng.uniform(-20.0, 20.0, size=(2600, 3))
+    xb = np.concatenate([xs[::3], rng.uniform(-20.0, 20.0, size=(1800, 3))])
+    fs, fb = rng.normal(size=(2600, 6)), rng.normal(size=(len(xb), 3))
+    gpu_ctx.set_precision(1)
+    v = np.zeros((2600, 6))
+    assert rel_err(N(gpu_ctx.msb(T(xs), T(xb), T(fb), T(v))), oracle_built.msb(xs, xb, fb, 1.0, 1.0)) < 2e-6
+    assert rel_err(N(gpu_ctx.mbs(T(xb), T(xs), T(fs))), oracle_built.mbs(xb, xs, fs, 1.0, 1.0)) < 2e-6
+    gpu_ctx.set_precision(0)
+
+
 def test_barrier_overflow_fills_the_gpu(gpu_ctx, monkeypatch):
     """Every target with more candidates than the cell kernel keeps: the
     overflow kernel evaluates the same pairs as the all-pairs kernel, so it takes
