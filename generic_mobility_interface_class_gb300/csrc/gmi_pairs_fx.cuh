@@ -33,7 +33,7 @@
 // block's largest load.  Such a source (fx_held) is held with an exponent for its
 // force and one for its torque, and its terms enter apart, T's with the shift 2k or
 // 3k in the term in place of T'', and integer parts shifted down beyond 24 (one
-// of the two enters times 2^-3 at most, a close pair's cross products times 2^-1, so
+// of the two enters times 2^-3 at most, a near pair's cross products times 2^-1, so
 // the low words' sum of 128 sources stays below 2^64).  With the block's largest load at distance 2^10 U its own w is still above 2^-30
 // of the unit, 54 bits above the accumulators' last place.  All targets of a warp
 // meet the same source, so nothing diverges.  Worst target of two
@@ -75,11 +75,13 @@ struct FxConsts {
     double pos_scale, unit;    // 2^51 / U, U
     double vscale, vfix;       // 1/(8 pi mu U), and what its rounding leaves out
     double wscale, wfix;       // 1/(8 pi mu U^2)
-    double as, ab, inv_as;     // radii (equal kinds: both the one radius)
+    double as, ab;             // radii (equal kinds: both the one radius)
     double a0, ar0;            // near field: 4U/(3a) (unequal: 4U/(3 as ab)), (U/a)^3
+    int turn;                  // Ar and Br of the near field carry 2^turn, with which (U/a)^3 exceeds 1/2
+    double ar0_turn;           // (U/a)^3 2^turn
     fxop k3;                   // far field: (as^2 + ab^2) / (3 U^2)
     unsigned long long t4;     // near up to r^2 = t4 U^2 (2^-58): (as + ab)^2 < 36 U^2, so more than 63 bits
-    fxop a_zero, ar_zero;      // at r = 0: A = 4U / (3 max(as, ab)), Ar = (U/a)^3
+    fxop a_zero, ar_zero;      // at r = 0: A = 4U / (3 max(as, ab)), Ar = (U/a)^3 2^turn
     fxop bb_b;                 // blob-blob near field: (U/a)^2, an eighth of it at scale 33
 };
 
@@ -131,25 +133,39 @@ GMI_FX_HD double fx_exp2(int e)  // 2^e, -1022 <= e <= 1023
 // of T'', Br of (e'.T'') e'.
 struct FxScalars {
     fxop A, B, C, Ar, Br;
+    int up;  // near field: C carries 2^up
 };
 
-// Near-field scalars of the segment kinds in FP64 (few pairs get here), at r = ru U;
-// C times `up`.
+// C times 2^up, up >= 1, in [1/2, 1): C is below 0.4 (largest at 4/3 of the radius), and
+// vanishes with r and next to r = ab - as.
+GMI_FX_HD void fx_normalised(double C, FxScalars &s)
+{
+    union {
+        double d;
+        unsigned long long u;
+    } c;
+    c.d = C;
+    const int up = 1022 - ((int)(c.u >> 52) & 2047);
+    s.up = up < 1 ? 1 : up > 64 ? 64 : up;
+    s.C = fx_from_double(C * fx_exp2(s.up));
+}
+
+// Near-field scalars of the segment kinds in FP64 (few pairs get here), at r = ru U.
 template <int KIND>
 #ifdef __CUDACC__
 __host__ __device__ __noinline__
 #endif
-FxScalars fx_near_scalars(double ru, double up, const FxConsts &K)
+FxScalars fx_near_scalars(double ru, const FxConsts &K)
 {
     const fxop none{0, 0.0f, 0.0f};
     FxScalars s;
     if (KIND == kFxSS) {
-        const double rho = ru * K.unit * K.inv_as, q = rho * (1.0 / 32.0), rho3 = rho * rho * rho;
+        const double rho = ru * K.unit / K.as, q = rho * (1.0 / 32.0), rho3 = rho * rho * rho;
         s.A = fx_from_double(K.a0 - K.a0 * 9.0 * q);
         s.B = fx_from_double(K.a0 * 3.0 * q);
-        s.Ar = fx_from_double(K.ar0 * (1.0 - 27.0 * q + (5.0 / 64.0) * rho3));
-        s.Br = fx_from_double(K.ar0 * (9.0 * q - (3.0 / 64.0) * rho3));
-        s.C = fx_from_double(0.5 * K.ar0 * ru * (1.0 - 12.0 * q) * up);
+        s.Ar = fx_from_double(K.ar0_turn * fma(5.0 / 64.0, rho3, fma(-27.0, q, 1.0)));
+        s.Br = fx_from_double(K.ar0_turn * fma(-3.0 / 64.0, rho3, 9.0 * q));
+        fx_normalised(0.5 * K.ar0 * ru * (1.0 - 12.0 * q), s);
         return s;
     }
     s.Ar = s.Br = none;
@@ -160,11 +176,11 @@ FxScalars fx_near_scalars(double ru, double up, const FxConsts &K)
         const double p = K.ab * K.ab + 2.0 * K.ab * (r + K.as) - 3.0 * (K.as - r) * (K.as - r);
         s.A = fx_from_double(K.a0 * (0.5 * (K.as + K.ab) - t * t * i3));
         s.B = fx_from_double(K.a0 * 3.0 * b * b * i3);
-        s.C = fx_from_double(K.unit * K.unit * u * u * p / (16.0 * K.ab * K.as * K.as * K.as * r2d) * up);
+        fx_normalised(K.unit * K.unit * u * u * p / (16.0 * K.ab * K.as * K.as * K.as * r2d), s);
     } else {
         s.A = K.a_zero;
         s.B = none;
-        s.C = K.as > K.ab ? fx_from_double(K.unit * K.unit * r / (K.as * K.as * K.as) * up) : none;
+        fx_normalised(K.as > K.ab ? K.unit * K.unit * r / (K.as * K.as * K.as) : 0.0, s);
     }
     return s;
 }
@@ -253,10 +269,10 @@ GMI_FX_HD double fx_distance(const fxsum &s, const fxop &ir, int k)
     return r2 * ird * fx_exp2(k);
 }
 
-// The cross products' terms of a pair closer than about U / 2 (k < -1), with C times
-// 2^up, up = -k - 1 (so below 2: C <= r / U), and the shift up in the term: C vanishes
-// with r, and these terms can be all of a target's sum (two segments 1e-4 radii apart, torques alone: error of v
-// 3e-12 with C at the others' scale, 3e-16 so).
+// The cross products' terms of a near pair, with C times 2^up and the shift up in the
+// term: C can be small, and these terms can be all of a target's sum (two
+// segments 1e-4 radii apart, torques alone: error of v 3e-12 with C at the others'
+// scale, 3e-16 so).
 template <int KIND, bool kWide, int N>
 GMI_FX_HD void fx_cross_terms(const fxop *e, const fxop &C, int up, const FxSource &S, FxAcc<N> &acc)
 {
@@ -279,7 +295,7 @@ GMI_FX_HD void fx_cross_terms(const fxop *e, const fxop &C, int up, const FxSour
 }
 
 // One source's contribution to one target's accumulators.  M_ss leaves out the cross
-// products of a close pair and sets `bit` in `close` (fx_close_cross adds them in a
+// products of a near pair and sets `bit` in `close` (fx_close_cross adds them in a
 // loop of its own: in this function they cost it 2 % of its time; the other kinds
 // lose 1 % by such a loop and 0.1 % by a branch here).
 template <int KIND, bool kWide, int N>
@@ -327,7 +343,7 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
     for (int c = 0; c < 3; ++c) e[c] = fx_product<29>(d[c], ir);
 
     FxScalars g;  // far field
-    int kk = k;
+    int kk = k, kw = 2 * k;
     {
         const fxop ir2 = fx_close<30>(fx_madw(ir.h, ir.h, 0), 2.0f * (ir.hf * ir.lf));
         const fxsum u = fx_mul(K.k3, ir2);  // 28 + 30
@@ -345,6 +361,7 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
     }
     if (near) {
         kk = 0;
+        kw = KIND == kFxSS ? K.turn : 0;
         if (zero) {  // r -> 0
             g.A = K.a_zero;
             g.B = g.Br = g.C = fxop{0, 0.0f, 0.0f};
@@ -358,15 +375,12 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
             g.B = fx_close<31>(u.h, u.x);
             g.A = fx_add(K.a_zero, -3, g.B);
         } else {
-            const int up = KIND == kFxSS || k >= -1 ? 0 : -k - 1;
-            g = fx_near_scalars<KIND>(fx_distance(s, ir, k), fx_exp2(up), K);
-            if (k < -1) {
-                if (KIND == kFxSS)
-                    close |= bit;
-                else
-                    fx_cross_terms<KIND, kWide>(e, g.C, up, S, acc);
-                g.C = fxop{0, 0.0f, 0.0f};
-            }
+            g = fx_near_scalars<KIND>(fx_distance(s, ir, k), K);
+            if (KIND == kFxSS)
+                close |= bit;
+            else
+                fx_cross_terms<KIND, kWide>(e, g.C, g.up, S, acc);
+            g.C = fxop{0, 0.0f, 0.0f};
         }
     }
 
@@ -387,11 +401,11 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
         for (int c = 0; c < 3; ++c) fx_mac(q, e[c], T[c]);
         Br = fx_product<30>(g.Br, fx_close<30>(q.h, q.x));
     }
-    const FxEnter nv = fx_enter<kWide>(S.gap + kk), nw = fx_enter<kWide>(S.gap + 2 * kk);
+    const FxEnter nv = fx_enter<kWide>(S.gap + kk), nw = fx_enter<kWide>(S.gap + kw);
     FxEnter tv = nv, tw = nw;  // of the torque's terms
     if (kWide) {
         tv = fx_enter<true>(S.tgap + 2 * kk);
-        tw = fx_enter<true>(S.tgap + 3 * kk);
+        tw = fx_enter<true>(S.tgap + kk + kw);
     }
     for (int c = 0; c < 3; ++c) {
         const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
@@ -424,15 +438,15 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
         }
 }
 
-// The cross products of a close pair of segments that fx_pair marked.
+// The cross products of a near pair of segments that fx_pair marked.
 template <bool kWide, int N>
 GMI_FX_HD void fx_close_cross(const long long *X, const FxSource &S, const FxConsts &K, FxAcc<N> &acc)
 {
     const FxSeparation p = fx_separation(X, S);
     fxop e[3];
     for (int c = 0; c < 3; ++c) e[c] = fx_product<29>(p.d[c], p.ir);
-    const fxop C = fx_near_scalars<kFxSS>(fx_distance(p.s, p.ir, p.k), fx_exp2(-p.k - 1), K).C;
-    fx_cross_terms<kFxSS, kWide>(e, C, -p.k - 1, S, acc);
+    const FxScalars g = fx_near_scalars<kFxSS>(fx_distance(p.s, p.ir, p.k), K);
+    fx_cross_terms<kFxSS, kWide>(e, g.C, g.up, S, acc);
 }
 
 template <int N> GMI_FX_HD void fx_clear(FxAcc<N> &a)
@@ -539,16 +553,22 @@ inline bool fx_consts(int kind, double as, double ab, double mu, FxConsts *K)
     K->wfix = K->wscale * fix;
     K->as = as;
     K->ab = ab;
-    K->inv_as = 1.0 / as;
     K->a0 = equal ? 4.0 * U / (3.0 * as) : 4.0 * U / (3.0 * as * ab);
-    K->ar0 = (U / as) * (U / as) * (U / as);
+    // (U/a)^3 in two parts: all rotation of near pairs and a target's own shares its error
+    const double a2 = as * as, a3c = a2 * as, a3_low = fma(a2, as, -a3c) + fma(as, as, -a2) * as, U3 = U * U * U;
+    const double q3 = U3 / a3c, q3_low = (fma(-q3, a3c, U3) - q3 * a3_low) / a3c;
+    K->ar0 = q3 + q3_low;
+    K->turn = 0;
+    while (equal && ldexp(K->ar0, K->turn) <= 0.5) ++K->turn;
+    K->ar0_turn = ldexp(K->ar0, K->turn);
     K->k3 = fx_split(fx_rint((as * as + ab * ab) / (3.0 * U * U) * 1152921504606846976.0));  // 28
     K->t4 = (unsigned long long)((as + ab) * (as + ab) / (U * U) * 288230376151711744.0);  // a whole number
     // the self term is the largest of most sums: the quotient's remainder too
     const double a3 = 3.0 * amax, a_zero = 4.0 * U / a3;
     K->a_zero = fx_from_double(a_zero);
     K->a_zero.lf += (float)((fma(-a_zero, a3, 4.0 * U) - a_zero * fma(3.0, amax, -a3)) / a3 * 4611686018427387904.0);
-    K->ar_zero = fx_from_double(K->ar0);
+    K->ar_zero = fx_from_double(ldexp(q3, K->turn));
+    K->ar_zero.lf += (float)(ldexp(q3_low, K->turn) * 4611686018427387904.0);
     K->bb_b = fx_from_double(U * U / (as * as));
     return true;
 }

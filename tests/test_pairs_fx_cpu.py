@@ -196,6 +196,47 @@ def test_every_target_of_close_pairs(host, kind, force, torque, distance):
             assert (error <= 2.0 ** -51 * size[:, b]).all(), float((error / size[:, b]).max())
 
 
+@pytest.mark.parametrize("size", [1.0, 2.5, 8.0])
+@pytest.mark.parametrize("radius", [1.0, 1.4, 1.99])
+@pytest.mark.parametrize("force,torque", [(0, 1), (1, 0), (1, 1)])
+def test_overlapping_segments_of_any_radius(host, radius, force, torque, size):
+    """Radii over the octave that shares a unit: near it the near-field
+    scalars are as small as an eighth of their range.
+
+    Tolerance, in the 2-norm over all targets: the FP64 formulas' own error is 4e-16
+    to 6e-16 here (200 terms); 2^-51 is allowed."""
+    rng = np.random.default_rng(20)
+    xs = radius * rng.uniform(-size, size, size=(200, 3)) + 3.3
+    f = rng.normal(size=(200, 6)) * np.repeat([force, torque], 3)
+    status, got = fx_sum(host, "ss", xs, xs, f, radius, radius)
+    assert status == 0
+    a = np.longdouble(radius)
+    scaled = f.astype(np.longdouble) / np.repeat([a / a, a], 3)
+    want, _ = extended_sum("ss", xs.astype(np.longdouble) / a, xs.astype(np.longdouble) / a, scaled)
+    want /= np.repeat([a, a * a], 3)
+    for b in (0, 3):
+        error, norm = ((v ** 2).sum() for v in (got[:, b:b + 3] - want[:, b:b + 3], want[:, b:b + 3]))
+        assert error <= (2.0 ** -51) ** 2 * norm, float(np.sqrt(error / norm))
+
+
+@pytest.mark.parametrize("kind", ["sb", "bs"])
+@pytest.mark.parametrize("a,b", [(1.96, 3.9), (3.9, 1.96), (1.0, 1.9), (1.9, 1.0)])
+def test_cross_products_of_overlapping_unequal_radii(host, oracle_built, kind, a, b):
+    """The angular velocities from forces, and the velocities from torques, of
+    overlapping segments and blobs, against the FP64 oracle, whose sums of 300
+    terms differ from the exact ones by about 1e-15 in the 2-norm."""
+    rng = np.random.default_rng(26)
+    xt, xs = (min(a, b) * rng.uniform(-1.0, 1.0, size=(n, 3)) + 3.3 for n in (200, 300))
+    f = rng.normal(size=(300, 6 if kind == "bs" else 3))
+    if kind == "bs":
+        f[:, :3] = 0.0
+    status, got = fx_sum(host, kind, xt, xs, f, a, b)
+    assert status == 0
+    want = oracle_sum(oracle_built, kind, xt, xs, f, a, b)
+    error = (got - want)[:, -3:]
+    assert np.linalg.norm(error) < 2.0 ** -49 * np.linalg.norm(want[:, -3:])
+
+
 def test_translation_and_range(host, oracle_built):
     """Far from the origin the positions stay exact; a cloud too wide, loads
     too large or not finite, and radii too different are reported."""
