@@ -28,12 +28,13 @@ constexpr int kWallTile = 128;  // sources staged at a time
 
 // 1/sqrt(x): the hardware estimate y (measured within 2^-20) and the
 // binomial series of (1 - e)^(-1/2), e = 1 - x y^2, to e^2: the next term,
-// 5/16 e^3, is below 2^-58.  A square that overflows counts as the largest number
-// (by an integer instruction): particles that far apart do not reach each
-// other, while 0 in place of y would make e a NaN.
+// 5/16 e^3, is below 2^-58.  By integer instructions a square that overflows counts
+// as the largest number (particles that far apart do not reach each other, while
+// 0 in place of y would make e a NaN) and one below 1e-120 as that, whose powers to
+// y^5 are finite: a source without loads in a target's place adds zeros.
 __device__ __forceinline__ double wall_rsqrt(double x)
 {
-    x = __hiloint2double(min(__double2hiint(x), 0x7fefffff), __double2loint(x));
+    x = __hiloint2double(max(min(__double2hiint(x), 0x7fefffff), 0x2704a872), __double2loint(x));
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x * y, y, 1.0);

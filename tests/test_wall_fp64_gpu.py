@@ -47,3 +47,15 @@ def test_wall_separations_whose_square_overflows(gpu_ctx, oracle_built):
     for bad in (np.nan, np.inf):
         x[17, 0] = bad
         assert not np.isfinite(gpu_ctx.mss_wall(T(x), T(f)).cpu().numpy()[:, :3]).any()
+
+
+def test_wall_source_without_loads_in_a_targets_place(gpu_ctx, oracle_built):
+    """It changes nothing but its own velocity, which is its neighbour's less
+    the neighbour's own."""
+    rng = np.random.default_rng(3)
+    x = rng.uniform(0.0, 9.0, size=(60, 3)) + np.array([0.0, 0.0, 1.05])
+    f = rng.normal(size=(60, 6))
+    gpu_ctx.set_precision(0)
+    want = oracle_built.mss_wall(x, f)
+    got = gpu_ctx.mss_wall(T(np.concatenate([x, x[:1]])), T(np.concatenate([f, np.zeros((1, 6))])), num=60)
+    assert rel_err(got.cpu().numpy(), want) < 2.0 ** -44
