@@ -21,19 +21,19 @@
 // FP64 kernel executed 65 FP64 instructions at 76 cycles each.  Integer limbs
 // alone (530 instructions, 146 of them wide multiplies) took 1.8 cycles each.
 // FP64 kernel -> integer limbs -> limb and FP32 (this one):
-//   12,800 segments                  20.4 -> 3.90 -> 2.81 ms  (5.1 TFLOP/s at 87 flop a pair)
+//   12,800 segments                  20.4 -> 3.90 -> 2.86 ms  (5.0 TFLOP/s at 87 flop a pair)
 //   4096 blobs                       1223 -> 229 -> 178 us
 //   12,800 segments, 4096 blobs,
-//   both ways                        9.72 -> 1.80 -> 1.36 ms
+//   both ways                        9.72 -> 1.80 -> 1.38 ms
 // Nothing outside the pair loop runs in FP64 (76 cycles an instruction, 95 a
 // conversion): positions and loads become integers, and sums FP64 numbers, by
 // integer instructions.  With FP64 there, 642 segments took 28.6 us (now 20.5),
 // 962 41.0 (34.8), 1669 blobs 55.3 (45.1), a solve of 962 particles 4.25 ms (3.80).
 // A sum of wide sources only (gmi_pairs_fx.cuh), such as torques without forces,
-// takes 18 % longer in M_ss and 9 % in M_bs and M_sb; with loads alike none or 1 %.
-// Error against extended precision (2-norm, mean of four draws), FP64 kernel ->
-// this: 60 to 700 segments 0.81 to 0.96 of it, 1500 segments 2.9e-16 -> 1.9e-16;
-// 50 to 1200 blobs 0.65 to 0.95; segments on blobs and back 0.82 to 1.05.
+// takes 22 % longer in M_ss and 9 % in M_bs and M_sb.
+// Error against extended precision (2-norm, mean of four draws) as a part of the FP64
+// kernels': 60 to 1500 segments 0.56 to 0.99, torques alone 0.47 to 0.92; 50 to 1200
+// blobs 0.59 to 0.86; segments on blobs and back 0.64 to 0.89 (radii 0.75 to 1.3).
 #include <algorithm>
 
 #include "gmi_fx_kernels.hpp"

@@ -1859,7 +1859,7 @@ static bool overlap(const double *a, size_t na, const double *b, size_t nb)
 // One pair sum of positions and loads in the reference's layouts, by the
 // kernel of the context's precision.  FP64 takes the wall kernel or, without a
 // wall, the fixed-point kernel, at every size: against the FP64 kernels M_ss of 320
-// segments went from 61 to 16.4 us, of 12,800 from 20.4 to 2.81 ms, M_bb of
+// segments went from 61 to 16.4 us, of 12,800 from 20.4 to 2.86 ms, M_bb of
 // 4096 blobs from 1223 to 178 us.  The FP64 kernels keep radii that the
 // fixed-point formats do not hold, and shapes pinned by gmi_set_shape.
 gmi_status pair_sum(gmi_context *ctx, int kind, const double *xt, int n_all_tgt, int tgt_start, int n_tgt,

@@ -34,13 +34,14 @@
 // force and one for its torque, and its terms enter apart, T's with the shift 2k or
 // 3k in the term in place of T'', and integer parts shifted down beyond 24 (one
 // of the two enters times 2^-3 at most, a near pair's cross products times 2^-1, so
-// the low words' sum of 128 sources stays below 2^64).  With the block's largest load at distance 2^10 U its own w is still above 2^-30
-// of the unit, 54 bits above the accumulators' last place.  All targets of a warp
-// meet the same source, so nothing diverges.  Worst target of two
-// groups 300 radii apart, torques only, the one group's 1e-6 of the other's: error
-// of w 3.6e-12 with one exponent, 6.8e-16 with two (FP64 formulas: 1.6e-15).  Where
-// a target's terms cancel (a lone force nearly along the separation, and its w) the
-// error is a few 2^-55 of the terms, up to five times that of the FP64 formulas.
+// the low words' sum of 128 sources stays below 2^64).  With the block's largest
+// load at distance 2^10 U its own w is still above 2^-30 of the unit, 54 bits above
+// the accumulators' last place.  All targets of a warp meet the same source, so
+// nothing diverges.  Worst target of two groups 300 radii apart, torques only, the
+// one group's 1e-6 of the other's: error of w 3.6e-12 with one exponent, 6.8e-16
+// with two (FP64 formulas: 1.6e-15).  Where a target's terms cancel (a lone force
+// nearly along the separation, and its w) the error is a few 2^-55 of the terms,
+// up to five times that of the FP64 formulas.
 #pragma once
 
 #include <math.h>
@@ -304,7 +305,7 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
 {
     constexpr bool kTorque = KIND == kFxSS || KIND == kFxBS;  // sources carry torques
     constexpr bool kAngular = KIND == kFxSS || KIND == kFxSB; // targets turn
-    constexpr bool kCross = kTorque || kAngular;
+    constexpr bool kCross = kTorque || kAngular, kShared = KIND == kFxSS && !kWide;
     long long D[3] = {X[0] - S.X[0], X[1] - S.X[1], X[2] - S.X[2]};  // |D| < 2^61
     int m;
     {
@@ -388,10 +389,13 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
     fxsum q{0, 0.0f};
     for (int c = 0; c < 3; ++c) fx_mac(q, e[c], S.F[c]);
     const fxop Bt = fx_product<30>(g.B, fx_close<30>(q.h, q.x));
+    // a cross product is the load's with C e, where v and w share that in the loop
+    // that counts, else C times the load's with e, which spares the rounding of C e at
+    // the scale of e: error of M_sb's w 1.03 -> 0.83 of the FP64 kernel's, no longer
     fxop T[3], cp[3], cn[3], Br;
     if (kCross)
         for (int c = 0; c < 3; ++c) {
-            cp[c] = fx_product<30>(e[c], g.C);
+            cp[c] = kShared ? fx_product<30>(e[c], g.C) : e[c];
             cn[c] = fx_neg(cp[c]);
         }
     if (kTorque)
@@ -416,8 +420,14 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
                 fx_add_term<true>(acc, c, q, nv);
                 q = fxsum{0, 0.0f};
             }
-            fx_mac(q, T[c1], cp[c2]);
-            fx_mac(q, T[c2], cn[c1]);
+            if (kShared) {
+                fx_mac(q, T[c1], cp[c2]);
+                fx_mac(q, T[c2], cn[c1]);
+            } else {
+                fxsum x = fx_mul(T[c1], cp[c2]);
+                fx_mac(x, T[c2], cn[c1]);
+                fx_mac(q, fx_close<30>(x.h, x.x), g.C);
+            }
         }
         fx_add_term<kWide>(acc, c, q, kTorque ? tv : nv);
     }
@@ -426,6 +436,7 @@ GMI_FX_HD void fx_pair(const long long *X, const FxSource &S, const FxConsts &K,
             const int c1 = (c + 1) % 3, c2 = (c + 2) % 3, o = N == 6 ? 3 + c : c;
             q = fx_mul(S.F[c1], cp[c2]);
             fx_mac(q, S.F[c2], cn[c1]);
+            if (!kShared) q = fx_mul(fx_close<30>(q.h, q.x), g.C);
             if (KIND == kFxSS) {
                 if (kWide) {
                     fx_add_term<true>(acc, o, q, nw);
