@@ -214,27 +214,97 @@ struct FxSum {
     double v[6];
 };
 
+// M_bb's near field, out of line as ss_near_coeffs: A, and B times dF
+static __device__ __noinline__ double2 fx_bb_near_fp64(double w, double f6pma, double d)
+{
+    return make_double2((1.0 - 3.0 * w) * f6pma, w * f6pma * d);
+}
+
+// A pair in FP64, far pairs in as few FP64 instructions as it takes: one factor
+// 1/(8 pi mu) on 1/r scales all coefficients, C d serves both cross products, and the
+// root is the hardware's estimate with one third-order step (gmi_wall_kernel.cu; the
+// square is held between 1e-300 and the largest number by an integer instruction, for
+// the pair at r = 0).  54 a pair in M_ss and 27 in M_bb, where pair_ss and pair_bb
+// execute 65 and 33.  A near pair only has other coefficients: a warp meets its own
+// 32 targets one lane at a time.
+template <int KIND>
+__device__ __forceinline__ void fx_pair_fp64(double dx, double dy, double dz, const double *F, const FxLaunch &a,
+                                             double f8, double q, unsigned long long near, double *v)
+{
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const double x = __hiloint2double(max(min(__double2hiint(r2), 0x7fefffff), 0x01a56e1f), __double2loint(r2));
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double h = fma(-x * y, y, 1.0), ir = fma(y * h, fma(0.375, h, 0.5), y);
+    const double dF = fma(dx, F[0], fma(dy, F[1], dz * F[2]));
+    double dT = 0.0, A, B, C, Ar = 0.0, Br = 0.0;
+    if constexpr (KIND == kFxSS) dT = fma(dx, F[3], fma(dy, F[4], dz * F[5]));
+    if ((unsigned long long)__double_as_longlong(r2) > near) {
+        const double ir2 = ir * ir, c1 = f8 * ir, c5 = c1 * ir2 * ir2;
+        C = c1 * ir2;
+        A = fma(q, C, c1);
+        B = fma(-3.0 * q, c5, C) * dF;
+        if constexpr (KIND == kFxSS) {
+            Ar = -0.5 * C;
+            Br = 1.5 * c5 * dT;
+        }
+    } else if constexpr (KIND == kFxSS) {
+        ss_near_coeffs<double>(r2, ir, dF, dT, a.eq, A, B, Ar, Br, C);
+    } else if constexpr (KIND == kFxBB) {
+        const double2 n = fx_bb_near_fp64(r2 * ir * a.eq.q32, a.eq.f6pma, ir * ir * dF);
+        A = n.x;
+        B = n.y;
+    } else {
+        unequal_coeffs<double>(r2, ir, dF, a.uq, A, B, C);
+    }
+    v[0] = fma(B, dx, fma(A, F[0], v[0]));
+    v[1] = fma(B, dy, fma(A, F[1], v[1]));
+    v[2] = fma(B, dz, fma(A, F[2], v[2]));
+    if constexpr (KIND == kFxBB) return;
+    const double cx = C * dx, cy = C * dy, cz = C * dz;
+    if constexpr (FxTraits<KIND>::torque) {
+        v[0] = fma(F[4], cz, fma(-F[5], cy, v[0]));
+        v[1] = fma(F[5], cx, fma(-F[3], cz, v[1]));
+        v[2] = fma(F[3], cy, fma(-F[4], cx, v[2]));
+    }
+    if constexpr (FxTraits<KIND>::nout == 6) {
+        v[3] = fma(F[1], cz, fma(-F[2], cy, v[3]));
+        v[4] = fma(F[2], cx, fma(-F[0], cz, v[4]));
+        v[5] = fma(F[0], cy, fma(-F[1], cx, v[5]));
+    }
+    if constexpr (KIND == kFxSS) {
+        v[3] = fma(Br, dx, fma(Ar, F[3], v[3]));
+        v[4] = fma(Br, dy, fma(Ar, F[4], v[4]));
+        v[5] = fma(Br, dz, fma(Ar, F[5], v[5]));
+    }
+}
+
 // The sources [j0, j1) on one target in FP64, for the blocks and targets that
 // the fixed-point formats do not hold.  M_bb four at a time, for the loads in
-// flight (the others gain nothing and lose 0.6 % of the sums that do fit):
-// 12,800 blobs spread over 2400 radii 13.2 -> 12.2 ms (the tiled FP64 kernel,
-// which stages them in shared memory: 12.0).
+// flight (the others gain nothing and lose 0.6 % of the sums that do fit).
+// What bounds it is the FP64 pipe, and that the splits suit the fixed-point loop: at
+// 1100 particles 315 CTAs load some SMs with three of them, where two are the mean.
+// With pair_ss and pair_bb here sets spread over 2400 radii took up to 1.28 of the
+// time of the tiled and warp FP64 kernels (now 0.5 to 0.98, but 1.17 for M_ss of 1150);
+// us, those kernels -> pair_* -> this:
+//   M_ss 300 60 -> 38 -> 35, 1100 180 -> 232 -> 195, 4000 2340 -> 1976 -> 1602
+//   M_bb 300 35 -> 23 -> 21, 1100 103 -> 131 -> 101, 4000 1222 -> 1236 -> 858
+//   M_bs 300 47 -> 25 -> 23, 1100 133 -> 146 -> 123, 4000 1571 -> 1316 -> 1104
 template <int KIND>
 static __device__ __noinline__ FxSum fx_sum_fp64(const FxLaunch &a, int ti, int j0, int j1)
 {
     FxSum s{};
     const double xi = a.xt[3 * (size_t)ti], yi = a.xt[3 * (size_t)ti + 1], zi = a.xt[3 * (size_t)ti + 2];
+    constexpr bool kOneSet = KIND == kFxSS || KIND == kFxBB;
+    const double f8 = kOneSet ? a.eq.f8pm : a.uq.f8pm, q = kOneSet ? a.eq.two_a2 * (1.0 / 3.0) : a.uq.far_c;
+    const unsigned long long near = (unsigned long long)__double_as_longlong(kOneSet ? a.eq.four_a2 : a.uq.sum2);
     constexpr int kAtOnce = KIND == kFxBB ? 4 : 1;
 #pragma unroll kAtOnce
     for (int j = j0; j < j1; ++j) {
         double F[6] = {0, 0, 0, 0, 0, 0};
         for (int c = 0; c < FxTraits<KIND>::nf; ++c) F[c] = a.fs[FxTraits<KIND>::nf * (size_t)j + c];
-        const double dx = xi - a.xs[3 * (size_t)j], dy = yi - a.xs[3 * (size_t)j + 1],
-                     dz = zi - a.xs[3 * (size_t)j + 2];
-        if constexpr (KIND == kFxSS) pair_ss<double>(dx, dy, dz, F, a.eq, s.v, s.v + 3);
-        if constexpr (KIND == kFxBB) pair_bb<double>(dx, dy, dz, F, a.eq, s.v);
-        if constexpr (KIND == kFxSB) pair_sb<double>(dx, dy, dz, F, a.uq, s.v, s.v + 3);
-        if constexpr (KIND == kFxBS) pair_bs<double>(dx, dy, dz, F, a.uq, s.v);
+        fx_pair_fp64<KIND>(xi - a.xs[3 * (size_t)j], yi - a.xs[3 * (size_t)j + 1], zi - a.xs[3 * (size_t)j + 2], F, a, f8,
+                           q, near, s.v);
     }
     return s;
 }

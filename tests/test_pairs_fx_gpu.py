@@ -64,6 +64,27 @@ def test_tiles_outside_the_formats(gpu_ctx, oracle_built):
     check_all(gpu_ctx, oracle_built, xs, fs, xb, fb[:, :3])
 
 
+@pytest.mark.parametrize("n", [33, 300, 1100])
+@pytest.mark.parametrize("b", [0.6, 1.0, 1.3])
+def test_whole_sets_outside_the_formats(gpu_ctx, oracle_built, n, b):
+    """Sets spread over thousands of radii, in FP64 throughout: distant,
+    overlapping and coincident pairs."""
+    rng = np.random.default_rng(n)
+    def spread(m):
+        x = rng.uniform(-4000.0, 4000.0, size=(m, 3))
+        x[1::3] = x[0:-1:3][:len(x[1::3])] + rng.normal(size=(len(x[1::3]), 3))
+        x[2::6] = x[0:-2:6][:len(x[2::6])]
+        return x
+    xs, xb = spread(n), spread(n + 40)
+    xb[3::4] = xs[:len(xb[3::4])] + 0.7 * rng.normal(size=(len(xb[3::4]), 3))
+    fs, fb = rng.normal(size=(n, 6)), rng.normal(size=(n + 40, 3))
+    gpu_ctx.set_precision(0)
+    check_all(gpu_ctx, oracle_built, xs, fs, xb, fb, b=b)
+    xs[n // 2, 1] = 1e200  # the square overflows: as far as can be
+    got, want = N(gpu_ctx.mss(T(xs), T(fs))), oracle_built.mss(xs, fs)
+    assert np.isfinite(want).all() and rel_err(got, want) < tol(n)
+
+
 def test_not_finite_loads_and_positions(gpu_ctx, oracle_built):
     """A NaN load reaches every target, an infinite one too; a NaN position
     its own row and, as a source, all."""
